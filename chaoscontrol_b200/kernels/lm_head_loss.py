@@ -93,8 +93,8 @@ class _LinearCeFn(torch.autograd.Function):
         x, weight, targets, lse, rw = ctx.saved_tensors
         roww = rw.float().contiguous() if ctx.has_w else None
         _, _, dX, part = LH.lm_head_train(x, None, weight, targets, gscale=1.0, rowweight=roww, lse=lse)
-        dW, _ = splitk_reduce(part)
-        return dX * gtotal.to(dX.dtype), (dW * gtotal).to(weight.dtype), None, None
+        dW, _ = splitk_reduce(part, scale=gtotal.float(), out_dtype=weight.dtype)
+        return dX * gtotal.to(dX.dtype), dW, None, None
 
 
 def _linear_ce(x, weight, targets, row_weight=None):

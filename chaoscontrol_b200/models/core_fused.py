@@ -71,9 +71,9 @@ class _PostScanFn(torch.autograd.Function):
         D = x2.shape[1]
         dx3 = go.reshape(-1, D).contiguous()
         du = G.gemm(dx3, Wproj, b_mn=True, epi=G.EPI_DSILU, r1=u, rowss=ss2, inv_dim=1.0 / D, eps=ctx.eps)
-        dWproj, _ = T.splitk_reduce(T._wgrad(dx3, f))
+        dWproj, _ = T.splitk_reduce(T._wgrad(dx3, f), out_dtype=Wproj.dtype)
         dx2 = G.gemm(du, Wfc_f, b_mn=True, epi=G.EPI_RMSBWD, r1=x2, r2=dx3, rowss=ss2, inv_dim=1.0 / D, eps=ctx.eps)
-        dWfc, dwn2 = T.splitk_reduce(T._wgrad(du, x2), colscale=wn2, W=Wfc)
+        dWfc, dwn2 = T.splitk_reduce(T._wgrad(du, x2), colscale=wn2, W=Wfc, out_dtype=Wfc.dtype)
         dx2 = dx2.view(ctx.shp)
         return dx2, dx2, dwn2.to(wn2.dtype), None, dWfc.to(Wfc.dtype), dWproj.to(Wproj.dtype)
 
@@ -109,7 +109,7 @@ class _BlockFn(torch.autograd.Function):
     def backward(ctx, go, _ghT):
         B, Tn, D = ctx.dims
         dx, g = T.layer_backward(go.reshape(B * Tn, D).contiguous(), ctx.c, ctx.w, B, Tn, None,
-                                 want_dh0=ctx.has_h0 and ctx.needs_input_grad[1])
+                                 want_dh0=ctx.has_h0 and ctx.needs_input_grad[1], grad_dtype=ctx.w.Wo.dtype)
         ctx.c = None
         wdt = ctx.w.Wo.dtype
         dsel, dinp, dgate, ddelta = (t.to(wdt) for t in g.dWp.split(D, 0))

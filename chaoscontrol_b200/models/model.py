@@ -152,7 +152,7 @@ class _TrunkFn(torch.autograd.Function):
         for i in reversed(range(L)):
             w, c = ctx.ws[i], ctx.ctxs[i]
             dhT = dhT_stack[i].float().contiguous() if use_dhT else None
-            dx, g = T.layer_backward(dx, c, w, B, Tn, dhT, want_dh0=ctx.has_h0)
+            dx, g = T.layer_backward(dx, c, w, B, Tn, dhT, want_dh0=ctx.has_h0, grad_dtype=w.Wo.dtype)
             D = w.Wo.shape[0]
             pd = w.Wo.dtype
             dsel, dinp, dgate, ddelta = (t.to(pd) for t in g.dWp.split(D, dim=0))

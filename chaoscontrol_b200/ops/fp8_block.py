@@ -27,6 +27,7 @@ import torch.nn.functional as F
 
 from . import _lib
 from . import gemm as G
+from .trunk import splitk_reduce
 
 E4M3_MAX = 448.0
 BLOCK = 128
@@ -220,7 +221,7 @@ class _BlockFP8LinearFn(torch.autograd.Function):
             if g2.is_cuda and _lib.available():
                 S = G.pick_splits(N, K, g2.shape[0])
                 part = G.gemm(g2, xb, a_mn=True, b_mn=True, splits=S, out_dtype=torch.float32)
-                gw = part.sum(0) if part.dim() == 3 else part
+                gw, _ = splitk_reduce(part, out_dtype=wdtype if wdtype == torch.bfloat16 else torch.float32)
             else:
                 gw = g2.float().t() @ xb.float()
             gw = gw.to(wdtype)

@@ -99,36 +99,46 @@ def embed_bwd(tokens: torch.Tensor, dx: torch.Tensor, V: int,
 
 def splitk_reduce(part: torch.Tensor, *, colscale: Optional[torch.Tensor] = None,
                   W: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-                  dcol_out: Optional[torch.Tensor] = None):
+                  dcol_out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.float32,
+                  scale: Optional[torch.Tensor] = None):
     """Sum split-K partials ``[S, N, K]`` (or ``[N, K]``).
 
-    Returns ``(dW [N,K] fp32, dcol [K] fp32 or None)`` with
+    Returns ``(dW [N,K], dcol [K] or None)`` with
     ``dW = colscale * sum`` and ``dcol = sum_n sum[n,k] * W[n,k]`` -- the
-    gradients of ``W`` and of the RMSNorm weight folded into it.
+    gradients of ``W`` and of the RMSNorm weight folded into it.  ``scale`` (a one-element
+    fp32 tensor) multiplies both.  Results are fp32; ``out_dtype=torch.bfloat16`` rounds them
+    once, as they are stored.
     """
     if part.dim() == 2:
         part = part.unsqueeze(0)
     S, N, K = part.shape
     if part.is_cuda and (colscale is None or colscale.dtype == torch.bfloat16) and (
-            W is None or (W.dtype == torch.bfloat16 and W.is_contiguous())):
+            W is None or (W.dtype == torch.bfloat16 and W.is_contiguous())) and (
+            out_dtype in (torch.float32, torch.bfloat16)):
         if out is None:
-            out = torch.empty(N, K, dtype=torch.float32, device=part.device)
-        assert out.dtype == torch.float32 and out.is_contiguous()
+            out = torch.empty(N, K, dtype=out_dtype, device=part.device)
+        assert out.dtype == out_dtype and out.is_contiguous()
         nb = (N + 7) // 8
         colpart = torch.empty(nb, K, dtype=torch.float32, device=part.device) if W is not None else None
         dcol = None
         if W is not None:
-            dcol = dcol_out if dcol_out is not None else torch.empty(K, dtype=torch.float32,
-                                                                     device=part.device)
-        _lib.check(_lib.lib().ccb_splitk_reduce(part.data_ptr(), S, part.stride(0), N, K,
-                                                _lib.ptr(colscale), _lib.ptr(W), out.data_ptr(), 0,
-                                                _lib.ptr(colpart), _lib.ptr(dcol), 0,
-                                                _lib.stream_ptr()), "splitk_reduce")
+            dcol = dcol_out if dcol_out is not None else torch.empty(K, dtype=out_dtype, device=part.device)
+            assert dcol.dtype == out_dtype
+        if scale is not None:
+            assert scale.dtype == torch.float32 and scale.numel() == 1
+        _lib.check(_lib.lib().ccb_splitk_reduce_as(part.data_ptr(), S, part.stride(0), N, K,
+                                                   _lib.ptr(colscale), _lib.ptr(W), out.data_ptr(),
+                                                   int(out_dtype == torch.bfloat16), 0, _lib.ptr(scale),
+                                                   _lib.ptr(colpart), _lib.ptr(dcol), 0,
+                                                   _lib.stream_ptr()), "splitk_reduce")
         return out, dcol
     s = part.float().sum(0)
-    dcol = (s * W.float()).sum(0) if W is not None else None
+    if scale is not None:
+        s = s * scale.float()
+    dcol = (s * W.float()).sum(0).to(out_dtype) if W is not None else None
     if colscale is not None:
         s = s * colscale.float()[None, :]
+    s = s.to(out_dtype)
     if out is not None:
         out.copy_(s)
         s = out
@@ -187,7 +197,7 @@ class LayerCtx:
 
 @dataclass
 class LayerGrads:
-    dWp: torch.Tensor       # [4D, D] fp32
+    dWp: torch.Tensor       # [4D, D] fp32 (or the grad_dtype asked for)
     dWo: torch.Tensor
     dWfc: torch.Tensor
     dWproj: torch.Tensor
@@ -244,31 +254,33 @@ def layer_forward(x: torch.Tensor, ss1: torch.Tensor, w: LayerWeights, B: int, T
 
 def layer_backward(dx3: torch.Tensor, ctx: LayerCtx, w: LayerWeights, B: int, T: int,
                    dhT: Optional[torch.Tensor] = None, *, want_dh0: bool = False,
-                   outs: Optional[dict] = None):
+                   outs: Optional[dict] = None, grad_dtype: torch.dtype = torch.float32):
     """Backward of :func:`layer_forward`.  Returns ``(dx, LayerGrads)``.
 
+    Weight gradients are fp32, or rounded once to ``grad_dtype`` as they are stored.
     ``outs`` may map ``dWp / dWo / dWfc / dWproj / dwn1 / dwn2`` to preallocated
     fp32 tensors (views of a flat gradient buffer) that receive the results.
     """
     R, D = ctx.x.shape
     inv_d = 1.0 / D
     o = outs or {}
+    gd = grad_dtype
     # feed-forward half
     du = gemm(dx3, w.Wproj, b_mn=True, epi=EPI_DSILU, r1=ctx.u, rowss=ctx.ss2, inv_dim=inv_d, eps=EPS)
-    dWproj, _ = splitk_reduce(_wgrad(dx3, ctx.f), out=o.get("dWproj"))
+    dWproj, _ = splitk_reduce(_wgrad(dx3, ctx.f), out=o.get("dWproj"), out_dtype=gd)
     dx2 = gemm(du, w.Wfc_f, b_mn=True, epi=EPI_RMSBWD, r1=ctx.x2, r2=dx3, rowss=ctx.ss2,
                inv_dim=inv_d, eps=EPS)
     dWfc, dwn2 = splitk_reduce(_wgrad(du, ctx.x2), colscale=w.wn2, W=w.Wfc, out=o.get("dWfc"),
-                               dcol_out=o.get("dwn2"))
+                               dcol_out=o.get("dwn2"), out_dtype=gd)
     # recurrence half
     dy = gemm(dx2, w.Wo, b_mn=True)
-    dWo, _ = splitk_reduce(_wgrad(dx2, ctx.y), out=o.get("dWo"))
+    dWo, _ = splitk_reduce(_wgrad(dx2, ctx.y), out=o.get("dWo"), out_dtype=gd)
     dP, dlog_a, dh0 = _scan_bwd(ctx.P, w.log_a32, ctx.h0, ctx.h, dy, dhT, ctx.ss1, inv_d, EPS, B, T,
                                 D, want_dh0)
     dx = gemm(dP, w.Wp_f, b_mn=True, epi=EPI_RMSBWD, r1=ctx.x, r2=dx2, rowss=ctx.ss1, inv_dim=inv_d,
               eps=EPS)
     dWp, dwn1 = splitk_reduce(_wgrad(dP, ctx.x), colscale=w.wn1, W=w.Wp, out=o.get("dWp"),
-                              dcol_out=o.get("dwn1"))
+                              dcol_out=o.get("dwn1"), out_dtype=gd)
     if "dlog_a" in o:
         o["dlog_a"].copy_(dlog_a)
     return dx, LayerGrads(dWp, dWo, dWfc, dWproj, dwn1, dwn2, dlog_a, dh0)
