@@ -309,6 +309,310 @@ scan_bwd_kernel(const __nv_bfloat16* __restrict__ P, long long ldp, const float*
   }
 }
 
+// ---- time-tiled scans for few channels -----------------------------------------------------------
+// The kernels above give every channel pair one thread for all T steps, so a batch of B rows keeps only
+// B * D / 256 blocks busy and each of them waits for memory and for the special functions of one step
+// after the other.  Here the warps of a block share the steps of 64 channels of one row: a tile is
+// NW * U steps, warp w takes U of them, evaluates their gates (the expensive part, independent of the
+// recurrence) and folds them into one affine map state -> A * state + b; the maps of the tile go through
+// shared memory, every warp composes them in order up to its own steps, and then runs its U steps from
+// the exact carry with the serial kernels' arithmetic.  One barrier per tile (the maps are double
+// buffered); the next tile's operands are requested before it.
+// CL > 1: a cluster of CL blocks shares one row's steps the same way, the composed map of each block's
+// tile goes to the other blocks' shared memory, so that even one row of 256 channels uses 32 SMs.
+// All fp32, as above: only the carry at a warp's first step is rounded differently.
+// a * b, except that two non-zero factors never give zero: a product of decays that underflows would turn an
+// infinite state into NaN where the serial kernels keep it infinite (the smallest normal number stands in).
+__device__ __forceinline__ float2 keep_normal(float2 prod, float2 a, float2 b) {
+  if (prod.x == 0.f && a.x != 0.f && b.x != 0.f) prod.x = 1.17549435e-38f;
+  if (prod.y == 0.f && a.y != 0.f && b.y != 0.f) prod.y = 1.17549435e-38f;
+  return prod;
+}
+__device__ __forceinline__ void st_cluster_f4(uint32_t addr, float4 v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
+// The carry of a tile.  In: this warp's map (A, b) and the state at the start of the (cluster's) tile.  Returns
+// the state at this warp's first step and leaves the state after the whole tile in `st`.
+template <int NW, int CL>
+__device__ __forceinline__ float2 tile_carry(float4 (&seg)[NW][32], float4 (&blk)[CL][32], int warp, int lane, int rank,
+                                             float4 map, float2& st) {
+  seg[warp][lane] = map;
+  __syncthreads();
+  float2 mine = st;
+  if constexpr (CL == 1) {
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      if (w == warp) mine = st;
+      const float4 v = seg[w][lane];
+      st = __ffma2_rn(f2(v.x, v.y), st, f2(v.z, v.w));
+    }
+  } else {
+    // the block's own composition: up to this warp, and whole
+    float2 A = f2s(1.f), bb = f2s(0.f), Am = A, bm = bb;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      if (w == warp) { Am = A; bm = bb; }
+      const float4 v = seg[w][lane];
+      A = keep_normal(__fmul2_rn(A, f2(v.x, v.y)), A, f2(v.x, v.y));
+      bb = __ffma2_rn(f2(v.x, v.y), bb, f2(v.z, v.w));
+    }
+    if (warp < CL) st_cluster_f4(mapa_shared(smem_u32(&blk[rank][lane]), (uint32_t)warp), make_float4(A.x, A.y, bb.x, bb.y));
+    cluster_sync_all();
+#pragma unroll
+    for (int r = 0; r < CL; ++r) {
+      if (r == rank) mine = st;
+      const float4 v = blk[r][lane];
+      st = __ffma2_rn(f2(v.x, v.y), st, f2(v.z, v.w));
+    }
+    mine = __ffma2_rn(Am, mine, bm);
+  }
+  return mine;
+}
+
+template <int U, int NW, int MINB, int CL>
+__global__ void __launch_bounds__(32 * NW, MINB)
+scan_tile_fwd_kernel(const __nv_bfloat16* __restrict__ P, long long ldp, const float* __restrict__ log_a,
+                     const float* __restrict__ h0, __nv_bfloat16* __restrict__ y,
+                     __nv_bfloat16* __restrict__ hout, float* __restrict__ hT, int T, int D,
+                     long long la_bstride) {
+  static_assert(CL <= NW, "warp r hands the block's map to block r of the cluster");
+  constexpr int TT = U * NW * CL;
+  __shared__ float4 seg[2][NW][32];
+  __shared__ float4 blk[2][CL][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = CL > 1 ? (int)cluster_ctarank() : 0;
+  const int first = (rank * NW + warp) * U;        // this warp's first step of a tile
+  if (CL > 1) cluster_sync_all();                  // every block runs before any writes to its shared memory
+  const int b = blockIdx.y;
+  const int d = (blockIdx.x * 32 + lane) * 2;
+  const bool on = d < D;
+  float2 nal2e = f2s(0.f), st = f2s(0.f);
+  if (on) {
+    const float* la = log_a + b * la_bstride + d;
+    nal2e = f2(-sigmoidf_fast(la[0]) * 1.4426950408889634f, -sigmoidf_fast(la[1]) * 1.4426950408889634f);
+    if (h0 != nullptr) st = f2(h0[(long long)b * D + d], h0[(long long)b * D + d + 1]);
+  }
+  const uint32_t* Pw = reinterpret_cast<const uint32_t*>(P + (long long)b * T * ldp + d);
+  const long long rowstride = ldp / 2;
+  const int dq = D / 2;
+  uint32_t* yw = reinterpret_cast<uint32_t*>(y + ((long long)b * T) * D + d);
+  uint32_t* hw = hout ? reinterpret_cast<uint32_t*>(hout + ((long long)b * T) * D + d) : nullptr;
+
+  uint32_t raw[U][4];
+  auto fetch = [&](int t0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (on && t0 + u < T) {
+        const uint32_t* row = Pw + (long long)(t0 + u) * rowstride;
+        raw[u][0] = __ldg(row);
+        raw[u][1] = __ldg(row + dq);
+        raw[u][2] = __ldg(row + 2 * dq);
+        raw[u][3] = __ldg(row + 3 * dq);
+      } else {
+        raw[u][0] = raw[u][1] = raw[u][2] = raw[u][3] = 0u;
+      }
+    }
+  };
+  fetch(first);
+  int buf = 0;
+  for (int t0 = 0; t0 < T; t0 += TT, buf ^= 1) {
+    const int tw = t0 + first;
+    float2 dec[U], upd[U], gate[U];
+    float2 A = f2s(1.f), bb = f2s(0.f);
+    if (tw < T) {                          // a warp past the end leaves the state as it is
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const Gates2 g = eval_gates2<false>(unpack_bf16x2(raw[u][0]), unpack_bf16x2(raw[u][1]),
+                                            unpack_bf16x2(raw[u][2]), unpack_bf16x2(raw[u][3]), nal2e);
+        const bool in = tw + u < T;
+        dec[u] = in ? g.decay : f2s(1.f);
+        upd[u] = in ? __fmul2_rn(g.sel, g.cand) : f2s(0.f);
+        gate[u] = g.gate;
+        A = __fmul2_rn(A, dec[u]);
+        bb = __ffma2_rn(dec[u], bb, upd[u]);
+      }
+    }
+    if (t0 + TT < T) fetch(tw + TT);
+    if (A.x == 0.f || A.y == 0.f) {
+      A = f2s(1.f);
+#pragma unroll
+      for (int u = 0; u < U; ++u) A = keep_normal(__fmul2_rn(A, dec[u]), A, dec[u]);
+    }
+    float2 h = tile_carry<NW, CL>(seg[buf], blk[buf], warp, lane, rank, make_float4(A.x, A.y, bb.x, bb.y), st);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (on && tw + u < T) {
+        h = __ffma2_rn(dec[u], h, upd[u]);
+        const long long o = (long long)(tw + u) * dq;
+        const float2 yv = __fmul2_rn(gate[u], h);
+        yw[o] = pack_bf16x2(yv.x, yv.y);
+        if (hw) hw[o] = pack_bf16x2(h.x, h.y);
+      }
+    }
+  }
+  if (hT != nullptr && rank == 0 && warp == 0 && on) {
+    hT[(long long)b * D + d] = st.x;
+    hT[(long long)b * D + d + 1] = st.y;
+  }
+}
+
+// Backward: the same split over t = T-1 .. 0.  The carried quantity c = dL/dh[t] * decay[t] obeys
+// c' = decay * (c + dy * gate), again an affine map; with the carry known each warp runs the serial
+// kernel's step.  d log_a is summed per warp and joined in warp order.
+template <int U, int NW, int MINB, int CL>
+__global__ void __launch_bounds__(32 * NW, MINB)
+scan_tile_bwd_kernel(const __nv_bfloat16* __restrict__ P, long long ldp, const float* __restrict__ log_a,
+                     const float* __restrict__ h0, const __nv_bfloat16* __restrict__ hstates,
+                     const __nv_bfloat16* __restrict__ dy, const float* __restrict__ dhT,
+                     const float* __restrict__ rowss, float inv_dim, float eps,
+                     __nv_bfloat16* __restrict__ dP, long long lddp, float* __restrict__ dloga_part,
+                     float* __restrict__ dh0, int T, int D, long long la_bstride) {
+  static_assert(CL <= NW, "warp r hands the block's map to block r of the cluster");
+  constexpr int TT = U * NW * CL;
+  __shared__ float4 seg[2][NW][32];
+  __shared__ float4 blk[2][CL][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = CL > 1 ? (int)cluster_ctarank() : 0;
+  const int first = (rank * NW + warp) * U;        // this warp's first step of a tile
+  if (CL > 1) cluster_sync_all();                  // every block runs before any writes to its shared memory
+  const int b = blockIdx.y;
+  const int d = (blockIdx.x * 32 + lane) * 2;
+  const bool on = d < D;
+  float2 a = f2s(0.f), carry = f2s(0.f), hinit = f2s(0.f);
+  if (on) {
+    const float* la = log_a + b * la_bstride + d;
+    a = f2(sigmoidf_fast(la[0]), sigmoidf_fast(la[1]));
+    if (dhT != nullptr) carry = f2(dhT[(long long)b * D + d], dhT[(long long)b * D + d + 1]);
+    if (h0 != nullptr) hinit = f2(h0[(long long)b * D + d], h0[(long long)b * D + d + 1]);
+  }
+  const float2 nal2e = f2(-a.x * 1.4426950408889634f, -a.y * 1.4426950408889634f);
+  const long long rowbase = (long long)b * T;
+  const int dq = D / 2;
+  const uint32_t* Pw = reinterpret_cast<const uint32_t*>(P + rowbase * ldp + d);
+  const long long prs = ldp / 2;
+  uint32_t* dPw = reinterpret_cast<uint32_t*>(dP + rowbase * lddp + d);
+  const long long dprs = lddp / 2;
+  const uint32_t* hw = reinterpret_cast<const uint32_t*>(hstates + rowbase * D + d);
+  const uint32_t* dyw = reinterpret_cast<const uint32_t*>(dy + rowbase * D + d);
+
+  uint32_t raw[U][4], dyr[U], hr[U + 1];
+  float rsr[U];
+  // step u of a tile that starts at position j0 of the reversed order is t = T - 1 - (j0 + u)
+  auto fetch = [&](int j0) {
+#pragma unroll
+    for (int u = 0; u <= U; ++u) {
+      const int t = T - 1 - (j0 + u);
+      hr[u] = (on && t >= 0) ? __ldg(hw + (long long)t * dq) : 0u;
+      if (u == U) break;
+      if (on && t >= 0) {
+        const uint32_t* row = Pw + (long long)t * prs;
+        raw[u][0] = __ldg(row);
+        raw[u][1] = __ldg(row + dq);
+        raw[u][2] = __ldg(row + 2 * dq);
+        raw[u][3] = __ldg(row + 3 * dq);
+        dyr[u] = __ldg(dyw + (long long)t * dq);
+      } else {
+        raw[u][0] = raw[u][1] = raw[u][2] = raw[u][3] = dyr[u] = 0u;
+      }
+      rsr[u] = (rowss && t >= 0) ? __ldg(rowss + rowbase + t) : 0.f;
+    }
+  };
+  fetch(first);
+  float2 da = f2s(0.f);
+  int buf = 0;
+  for (int j0 = 0; j0 < T; j0 += TT, buf ^= 1) {
+    const int jw = j0 + first;
+    Gates2 g[U];
+    float2 dyv[U], hc[U + 1];
+    float rs[U];
+    float2 A = f2s(1.f), bb = f2s(0.f);
+    hc[U] = unpack_bf16x2(hr[U]);
+    if (jw < T) {                          // a warp past the beginning leaves the carry as it is
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        g[u] = eval_gates2<true>(unpack_bf16x2(raw[u][0]), unpack_bf16x2(raw[u][1]), unpack_bf16x2(raw[u][2]),
+                                 unpack_bf16x2(raw[u][3]), nal2e);
+        dyv[u] = unpack_bf16x2(dyr[u]);
+        hc[u] = unpack_bf16x2(hr[u]);
+        rs[u] = rowss ? rsqrtf(rsr[u] * inv_dim + eps) : 1.f;
+        if (jw + u < T) {
+          A = __fmul2_rn(A, g[u].decay);
+          bb = __fmul2_rn(g[u].decay, __ffma2_rn(dyv[u], g[u].gate, bb));
+        }
+      }
+    }
+    if (j0 + TT < T) fetch(jw + TT);
+    if (A.x == 0.f || A.y == 0.f) {
+      A = f2s(1.f);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (jw + u < T) A = keep_normal(__fmul2_rn(A, g[u].decay), A, g[u].decay);
+    }
+    float2 c = tile_carry<NW, CL>(seg[buf], blk[buf], warp, lane, rank, make_float4(A.x, A.y, bb.x, bb.y), carry);
+    const float2 one = f2s(1.f), neg1 = f2s(-1.f);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = T - 1 - (jw + u);
+      if (t >= 0) {
+        const float2 hprev = t > 0 ? hc[u + 1] : hinit;
+        const float2 rs2 = f2s(rs[u]);
+        // y = gate * h;  h = decay * hprev + sel * cand
+        const float2 dgate = __fmul2_rn(dyv[u], hc[u]);
+        const float2 dh = __ffma2_rn(dyv[u], g[u].gate, c);
+        const float2 ddec = __fmul2_rn(dh, hprev);
+        c = __fmul2_rn(dh, g[u].decay);
+        const float2 ds = __fmul2_rn(__fmul2_rn(dh, g[u].cand), __fmul2_rn(g[u].sel, __ffma2_rn(g[u].sel, neg1, one)));
+        const float2 dc = __fmul2_rn(__fmul2_rn(dh, g[u].sel), __ffma2_rn(__fmul2_rn(g[u].cand, neg1), g[u].cand, one));
+        const float2 dg = __fmul2_rn(dgate, __fmul2_rn(g[u].gate, __ffma2_rn(g[u].gate, neg1, one)));
+        // decay = exp(-delta * a): d/d delta = -a * decay ; d/d a = -delta * decay
+        const float2 dd = __fmul2_rn(__fmul2_rn(ddec, __fmul2_rn(f2(-a.x, -a.y), g[u].decay)), g[u].sp_sig);
+        da = __ffma2_rn(__fmul2_rn(ddec, g[u].delta), __fmul2_rn(g[u].decay, neg1), da);
+        if (on) {
+          const float2 o0 = __fmul2_rn(ds, rs2), o1 = __fmul2_rn(dc, rs2), o2 = __fmul2_rn(dg, rs2),
+                       o3 = __fmul2_rn(dd, rs2);
+          uint32_t* orow = dPw + (long long)t * dprs;
+          orow[0] = pack_bf16x2(o0.x, o0.y);
+          orow[dq] = pack_bf16x2(o1.x, o1.y);
+          orow[2 * dq] = pack_bf16x2(o2.x, o2.y);
+          orow[3 * dq] = pack_bf16x2(o3.x, o3.y);
+        }
+      }
+    }
+  }
+  if (dloga_part != nullptr) {
+    __syncthreads();                       // the maps of the last tile have been read
+    float2* join = reinterpret_cast<float2*>(&seg[0][0][0]);
+    join[warp * 32 + lane] = da;
+    __syncthreads();
+    float2 t = f2s(0.f);
+    if (warp == 0) {
+      t = join[lane];
+#pragma unroll
+      for (int w = 1; w < NW; ++w) t = __fadd2_rn(t, join[w * 32 + lane]);
+    }
+    if constexpr (CL > 1) {                // block sums to block 0, added in block order
+      cluster_sync_all();                  // block 0 has read the maps of its last tile
+      if (warp == 0) st_cluster_f4(mapa_shared(smem_u32(&blk[0][rank][lane]), 0u), make_float4(t.x, t.y, 0.f, 0.f));
+      cluster_sync_all();
+      if (warp == 0 && rank == 0) {
+        t = f2(blk[0][0][lane].x, blk[0][0][lane].y);
+#pragma unroll
+        for (int r = 1; r < CL; ++r) t = __fadd2_rn(t, f2(blk[0][r][lane].x, blk[0][r][lane].y));
+      }
+    }
+    if (warp == 0 && rank == 0 && on) {
+      // d a / d log_a = a (1 - a)
+      dloga_part[(long long)b * D + d] = t.x * a.x * (1.f - a.x);
+      dloga_part[(long long)b * D + d + 1] = t.y * a.y * (1.f - a.y);
+    }
+  }
+  if (dh0 != nullptr && rank == 0 && warp == 0 && on) {
+    dh0[(long long)b * D + d] = carry.x;
+    dh0[(long long)b * D + d + 1] = carry.y;
+  }
+}
+
 // Plain (unfused) diagonal scan kept for API parity with the reference's
 // ssm_scan(decay, update): fp32 decay, bf16 or fp32 update, fp32 states out.
 // Plain recurrence state[t] = decay[t] * state[t-1] + update[t] for the public ssm_scan op, in
@@ -381,12 +685,73 @@ extern "C" int ccb_scan_poly_exp(int mode) {
   return old;
 }
 
+template <typename K, typename... A>
+static int launch_tile(K kern, int cl, int threads, int64_t B, int64_t D, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((D / 2 + 31) / 32), (unsigned)B, (unsigned)cl);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = (unsigned)cl;
+  cfg.attrs = at; cfg.numAttrs = cl > 1 ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  count_launch();
+  return e == cudaSuccess ? 0 : set_error("scan launch: %s", cudaGetErrorString(e));
+}
+
+template <int U, int NW, int MINB, int CL>
+static int launch_tile_fwd(const void* P, int64_t ldp, const float* log_a, const float* h0, void* y, void* hout, float* hT,
+                           int64_t B, int64_t T, int64_t D, int64_t la_bstride, cudaStream_t stream) {
+  return launch_tile(scan_tile_fwd_kernel<U, NW, MINB, CL>, CL, 32 * NW, B, D, stream, (const __nv_bfloat16*)P,
+                     (long long)ldp, log_a, h0, (__nv_bfloat16*)y, (__nv_bfloat16*)hout, hT, (int)T, (int)D,
+                     (long long)la_bstride);
+}
+
+template <int U, int NW, int MINB, int CL>
+static int launch_tile_bwd(const void* P, int64_t ldp, const float* log_a, const float* h0, const void* hstates,
+                           const void* dy, const float* dhT, const float* rowss, float inv_dim, float eps, void* dP,
+                           int64_t lddp, float* dloga_part, float* dh0, int64_t B, int64_t T, int64_t D,
+                           int64_t la_bstride, cudaStream_t stream) {
+  return launch_tile(scan_tile_bwd_kernel<U, NW, MINB, CL>, CL, 32 * NW, B, D, stream, (const __nv_bfloat16*)P,
+                     (long long)ldp, log_a, h0, (const __nv_bfloat16*)hstates, (const __nv_bfloat16*)dy, dhT, rowss,
+                     inv_dim, eps, (__nv_bfloat16*)dP, (long long)lddp, dloga_part, dh0, (int)T, (int)D,
+                     (long long)la_bstride);
+}
+
+// Which scan.  `warps` = 64-channel warps of the whole batch.  A serial thread needs every SM full of them to
+// hide a step's latency; measured on a B200, T = 512, D = 256, serial / time-tiled in us (events, cold L2):
+//   forward   B = 1: 117 / 11   64: 126 / 32   256: 146 / 91    512: 189 / 167   1024: 283 / 318
+//   backward  B = 1: 181 / 20   64: 191 / 63   256: 228 / 185   512: 318 / 353   1024: 576 / 687
+// so the line lies at 16 (forward) and 8 (backward) warps per SM.  Below 64 steps a tile is partly empty and the
+// lines are equal nearer: B = 256, T = 16: 13 / 17 and 19 / 26; B = 128, T = 32: 15 / 13 and 23 / 19.
+static bool scan_tiled(int64_t warps, int64_t T, int per_sm) {
+  return g_scan_poly_exp == 2 && warps <= (int64_t)(T >= 64 ? per_sm : 4) * ccb_num_sms();
+}
+// Blocks of a cluster: while they fit two to an SM and each still has steps (B = 1: 23 us with one block, 11 with
+// eight; 16 rows of 256 channels: 25 with one, 17 with four, 19 with eight).
+static int scan_cluster(int64_t warps, int64_t T, int tile) {
+  int cl = 8;
+  while (cl > 1 && (warps * cl > 2 * ccb_num_sms() || (int64_t)tile * (cl / 2) >= T)) cl /= 2;
+  return cl;
+}
+
 extern "C" int ccb_scan_fwd(const void* P, int64_t ldp, const float* log_a, const float* h0,
                             void* y, void* hout, float* hT, int64_t B, int64_t T, int64_t D,
                             int64_t la_bstride, void* stream) {
   if (B <= 0 || T <= 0) return 0;
   if (D % 8 != 0 || ldp % 2 != 0) return set_error("ccb_scan_fwd: D must be a multiple of 8");
   dim3 grid((unsigned)((D / 2 + SCAN_THREADS - 1) / SCAN_THREADS), (unsigned)B);
+  const int64_t warps = B * ((D + 63) / 64);
+  if (scan_tiled(warps, T, 16)) {
+    auto launch = launch_tile_fwd<8, 8, 2, 1>;
+    switch (scan_cluster(warps, T, 64)) {
+      case 8: launch = launch_tile_fwd<8, 8, 2, 8>; break;
+      case 4: launch = launch_tile_fwd<8, 8, 2, 4>; break;
+      case 2: launch = launch_tile_fwd<8, 8, 2, 2>; break;
+    }
+    return launch(P, ldp, log_a, h0, y, hout, hT, B, T, D, la_bstride, (cudaStream_t)stream);
+  }
   // forward: six steps loaded ahead and six resident blocks per SM (72 registers) measured best: 0.286 ms at
   // 524 288 rows against 0.311 ms with eight steps ahead and four blocks
   auto kern = g_scan_poly_exp == 2 ? scan_fwd_kernel<2, 6, 6> : (g_scan_poly_exp == 1 ? scan_fwd_kernel<1> : scan_fwd_kernel<0>);
@@ -406,6 +771,17 @@ extern "C" int ccb_scan_bwd(const void* P, int64_t ldp, const float* log_a, cons
   if (B <= 0 || T <= 0) return 0;
   if (D % 8 != 0) return set_error("ccb_scan_bwd: D must be a multiple of 8");
   dim3 grid((unsigned)((D / 2 + SCAN_THREADS - 1) / SCAN_THREADS), (unsigned)B);
+  const int64_t warps = B * ((D + 63) / 64);
+  if (scan_tiled(warps, T, 8)) {
+    auto launch = launch_tile_bwd<4, 8, 2, 1>;
+    switch (scan_cluster(warps, T, 32)) {
+      case 8: launch = launch_tile_bwd<4, 8, 2, 8>; break;
+      case 4: launch = launch_tile_bwd<4, 8, 2, 4>; break;
+      case 2: launch = launch_tile_bwd<4, 8, 2, 2>; break;
+    }
+    return launch(P, ldp, log_a, h0, hstates, dy, dhT, rowss, inv_dim, eps, dP, lddp, dloga_part, dh0, B, T, D,
+                  la_bstride, (cudaStream_t)stream);
+  }
   // backward: eight steps ahead, four blocks per SM (116 registers): 0.538 ms; six blocks with six / four steps
   // ahead measured 0.632 / 0.706 ms (fewer loads in flight cost more than the extra warps bring)
   auto kern = g_scan_poly_exp == 2 ? scan_bwd_kernel<2> : (g_scan_poly_exp == 1 ? scan_bwd_kernel<1> : scan_bwd_kernel<0>);

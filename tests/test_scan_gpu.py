@@ -143,3 +143,57 @@ def test_ssm_scan_rejects_unlisted_dtype_pairs():
         S.ssm_scan(d, u)
     with pytest.raises(TypeError):
         S.ssm_scan(d.double(), u.double())
+
+
+# steps: one, off and on the 32- and 64-step tiles, past a cluster's tile; rows: clusters of 8, 4, 2 and 1 blocks;
+# channels: fewer than a warp's 64, and a last warp that is partly empty
+@pytest.mark.parametrize("B,T,D", [(1, 1, 8), (1, 63, 64), (1, 65, 72), (1, 513, 256), (2, 1100, 136), (60, 130, 64),
+                                   (100, 97, 64), (130, 70, 128), (300, 33, 8)])
+@pytest.mark.parametrize("full", [False, True])
+def test_time_tiled_scan_against_serial_arithmetic(B, T, D, full):
+    """The time-tiled kernels (few channels) against the serial scalar kernels (mode 0) on the same operands; ``full``
+    adds every optional operand.  Both round to fp32 per step and evaluate the same gates, so the 32-bit results
+    agree as the arithmetic modes do among themselves and the bf16 ones to an ulp of their largest value."""
+    g = torch.Generator(device="cuda").manual_seed(B * T + D)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    P, dy = (rnd(B * T, 4 * D) * 1.5).bfloat16(), rnd(B * T, D).bfloat16()
+    log_a = rnd(B, D) if full else rnd(D)
+    h0, dhT = (rnd(B, D), rnd(B, D)) if full else (None, None)
+    ss = torch.rand(B * T, generator=g, device="cuda") * D + 0.5 if full else None
+    res = []
+    for mode in (0, 2):
+        old = _lib.lib().ccb_scan_poly_exp(mode)
+        try:
+            y, h, hT = S.scan_fused_fwd(P, log_a, h0, B, T, D)
+            hb = res[0][1] if res else h                     # the same states for both backward kernels
+            dP, dla, dh0 = S.scan_fused_bwd(P, log_a, h0, hb, dy, dhT, ss, 1.0 / D, 1e-6, B, T, D, want_dh0=full)
+        finally:
+            _lib.lib().ccb_scan_poly_exp(old)
+        res.append((y, h, hT, dP, dla, dh0))
+    _lib.assert_ok()
+    for name, a, b in zip(("y", "h", "hT", "dP", "dlog_a", "dh0"), *res):
+        if a is None:
+            assert b is None
+            continue
+        tol = 2.0 ** -7 if a.dtype == torch.bfloat16 else 5e-4
+        assert (a.float() - b.float()).abs().max().item() <= tol * a.float().abs().max().item() + 1e-6, name
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_time_tiled_scan_keeps_infinite_states(bad):
+    """An infinite state under decays whose product underflows stays infinite, as in the serial kernels."""
+    B, T, D = 1, 600, 64
+    P = torch.zeros(B * T, 4 * D, device="cuda").bfloat16()
+    P[:, 3 * D:] = 20.0                                      # decay = exp(-20 * sigmoid(log_a)): 1e-4 a step
+    log_a, h0 = torch.zeros(D, device="cuda"), torch.zeros(B, D, device="cuda")
+    h0[0, 3] = bad
+    out = []
+    for mode in (0, 2):
+        old = _lib.lib().ccb_scan_poly_exp(mode)
+        try:
+            out.append(S.scan_fused_fwd(P, log_a, h0, B, T, D))
+        finally:
+            _lib.lib().ccb_scan_poly_exp(old)
+    for a, b in zip(*out):
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+    assert (out[0][2][0, 3].isinf() if bad == float("inf") else out[0][2][0, 3].isnan())
