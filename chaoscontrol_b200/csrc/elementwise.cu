@@ -577,6 +577,85 @@ rmsnorm_bwd_vec_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
   }
 }
 
+// ss[r] = sum_d v^2 with v = a (+ b, rounded to bf16 and stored to `sum`): the row statistics that the trunk's
+// GEMM epilogues take, for a residual stream that no kernel of this library produced.  One pass over the
+// row, a warp or part of one to a row as above.  (The same through fp32 copies of the tensor: 183 us at
+// 131 072 x 256, of 1.44 ms for the block's forward and backward.)
+template <int LPR, int NV>
+__global__ void __launch_bounds__(256)
+row_ss_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
+              __nv_bfloat16* __restrict__ sum, float* __restrict__ ss, long long R, int D) {
+  constexpr int RPW = 32 / LPR;
+  const int l = threadIdx.x % LPR;
+  const long long r = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * RPW + (threadIdx.x & 31) / LPR;
+  const bool on = r < R;                              // no early exit: the shuffles take the whole warp
+  const RowVec<NV> ar = load_row_vec<LPR, NV>(a + (on ? r : 0) * D, l, D);
+  RowVec<NV> br;
+  if (b) br = load_row_vec<LPR, NV>(b + (on ? r : 0) * D, l, D);
+  float acc = 0.f;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    float f[8];
+    unpack8(ar.q[v], f);
+    if (b) {
+      float g[8];
+      unpack8(br.q[v], g);
+      uint4 o;
+      o.x = pack_bf16x2(f[0] + g[0], f[1] + g[1]); o.y = pack_bf16x2(f[2] + g[2], f[3] + g[3]);
+      o.z = pack_bf16x2(f[4] + g[4], f[5] + g[5]); o.w = pack_bf16x2(f[6] + g[6], f[7] + g[7]);
+      unpack8(o, f);
+      const int c = (v * LPR + l) * 8;
+      if (on && c < D) *reinterpret_cast<uint4*>(sum + r * D + c) = o;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc += f[i] * f[i];
+  }
+  acc = row_sum<LPR>(acc);
+  if (on && l == 0) ss[r] = acc;
+}
+
+// A layer's weights as its GEMMs read them, in one launch: the four [D, D] projections packed (Wp, when
+// they are not already) and packed with the norm weight folded in (Wp_f), the feed-forward weight folded
+// (Wfc_f), and log_a in fp32.  All a few hundred KB: a launch's latency is what it costs, so one launch
+// takes the place of four (a 512-token evaluation chunk of one block spent 9 of its 61 us on them).
+struct LayerFold {
+  const __nv_bfloat16* w[4];      // select, in, gate, delta  [D, D]
+  const __nv_bfloat16 *wn1, *fc, *wn2, *log_a;
+  __nv_bfloat16 *Wp, *Wp_f, *Wfc_f;   // Wp may be null
+  float* log_a32;
+  int D, F;
+};
+__global__ void __launch_bounds__(256) layer_fold_kernel(const LayerFold p) {
+  const long long dd = (long long)p.D * p.D / 8, ff = (long long)p.F * p.D / 8;
+  const long long n = 4 * dd + ff + p.D / 8;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    if (i >= 4 * dd + ff) {
+      const long long c = (i - 4 * dd - ff) * 8;
+      float f[8];
+      unpack8(__ldg(reinterpret_cast<const uint4*>(p.log_a + c)), f);
+      *reinterpret_cast<float4*>(p.log_a32 + c) = make_float4(f[0], f[1], f[2], f[3]);
+      *reinterpret_cast<float4*>(p.log_a32 + c + 4) = make_float4(f[4], f[5], f[6], f[7]);
+      continue;
+    }
+    const bool proj = i < 4 * dd;
+    const long long e = proj ? i % dd : i - 4 * dd;          // 16-byte vector inside its matrix
+    const int col = (int)(e * 8 % p.D);
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(proj ? p.w[i / dd] : p.fc) + e);
+    float f[8], g[8];
+    unpack8(q, f);
+    unpack8(__ldg(reinterpret_cast<const uint4*>((proj ? p.wn1 : p.wn2) + col)), g);
+    uint4 o;
+    o.x = pack_bf16x2(f[0] * g[0], f[1] * g[1]); o.y = pack_bf16x2(f[2] * g[2], f[3] * g[3]);
+    o.z = pack_bf16x2(f[4] * g[4], f[5] * g[5]); o.w = pack_bf16x2(f[6] * g[6], f[7] * g[7]);
+    if (proj) {
+      reinterpret_cast<uint4*>(p.Wp_f)[i] = o;
+      if (p.Wp) reinterpret_cast<uint4*>(p.Wp)[i] = q;
+    } else {
+      reinterpret_cast<uint4*>(p.Wfc_f)[e] = o;
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // RMSNorm of any even width and 4-byte alignment (one warp per row), fp32 statistics.
 // y = x * rsqrt(mean(x^2) + eps) * w ; optional residual add x = x + res first.
@@ -992,6 +1071,43 @@ static void rmsnorm_dispatch(int64_t D, F f) {
   else if (D <= 768) f(integral_constant<int, 32>(), integral_constant<int, 3>());
   else if (D <= 1024) f(integral_constant<int, 32>(), integral_constant<int, 4>());
   else f(integral_constant<int, 32>(), integral_constant<int, 6>());
+}
+
+// ss[r] = sum_d (a (+ b))^2; with b, `sum` receives a + b.  Returns 1, launching nothing, for rows that are not
+// whole aligned 16-byte vectors or are wider than 1536.
+extern "C" int ccb_row_ss(const void* a, const void* b, void* sum, float* ss, int64_t R, int64_t D, void* stream) {
+  if (R <= 0) return 0;
+  if (!rmsnorm_vec_ok(D, a, b, sum, nullptr)) return 1;
+  rmsnorm_dispatch(D, [&](auto lpr, auto nv) {
+    constexpr int LPR = decltype(lpr)::value, NV = decltype(nv)::value;
+    const int64_t rows = 8 * (32 / LPR);
+    row_ss_kernel<LPR, NV><<<(unsigned)((R + rows - 1) / rows), 256, 0, (cudaStream_t)stream>>>(
+        (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)sum, ss, R, (int)D);
+  });
+  CCB_CHECK_LAUNCH("row_ss");
+  return 0;
+}
+
+// See layer_fold_kernel.  Returns 1, launching nothing, for operands that are not 16-byte aligned.
+extern "C" int ccb_layer_fold(const void* sel, const void* in, const void* gate, const void* delta, const void* wn1,
+                              const void* fc, const void* wn2, const void* log_a, void* Wp, void* Wp_f, void* Wfc_f,
+                              float* log_a32, int64_t D, int64_t F, void* stream) {
+  if (D <= 0 || F <= 0) return 0;
+  const uintptr_t all = (uintptr_t)sel | (uintptr_t)in | (uintptr_t)gate | (uintptr_t)delta | (uintptr_t)wn1 |
+                        (uintptr_t)fc | (uintptr_t)wn2 | (uintptr_t)log_a | (uintptr_t)Wp | (uintptr_t)Wp_f |
+                        (uintptr_t)Wfc_f | (uintptr_t)log_a32;
+  if (D % 8 != 0 || (all & 15) != 0) return 1;
+  LayerFold p;
+  p.w[0] = (const __nv_bfloat16*)sel; p.w[1] = (const __nv_bfloat16*)in;
+  p.w[2] = (const __nv_bfloat16*)gate; p.w[3] = (const __nv_bfloat16*)delta;
+  p.wn1 = (const __nv_bfloat16*)wn1; p.fc = (const __nv_bfloat16*)fc;
+  p.wn2 = (const __nv_bfloat16*)wn2; p.log_a = (const __nv_bfloat16*)log_a;
+  p.Wp = (__nv_bfloat16*)Wp; p.Wp_f = (__nv_bfloat16*)Wp_f; p.Wfc_f = (__nv_bfloat16*)Wfc_f;
+  p.log_a32 = log_a32;
+  p.D = (int)D; p.F = (int)F;
+  layer_fold_kernel<<<grid_for((4 * D * D + F * D + D) / 8, 256), 256, 0, (cudaStream_t)stream>>>(p);
+  CCB_CHECK_LAUNCH("layer_fold");
+  return 0;
 }
 
 extern "C" int ccb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* xsum,

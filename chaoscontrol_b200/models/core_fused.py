@@ -55,8 +55,11 @@ class _PostScanFn(torch.autograd.Function):
     def forward(ctx, x_pre, scan_out, wn2, eps, Wfc, Wproj):
         shp = x_pre.shape
         D = shp[-1]
-        x2 = (x_pre + scan_out).reshape(-1, D).contiguous()
-        ss2 = x2.float().square().sum(-1)
+        if x_pre.shape == scan_out.shape:
+            x2, ss2 = T.add_row_ss(x_pre.reshape(-1, D), scan_out.reshape(-1, D))
+        else:
+            x2 = (x_pre + scan_out).reshape(-1, D).contiguous()
+            ss2 = T.row_ss(x2)
         Wfc_f = T.fold_colscale(Wfc.contiguous(), wn2.contiguous())
         f = torch.empty(x2.shape[0], Wfc.shape[0], dtype=x2.dtype, device=x2.device)
         u = G.gemm(x2, Wfc_f, epi=G.EPI_ROWSCALE_SILU, rowss=ss2, inv_dim=1.0 / D, eps=eps, c2=f)
@@ -93,10 +96,10 @@ class _BlockFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, h0, sel, inp, gate, delta, out, fc, proj, wn1, wn2, log_a):
         B, Tn, D = x.shape
-        w = T.LayerWeights(Wp=torch.cat([sel, inp, gate, delta], 0), Wo=out.contiguous(), Wfc=fc.contiguous(),
-                           Wproj=proj.contiguous(), wn1=wn1.contiguous(), wn2=wn2.contiguous(), log_a=log_a).prepare()
+        w = T.LayerWeights.from_parts(sel, inp, gate, delta, Wo=out, Wfc=fc, Wproj=proj, wn1=wn1, wn2=wn2,
+                                      log_a=log_a)
         x2d = x.reshape(B * Tn, D).contiguous()
-        ss1 = x2d.float().square().sum(-1)
+        ss1 = T.row_ss(x2d)
         h0f = None if h0 is None else h0.float().contiguous()
         x3, _ss3, hT, c = T.layer_forward(x2d, ss1, w, B, Tn, h0f, save=True)
         ctx.w, ctx.c, ctx.dims = w, c, (B, Tn, D)

@@ -106,9 +106,8 @@ def _layer_weights(params: tuple, i: int) -> T.LayerWeights:
               delta.data_ptr() == base + 3 * step and sel.is_contiguous())
     if packed:
         Wp = torch.as_strided(sel, (4 * sel.shape[0], sel.shape[1]), (sel.shape[1], 1))
-    else:
-        Wp = torch.cat((sel, inp, gate, delta), dim=0)
-    return T.LayerWeights(Wp=Wp, Wo=out, Wfc=fc, Wproj=proj, wn1=wn1, wn2=wn2, log_a=log_a).prepare()
+        return T.LayerWeights(Wp=Wp, Wo=out, Wfc=fc, Wproj=proj, wn1=wn1, wn2=wn2, log_a=log_a).prepare()
+    return T.LayerWeights.from_parts(sel, inp, gate, delta, Wo=out, Wfc=fc, Wproj=proj, wn1=wn1, wn2=wn2, log_a=log_a)
 
 
 class _TrunkFn(torch.autograd.Function):

@@ -82,6 +82,8 @@ _SIGS = {
     "ccb_colsum": ([vp, i64, i64, vp, i64, vp], C.c_int),
     "ccb_colsum_as": ([vp, i64, i64, vp, i64, i64, vp], C.c_int),
     "ccb_fold_colscale": ([vp, vp, vp, i64, i64, vp], C.c_int),
+    "ccb_row_ss": ([vp, vp, vp, vp, i64, i64, vp], C.c_int),
+    "ccb_layer_fold": ([vp] * 12 + [i64, i64, vp], C.c_int),
     "ccb_rmsnorm_fwd": ([vp, vp, vp, vp, vp, vp, i64, i64, f32, vp], C.c_int),
     "ccb_rmsnorm_bwd_blocks": ([i64], i64),
     "ccb_rmsnorm_bwd": ([vp, vp, vp, vp, vp, vp, vp, i64, i64, vp], C.c_int),

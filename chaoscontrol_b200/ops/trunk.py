@@ -51,6 +51,31 @@ def fold_colscale(W: torch.Tensor, wn: torch.Tensor) -> torch.Tensor:
     return (W.float() * wn.float()[None, :]).to(W.dtype)
 
 
+def row_ss(x: torch.Tensor) -> torch.Tensor:
+    """fp32 ``[R]`` row sums of squares of a contiguous ``[R, D]``."""
+    if x.is_cuda and x.dtype == torch.bfloat16:
+        ss = torch.empty(x.shape[0], dtype=torch.float32, device=x.device)
+        rc = _lib.lib().ccb_row_ss(x.data_ptr(), None, None, ss.data_ptr(), x.shape[0], x.shape[1], _lib.stream_ptr())
+        if rc <= 0:
+            _lib.check(rc, "row_ss")
+            return ss
+    return x.float().square().sum(-1)
+
+
+def add_row_ss(a: torch.Tensor, b: torch.Tensor):
+    """``(a + b, its row sums of squares)`` of two ``[R, D]`` tensors."""
+    if a.is_cuda and a.dtype == b.dtype == torch.bfloat16 and a.is_contiguous() and b.is_contiguous():
+        out = torch.empty_like(a)
+        ss = torch.empty(a.shape[0], dtype=torch.float32, device=a.device)
+        rc = _lib.lib().ccb_row_ss(a.data_ptr(), b.data_ptr(), out.data_ptr(), ss.data_ptr(), a.shape[0], a.shape[1],
+                                   _lib.stream_ptr())
+        if rc <= 0:
+            _lib.check(rc, "row_ss")
+            return out, ss
+    x = (a + b).contiguous()
+    return x, x.float().square().sum(-1)
+
+
 def embed_fwd(tokens: torch.Tensor, E: torch.Tensor):
     """Gather rows of ``E`` and their sums of squares.  Returns ``(x [R,D], ss [R])``."""
     flat = tokens.reshape(-1)
@@ -174,7 +199,45 @@ class LayerWeights:
     Wfc_f: torch.Tensor = field(default=None)    # Wfc * wn2
     log_a32: torch.Tensor = field(default=None)
 
+    @classmethod
+    def from_parts(cls, sel, inp, gate, delta, *, Wo, Wfc, Wproj, wn1, wn2, log_a) -> "LayerWeights":
+        """Packed and prepared from four separate ``[D, D]`` projections."""
+        rest = dict(Wo=Wo.contiguous(), Wfc=Wfc.contiguous(), Wproj=Wproj.contiguous(), wn1=wn1.contiguous(),
+                    wn2=wn2.contiguous(), log_a=log_a)
+        w = cls(Wp=None, **rest)
+        if not w._fold_launch([t.contiguous() for t in (sel, inp, gate, delta)]):
+            w.Wp = torch.cat([sel, inp, gate, delta], 0)
+            w.prepare()
+        return w
+
+    def _fold_launch(self, parts: Optional[list] = None) -> bool:
+        """:meth:`prepare` as one kernel launch; False (nothing done) for operands it does not take.
+        ``parts``: the four projections, to be packed as well."""
+        ops = [self.Wfc, self.wn1, self.wn2, self.log_a, *(parts if parts is not None else [self.Wp])]
+        if not all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() for t in ops):
+            return False
+        F_, D = self.Wfc.shape
+        dev = self.Wfc.device
+        Wp = torch.empty(4 * D, D, dtype=torch.bfloat16, device=dev) if parts is not None else None
+        Wp_f = torch.empty(4 * D, D, dtype=torch.bfloat16, device=dev)
+        Wfc_f = torch.empty_like(self.Wfc)
+        la = torch.empty(D, dtype=torch.float32, device=dev)
+        src = ([t.data_ptr() for t in parts] if parts is not None else
+               [self.Wp.data_ptr() + 2 * i * D * D for i in range(4)])
+        rc = _lib.lib().ccb_layer_fold(*src, self.wn1.data_ptr(), self.Wfc.data_ptr(), self.wn2.data_ptr(),
+                                       self.log_a.data_ptr(), _lib.ptr(Wp), Wp_f.data_ptr(), Wfc_f.data_ptr(),
+                                       la.data_ptr(), D, F_, _lib.stream_ptr())
+        if rc > 0:
+            return False
+        _lib.check(rc, "layer_fold")
+        if Wp is not None:
+            self.Wp = Wp
+        self.Wp_f, self.Wfc_f, self.log_a32 = Wp_f, Wfc_f, la
+        return True
+
     def prepare(self) -> "LayerWeights":
+        if self._fold_launch():
+            return self
         self.Wp_f = fold_colscale(self.Wp, self.wn1)
         self.Wfc_f = fold_colscale(self.Wfc, self.wn2)
         self.log_a32 = self.log_a.float().contiguous()
