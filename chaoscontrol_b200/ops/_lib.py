@@ -39,6 +39,15 @@ class GemmArgs(C.Structure):
     ]
 
 
+class LayerArgs(C.Structure):
+    """``CcbLayerArgs`` of ``csrc/layer.cu``."""
+    _fields_ = [("B", i64), ("T", i64), ("D", i64), ("F", i64), ("eps", f32), ("grad_bf16", i64)] + [
+        (n, vp) for n in ("Wp_f", "Wfc_f", "Wo", "Wproj", "Wp", "Wfc", "wn1", "wn2", "log_a", "h0",
+                          "x", "ss1", "P", "y", "h", "x2", "u", "f", "ss2", "x3", "ss3", "hT",
+                          "dx3", "dhT", "ws16", "ws32", "dx", "dWp", "dWo", "dWfc", "dWproj", "dwn1", "dwn2",
+                          "dlog_a", "dh0")]
+
+
 (EPI_STORE, EPI_ROWSCALE, EPI_ROWSCALE_SILU, EPI_RESID_SS, EPI_DSILU, EPI_RMSBWD, EPI_LSE_PART,
  EPI_CE_GRAD) = range(8)
 
@@ -84,6 +93,10 @@ _SIGS = {
     "ccb_fold_colscale": ([vp, vp, vp, i64, i64, vp], C.c_int),
     "ccb_row_ss": ([vp, vp, vp, vp, i64, i64, vp], C.c_int),
     "ccb_layer_fold": ([vp] * 12 + [i64, i64, vp], C.c_int),
+    "ccb_layer_forward": ([C.POINTER(LayerArgs), vp], C.c_int),
+    "ccb_layer_backward": ([C.POINTER(LayerArgs), vp], C.c_int),
+    "ccb_layer_bwd_ws16": ([i64, i64, i64], i64),
+    "ccb_layer_bwd_ws32": ([i64, i64, i64, i64], i64),
     "ccb_rmsnorm_fwd": ([vp, vp, vp, vp, vp, vp, i64, i64, f32, vp], C.c_int),
     "ccb_rmsnorm_bwd_blocks": ([i64], i64),
     "ccb_rmsnorm_bwd": ([vp, vp, vp, vp, vp, vp, vp, i64, i64, vp], C.c_int),
@@ -161,7 +174,8 @@ def check(rc: int, what: str = "") -> None:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle of torch.cuda.current_stream(), without the Stream object built around it (a few us a launch)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def ptr(t: Optional[torch.Tensor]) -> Optional[int]:

@@ -25,6 +25,7 @@ is how the algebra is tested against autograd of the plain module.
 """
 from __future__ import annotations
 
+import ctypes as C
 from dataclasses import dataclass, field
 from typing import Optional
 
@@ -259,6 +260,28 @@ class LayerCtx:
 
 
 @dataclass
+class PackedCtx:
+    """The same activations of a layer that ran as one native call: all bf16 ones in ``acts``."""
+    x: torch.Tensor
+    ss1: torch.Tensor
+    acts: torch.Tensor      # P [R,4D] | y [R,D] | h [R,D] | x2 [R,D] | u [R,F] | f [R,F]
+    ss2: torch.Tensor
+    h0: Optional[torch.Tensor]
+    F: int
+
+    def _part(self, start: int, width: int) -> torch.Tensor:
+        R = self.x.shape[0]
+        return self.acts[start * R:(start + width) * R].view(R, width)
+
+    P = property(lambda c: c._part(0, 4 * c.x.shape[1]))
+    y = property(lambda c: c._part(4 * c.x.shape[1], c.x.shape[1]))
+    h = property(lambda c: c._part(5 * c.x.shape[1], c.x.shape[1]))
+    x2 = property(lambda c: c._part(6 * c.x.shape[1], c.x.shape[1]))
+    u = property(lambda c: c._part(7 * c.x.shape[1], c.F))
+    f = property(lambda c: c._part(7 * c.x.shape[1] + c.F, c.F))
+
+
+@dataclass
 class LayerGrads:
     dWp: torch.Tensor       # [4D, D] fp32 (or the grad_dtype asked for)
     dWo: torch.Tensor
@@ -297,9 +320,92 @@ def _scan_bwd(P, log_a32, h0, h, dy, dhT, rowss, inv_dim, eps, B, T, D, want_dh0
     return dP.to(P.dtype), grads[1], (grads[2] if len(grads) > 2 else None)
 
 
+def _plain_bf16(*ts) -> bool:
+    return all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() for t in ts)
+
+
+def _plain_f32(*ts) -> bool:
+    return all(t is None or (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()) for t in ts)
+
+
+def _layer_args(w: LayerWeights, B: int, T: int, D: int, F_: int, x, ss1, h0, acts, ss2) -> "_lib.LayerArgs":
+    a = _lib.LayerArgs()
+    a.B, a.T, a.D, a.F, a.eps = B, T, D, F_, EPS
+    a.Wp_f, a.Wfc_f, a.Wo, a.Wproj = w.Wp_f.data_ptr(), w.Wfc_f.data_ptr(), w.Wo.data_ptr(), w.Wproj.data_ptr()
+    a.log_a, a.h0 = w.log_a32.data_ptr(), _lib.ptr(h0)
+    a.x, a.ss1, a.ss2 = x.data_ptr(), ss1.data_ptr(), ss2.data_ptr()
+    rd = 2 * x.numel()
+    a.P = p = acts.data_ptr()
+    a.y, a.h, a.x2, a.u = p + 4 * rd, p + 5 * rd, p + 6 * rd, p + 7 * rd
+    a.f = p + 7 * rd + 2 * x.shape[0] * F_
+    return a
+
+
+def _layer_forward_native(x, ss1, w, B, T, h0, save):
+    """:func:`layer_forward` as one native call; None when an operand is not plain."""
+    R, D = x.shape
+    F_ = w.Wfc.shape[0]
+    if not (R == B * T and R > 0 and D % 8 == 0 and F_ % 8 == 0 and w.log_a32.dim() == 1 and
+            _plain_bf16(x, w.Wp_f, w.Wfc_f, w.Wo, w.Wproj) and _plain_f32(ss1, w.log_a32, h0)):
+        return None
+    dev = x.device
+    acts = torch.empty(R * (7 * D + 2 * F_), dtype=torch.bfloat16, device=dev)
+    x3 = torch.empty_like(x)
+    ss2 = torch.empty(R, dtype=torch.float32, device=dev)
+    ss3 = torch.empty(R, dtype=torch.float32, device=dev)
+    hT = torch.empty(B, D, dtype=torch.float32, device=dev)
+    a = _layer_args(w, B, T, D, F_, x, ss1, h0, acts, ss2)
+    if not save:
+        a.h = None
+    a.x3, a.ss3, a.hT = x3.data_ptr(), ss3.data_ptr(), hT.data_ptr()
+    _lib.check(_lib.lib().ccb_layer_forward(C.byref(a), _lib.stream_ptr()), "layer_forward")
+    return x3, ss3, hT, (PackedCtx(x, ss1, acts, ss2, h0, F_) if save else None)
+
+
+_GRAD_KEYS = ("dWp", "dWo", "dWfc", "dWproj", "dwn1", "dwn2", "dlog_a")
+
+
+def _layer_backward_native(dx3, ctx, w, B, T, dhT, want_dh0, outs, grad_dtype):
+    """:func:`layer_backward` as one native call; None when an operand is not plain."""
+    R, D = ctx.x.shape
+    F_ = ctx.F
+    if not (_plain_bf16(dx3, w.Wp_f, w.Wfc_f, w.Wo, w.Wproj, w.Wp, w.Wfc, w.wn1, w.wn2) and
+            _plain_f32(w.log_a32, dhT) and dx3.shape == ctx.x.shape):
+        return None
+    dev = dx3.device
+    if outs:
+        if grad_dtype != torch.float32 or any(k not in outs for k in _GRAD_KEYS) or not _plain_f32(
+                *(outs[k] for k in _GRAD_KEYS)):
+            return None
+        g = [outs[k] for k in _GRAD_KEYS]
+    elif grad_dtype in (torch.float32, torch.bfloat16):
+        sizes = (4 * D * D, D * D, F_ * D, D * F_, D, D, D)
+        flat = torch.empty(sum(sizes), dtype=grad_dtype, device=dev).split(sizes)
+        g = [flat[0].view(4 * D, D), flat[1].view(D, D), flat[2].view(F_, D), flat[3].view(D, F_), *flat[4:]]
+    else:
+        return None
+    L = _lib.lib()
+    ws16 = torch.empty(L.ccb_layer_bwd_ws16(R, D, F_), dtype=torch.bfloat16, device=dev)
+    ws32 = torch.empty(L.ccb_layer_bwd_ws32(B, T, D, F_), dtype=torch.float32, device=dev)
+    dx = torch.empty_like(dx3)
+    dh0 = torch.empty(B, D, dtype=torch.float32, device=dev) if want_dh0 else None
+    a = _layer_args(w, B, T, D, F_, ctx.x, ctx.ss1, ctx.h0, ctx.acts, ctx.ss2)
+    a.grad_bf16 = int(grad_dtype == torch.bfloat16)
+    a.Wp, a.Wfc, a.wn1, a.wn2 = w.Wp.data_ptr(), w.Wfc.data_ptr(), w.wn1.data_ptr(), w.wn2.data_ptr()
+    a.dx3, a.dhT, a.ws16, a.ws32 = dx3.data_ptr(), _lib.ptr(dhT), ws16.data_ptr(), ws32.data_ptr()
+    a.dx, a.dh0 = dx.data_ptr(), _lib.ptr(dh0)
+    a.dWp, a.dWo, a.dWfc, a.dWproj, a.dwn1, a.dwn2, a.dlog_a = (t.data_ptr() for t in g)
+    _lib.check(L.ccb_layer_backward(C.byref(a), _lib.stream_ptr()), "layer_backward")
+    return dx, LayerGrads(*g, dh0)
+
+
 def layer_forward(x: torch.Tensor, ss1: torch.Tensor, w: LayerWeights, B: int, T: int,
                   h0: Optional[torch.Tensor] = None, *, save: bool = True):
     """One block.  Returns ``(x3, ss3, hT, ctx)``; ``ctx`` is None when ``save`` is False."""
+    if x.is_cuda:
+        res = _layer_forward_native(x, ss1, w, B, T, h0, save)
+        if res is not None:
+            return res
     R, D = x.shape
     F_ = w.Wfc.shape[0]
     inv_d = 1.0 / D
@@ -324,6 +430,10 @@ def layer_backward(dx3: torch.Tensor, ctx: LayerCtx, w: LayerWeights, B: int, T:
     ``outs`` may map ``dWp / dWo / dWfc / dWproj / dwn1 / dwn2`` to preallocated
     fp32 tensors (views of a flat gradient buffer) that receive the results.
     """
+    if isinstance(ctx, PackedCtx):
+        res = _layer_backward_native(dx3, ctx, w, B, T, dhT, want_dh0, outs, grad_dtype)
+        if res is not None:
+            return res
     R, D = ctx.x.shape
     inv_d = 1.0 / D
     o = outs or {}

@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from chaoscontrol_b200.ops import trunk as T
+from chaoscontrol_b200.ops import trunk
 
 pytestmark = pytest.mark.gpu
 
@@ -18,9 +18,9 @@ def test_layer_fold(D, F, packed, shift):
     fc = rnd(F * D + shift)[shift:].view(F, D)
     rest = dict(Wo=rnd(D, D), Wfc=fc, Wproj=rnd(D, F), wn1=wn1, wn2=wn2, log_a=log_a)
     if packed:
-        w = T.LayerWeights(Wp=Wp, **rest).prepare()
+        w = trunk.LayerWeights(Wp=Wp, **rest).prepare()
     else:
-        w = T.LayerWeights.from_parts(*(t.clone() for t in Wp.split(D, 0)), **rest)
+        w = trunk.LayerWeights.from_parts(*(t.clone() for t in Wp.split(D, 0)), **rest)
     assert torch.equal(w.Wp, Wp)
     assert torch.equal(w.Wp_f, (Wp.float() * wn1.float()).bfloat16())
     assert torch.equal(w.Wfc_f, (fc.float() * wn2.float()).bfloat16())
@@ -33,8 +33,47 @@ def test_row_ss(R, D):
     a, b = (torch.randn(R, D, generator=g, device="cuda").bfloat16() for _ in range(2))
     tol = (D + 1) * 2.0 ** -24                       # D products added in fp32, all of one sign
     ref = a.double().square().sum(-1)
-    assert ((T.row_ss(a).double() - ref).abs() <= tol * ref).all()
-    s, ss = T.add_row_ss(a, b)
+    assert ((trunk.row_ss(a).double() - ref).abs() <= tol * ref).all()
+    s, ss = trunk.add_row_ss(a, b)
     assert torch.equal(s, a + b)
     ref = (a + b).double().square().sum(-1)
     assert ((ss.double() - ref).abs() <= tol * ref).all()
+
+
+@pytest.mark.parametrize("B,T,D,F", [(1, 1, 64, 128), (3, 70, 128, 256), (2, 65, 192, 768), (5, 200, 256, 512),
+                                     (2, 129, 320, 640), (1, 300, 512, 1024)])
+@pytest.mark.parametrize("state", [False, True])
+def test_native_layer_matches_separate_launches(B, T, D, F, state, monkeypatch):
+    """One native call issues the launches of the step-by-step sequence: the same bits."""
+    g = torch.Generator(device="cuda").manual_seed(D + T)
+    rnd = lambda *s, k=1.0: (torch.randn(*s, generator=g, device="cuda") * k)
+    w = _weights(rnd, D, F)
+    x, dx3 = rnd(B * T, D).bfloat16(), rnd(B * T, D).bfloat16()
+    h0, dhT = (rnd(B, D), rnd(B, D)) if state else (None, None)
+    ss = trunk.row_ss(x)
+    res = []
+    for native in (True, False):
+        if not native:
+            monkeypatch.setattr(trunk, "_layer_forward_native", lambda *a, **k: None)
+        x3, ss3, hT, c = trunk.layer_forward(x, ss, w, B, T, h0)
+        assert isinstance(c, trunk.PackedCtx) == native
+        x3n, ss3n, hTn, none = trunk.layer_forward(x, ss, w, B, T, h0, save=False)
+        assert none is None and torch.equal(x3, x3n) and torch.equal(hT, hTn)
+        row = [x3, ss3, hT]
+        for dt in (torch.float32, torch.bfloat16):
+            dx, gr = trunk.layer_backward(dx3, c, w, B, T, dhT, want_dh0=state, grad_dtype=dt)
+            row += [dx, gr.dWp, gr.dWo, gr.dWfc, gr.dWproj, gr.dwn1, gr.dwn2, gr.dlog_a.to(dt)]
+            row += [gr.dh0] if state else []
+        outs = {k: torch.empty_like(getattr(gr, k), dtype=torch.float32)
+                for k in ("dWp", "dWo", "dWfc", "dWproj", "dwn1", "dwn2", "dlog_a")}
+        trunk.layer_backward(dx3, c, w, B, T, dhT, outs=outs)
+        res.append(row + list(outs.values()))
+    assert len(res[0]) == len(res[1])
+    for i, (a, b) in enumerate(zip(*res)):
+        assert a.dtype == b.dtype and torch.equal(a, b), i
+
+
+def _weights(rnd, D, F):
+    lin = lambda n, k: rnd(n, k, k=k ** -0.5).bfloat16()
+    return trunk.LayerWeights(Wp=lin(4 * D, D), Wo=lin(D, D), Wfc=lin(F, D), Wproj=lin(D, F), wn1=rnd(D).bfloat16(),
+                          wn2=rnd(D).bfloat16(), log_a=rnd(D).bfloat16()).prepare()
