@@ -237,9 +237,9 @@ embed_bwd_join_kernel(const long long* __restrict__ first_pos, const long long* 
 }
 
 // ---------------------------------------------------------------------------
-// Split-K reduction.  out[n,k] (+)= scale * colscale[k] * sum_s part[s,n,k], stored as fp32 or bf16
+// Split-K reduction.  out[n,k] (+)= colscale[k] * sum_s part[s,n,k], stored as fp32 or bf16
 // (the parameter's own dtype, so no cast pass follows); when W is given also emits per-row-block
-// partial column sums of scale * sum[n,k] * W[n,k] (the gradient of an RMSNorm weight folded into W),
+// partial column sums of sum[n,k] * W[n,k] (the gradient of an RMSNorm weight folded into W),
 // reduced by a second tiny kernel so the result is deterministic.
 //
 // Bound by the latency of the partials' loads (they sit in L2): a weight gradient of the trunk is only
@@ -267,7 +267,7 @@ template <int G, typename OT>
 __global__ void __launch_bounds__(128 * G)
 splitk_tile_kernel(const float* __restrict__ part, int S, long long split_stride, int N, int K,
                    const __nv_bfloat16* __restrict__ colscale, const __nv_bfloat16* __restrict__ W,
-                   OT* __restrict__ out, const float* __restrict__ scale, float* __restrict__ colpart) {
+                   OT* __restrict__ out, float* __restrict__ colpart) {
   __shared__ float4 join[G > 1 ? (G - 1) * 128 : 1];
   __shared__ float4 colj[128];
   const int slot = threadIdx.x & 127, g = threadIdx.x >> 7;
@@ -302,10 +302,6 @@ splitk_tile_kernel(const float* __restrict__ part, int S, long long split_stride
   if (g == 0) {
     float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
     if (ok) {
-      if (scale != nullptr) {
-        const float sc = __ldg(scale);
-        acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc;
-      }
       if (W != nullptr) {
         const uint2 q = __ldg(reinterpret_cast<const uint2*>(W + o));
         const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y);
@@ -339,10 +335,8 @@ template <typename OT>
 __global__ void splitk_reduce_kernel(const float* __restrict__ part, int S, long long split_stride,
                                      int N, int K, const __nv_bfloat16* __restrict__ colscale,
                                      const __nv_bfloat16* __restrict__ W, OT* __restrict__ out,
-                                     int accumulate, const float* __restrict__ scale,
-                                     float* __restrict__ colpart) {
+                                     int accumulate, float* __restrict__ colpart) {
   const int n0 = blockIdx.x * SPK_ROWS;
-  const float sc = scale ? *scale : 1.f;
   for (int k = threadIdx.x; k < K; k += blockDim.x) {
     const float cs = colscale ? __bfloat162float(colscale[k]) : 1.f;
     float cacc = 0.f;
@@ -360,7 +354,6 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int S, long
           s += v0; s += v1; s += v2; s += v3;
         }
         for (; sp < S; ++sp) s += pp[(long long)sp * split_stride];
-        s *= sc;
         const long long o = (long long)n * K + k;
         if (W) cacc += s * __bfloat162float(W[o]);
         const float val = s * cs;
@@ -988,7 +981,7 @@ static int launch_colsum(const float* part, int64_t NB, int64_t K, void* out, in
 template <typename OT>
 static int launch_splitk(const float* part, int64_t S, int64_t split_stride, int64_t N, int64_t K,
                          const __nv_bfloat16* colscale, const __nv_bfloat16* W, OT* out, int64_t accumulate,
-                         const float* scale, float* colpart, cudaStream_t s) {
+                         float* colpart, cudaStream_t s) {
   const unsigned nb = (unsigned)((N + SPK_ROWS - 1) / SPK_ROWS);
   const uintptr_t wide = (uintptr_t)part | (uintptr_t)out;                  // 16-byte accesses
   const uintptr_t half = (uintptr_t)colscale | (uintptr_t)W;                // 8-byte accesses
@@ -997,30 +990,30 @@ static int launch_splitk(const float* part, int64_t S, int64_t split_stride, int
   if (tile) {
     const dim3 grid(nb, (unsigned)((K + SPK_COLS - 1) / SPK_COLS));
     // groups: each keeps at least four partials, so that its loads are in flight together
-    if (S <= 4) splitk_tile_kernel<1, OT><<<grid, 128, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out, scale, colpart);
-    else if (S <= 8) splitk_tile_kernel<2, OT><<<grid, 256, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out, scale, colpart);
-    else if (S <= 24) splitk_tile_kernel<4, OT><<<grid, 512, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out, scale, colpart);
-    else splitk_tile_kernel<8, OT><<<grid, 1024, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out, scale, colpart);
+    if (S <= 4) splitk_tile_kernel<1, OT><<<grid, 128, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out, colpart);
+    else if (S <= 8) splitk_tile_kernel<2, OT><<<grid, 256, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out, colpart);
+    else if (S <= 24) splitk_tile_kernel<4, OT><<<grid, 512, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out, colpart);
+    else splitk_tile_kernel<8, OT><<<grid, 1024, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out, colpart);
   } else {
     splitk_reduce_kernel<OT><<<nb, 256, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out,
-                                                (int)accumulate, scale, colpart);
+                                                (int)accumulate, colpart);
   }
   CCB_CHECK_LAUNCH("splitk_reduce");
   return 0;
 }
 
-// `out` and `colsum_out` are fp32, or bf16 with out_bf16; `scale` is an optional device scalar.
+// `out` and `colsum_out` are fp32, or bf16 with out_bf16.
 extern "C" int ccb_splitk_reduce_as(const float* part, int64_t S, int64_t split_stride, int64_t N, int64_t K,
                                     const void* colscale, const void* W, void* out, int64_t out_bf16,
-                                    int64_t accumulate, const float* scale, float* colpart, void* colsum_out,
+                                    int64_t accumulate, float* colpart, void* colsum_out,
                                     int64_t colsum_accumulate, void* stream) {
   if (N <= 0 || K <= 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   const __nv_bfloat16* cs = (const __nv_bfloat16*)colscale;
   const __nv_bfloat16* w = (const __nv_bfloat16*)W;
   float* cp = W ? colpart : nullptr;
-  const int rc = out_bf16 ? launch_splitk(part, S, split_stride, N, K, cs, w, (__nv_bfloat16*)out, accumulate, scale, cp, s)
-                          : launch_splitk(part, S, split_stride, N, K, cs, w, (float*)out, accumulate, scale, cp, s);
+  const int rc = out_bf16 ? launch_splitk(part, S, split_stride, N, K, cs, w, (__nv_bfloat16*)out, accumulate, cp, s)
+                          : launch_splitk(part, S, split_stride, N, K, cs, w, (float*)out, accumulate, cp, s);
   if (rc) return rc;
   if (cp && colsum_out)
     return launch_colsum(cp, (N + SPK_ROWS - 1) / SPK_ROWS, K, colsum_out, (int)out_bf16, colsum_accumulate, s);
@@ -1031,7 +1024,7 @@ extern "C" int ccb_splitk_reduce(const float* part, int64_t S, int64_t split_str
                                  int64_t K, const void* colscale, const void* W, float* out,
                                  int64_t accumulate, float* colpart, float* colsum_out,
                                  int64_t colsum_accumulate, void* stream) {
-  return ccb_splitk_reduce_as(part, S, split_stride, N, K, colscale, W, out, 0, accumulate, nullptr, colpart,
+  return ccb_splitk_reduce_as(part, S, split_stride, N, K, colscale, W, out, 0, accumulate, colpart,
                               colsum_out, colsum_accumulate, stream);
 }
 

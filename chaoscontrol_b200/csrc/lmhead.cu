@@ -75,6 +75,7 @@ struct LmHeadArgs {
   const long long* targets; // [R]
   const float* rowweight;   // [R] or null
   float gscale;             // d loss / d (per-row CE), e.g. 1/R
+  const float* gscale_dev;  // optional device scalar that multiplies gscale (an upstream gradient)
   float* lse;               // [R] natural-log lse (out in LSE/TRAIN, in for DW)
   float* loss;              // [R] per-row CE (out, LSE/TRAIN)
   float* entropy;           // [R] softmax entropy in nats (out, LSE; optional)
@@ -108,7 +109,7 @@ __device__ __forceinline__ float ex2f(float x) {
   return y;
 }
 
-// DEEP = 1 (one-sweep training only): the unit's X tile is the logits MMA's A operand from tensor
+// DEEP = 1 (single-sweep kernels: one-sweep training, training with a given lse, dW): the unit's X tile is the logits MMA's A operand from tensor
 // memory instead of shared memory, the 64 KiB it occupied become a THIRD W' stage, and one logits
 // buffer (handed back as soon as the epilogue holds it in registers) makes room for X in tensor
 // memory.  With two stages a W' tile is pinned from its logits MMA until the dX MMA of the same tile
@@ -175,8 +176,7 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
   // The same was tried for one-sweep training (X in [128,256), ONE logits buffer released as soon
   // as the epilogue holds it in registers, dX in [256,512)): 7.95 -> 8.10 ms, i.e. no gain once
   // the second MMA shares the pipe, so training keeps A in shared memory and two logits buffers.
-  static_assert(DEEP == 0 || MODE == MODE_TRAIN1 || MODE == MODE_DW,
-                "the deep-ring variant exists for one-sweep training and for the dW kernel");
+  static_assert(DEEP == 0 || MODE != MODE_LSE, "the deep-ring variant exists for the single-sweep training kernels");
   // DEEP dW kernel: the logits tile is computed TRANSPOSED (lanes = vocabulary rows of the unit's W'
   // tile, which is the A operand and therefore can live in tensor memory; columns = token rows of the
   // streamed X tile), so that the dW kernel gets the same three-stage ring as the dX kernel.
@@ -190,7 +190,7 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
   auto stage_ptr = [&](int st) -> uint8_t* {
     return smem + (st < 2 ? LH_OFF_STG + st * LH_TILE : LH_OFF_RES);
   };
-  const int n_sweeps = (MODE == MODE_TRAIN && !p.skip_lse) ? 2 : 1;
+  const int n_sweeps = (MODE == MODE_TRAIN && DEEP == 0 && !p.skip_lse) ? 2 : 1;
 
   if (warp == 0) {
     // =========================== TMA producer ================================
@@ -360,6 +360,7 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
     const int row_in_tile = q * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     float* xchg = reinterpret_cast<float*>(smem + LH_OFF_X);     // [PARTS][128]
+    const float gscale = p.gscale_dev ? p.gscale * __ldg(p.gscale_dev) : p.gscale;
     uint32_t n_d1 = 0, n_g = 0, n_d2 = 0, n_x = 0, n_xt = 0;
     bool ok = true;
     // Every wait below is made warp-uniform, so the warp-collective TMEM loads
@@ -419,7 +420,7 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         c1 = rs * LOG2E;
         tgt = row_ok ? (int)p.targets[r] : -1;
         const float w = (row_ok && p.rowweight) ? p.rowweight[r] : 1.f;
-        gs = row_ok ? p.gscale * w * rs : 0.f;
+        gs = row_ok ? gscale * w * rs : 0.f;
         if (need_lse) c2 = row_ok ? p.lse[r] * LOG2E : 0.f;
       };
       if (MODE != MODE_DW) load_row(unit, MODE == MODE_TRAIN && p.skip_lse);
@@ -484,7 +485,7 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         };
         auto scale_of = [&](const RawRow& x, float& rsv) -> float {
           rsv = p.rowss ? rsqrtf(x.ss * p.inv_dim + p.eps) : 1.f;
-          return p.gscale * x.w * rsv;
+          return gscale * x.w * rsv;
         };
         RawRow wraw = {0.f, INFINITY, 0.f, -1}, graw[NG];
         if (writer) wraw = fetch_raw(inner0 * LH_ROWS + row_in_tile);
@@ -916,9 +917,10 @@ static int launch_lmhead_p(const void* X, const void* W, LmHeadArgs& a, cudaStre
 template <int MODE>
 static int launch_lmhead(const void* X, const void* W, LmHeadArgs& a, cudaStream_t stream) {
   const int parts = g_lh_parts ? g_lh_parts : (MODE == MODE_LSE ? 4 : 2);
-  if ((MODE == MODE_TRAIN1 || MODE == MODE_DW) && g_lh_deep) {
-    // the variant is instantiated for these two modes only
-    constexpr int MD = (MODE == MODE_DW) ? MODE_DW : MODE_TRAIN1;
+  // Training with the forward's lse is one sweep as well and takes the same three-stage ring
+  // (65 536 rows, V = 16 384: loss forward and backward 2.84 -> 2.62 ms; the two-stage kernel took 1.13 of it).
+  if (MODE != MODE_LSE && (MODE != MODE_TRAIN || a.skip_lse) && g_lh_deep) {
+    constexpr int MD = (MODE == MODE_LSE) ? MODE_TRAIN1 : MODE;      // not instantiated for scoring
     return parts == 2 ? launch_lmhead_p<MD, 2, 1>(X, W, a, stream) : launch_lmhead_p<MD, 4, 1>(X, W, a, stream);
   }
   return parts == 2 ? launch_lmhead_p<MODE, 2>(X, W, a, stream)
@@ -989,13 +991,14 @@ extern "C" int ccb_lmhead_lse(const void* X, const void* W, const float* rowss, 
 // 2 = one sweep with a fixed per-row reference (MODE_TRAIN1), lse[] is written.
 extern "C" int ccb_lmhead_train(const void* X, const void* W, const float* rowss, float eps,
                                 const int64_t* targets, const float* rowweight, float gscale,
-                                float* lse, int64_t lse_is_input, float* loss, void* dX, int64_t R,
+                                const float* gscale_dev, float* lse, int64_t lse_is_input, float* loss, void* dX, int64_t R,
                                 int64_t V, int64_t D, void* stream) {
   LmHeadArgs a = {};
   int rc = lmhead_common(a, R, V, D, rowss, eps, targets);
   if (rc) return rc < 0 ? rc : 0;
   a.rowweight = rowweight;
   a.gscale = gscale;
+  a.gscale_dev = gscale_dev;
   a.lse = lse;
   a.skip_lse = lse_is_input == 1 ? 1 : 0;
   a.loss = loss;
@@ -1009,7 +1012,7 @@ extern "C" int ccb_lmhead_train(const void* X, const void* W, const float* rowss
 // dWpart[row_chunks, V, D] fp32: partial gradients of W' = W_lm * w_norm.
 extern "C" int ccb_lmhead_dw(const void* X, const void* W, const float* rowss, float eps,
                              const int64_t* targets, const float* rowweight, float gscale,
-                             const float* lse, float* dWpart, int64_t row_chunks, int64_t R,
+                             const float* gscale_dev, const float* lse, float* dWpart, int64_t row_chunks, int64_t R,
                              int64_t V, int64_t D, void* stream) {
   LmHeadArgs a = {};
   int rc = lmhead_common(a, R, V, D, rowss, eps, targets);
@@ -1023,6 +1026,7 @@ extern "C" int ccb_lmhead_dw(const void* X, const void* W, const float* rowss, f
                      (long long)row_chunks, a.row_chunks);
   a.rowweight = rowweight;
   a.gscale = gscale;
+  a.gscale_dev = gscale_dev;
   a.lse = const_cast<float*>(lse);
   a.dWpart = dWpart;
   a.X = (const __nv_bfloat16*)X;

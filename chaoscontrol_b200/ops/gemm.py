@@ -110,13 +110,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
 def gemm_lm(x: torch.Tensor, w: torch.Tensor, *, epi: int, targets: torch.Tensor,
             rowss: Optional[torch.Tensor], inv_dim: float, eps: float, lse: Optional[torch.Tensor] = None,
             rowweight: Optional[torch.Tensor] = None, alpha: float = 1.0,
+            alpha_dev: Optional[torch.Tensor] = None,
             out: Optional[torch.Tensor] = None, zt_out: Optional[torch.Tensor] = None):
     """LM-head epilogues on ``logits = rs * (x @ w.T)`` (``x`` ``[R, D]``, ``w`` ``[V, D]``, bf16, CUDA).
 
     ``EPI_LSE_PART`` returns ``(partials [2 * ceil(V / 256), R, 2] fp32, zt [R])``: log2-domain
     ``(max, sum)`` per half tile and the target logit; no logits are written.
     ``EPI_CE_GRAD`` returns the bf16 ``[R, V]`` gradient of the summed, ``alpha * rowweight``-weighted
-    cross-entropy w.r.t. the un-scaled GEMM output, and fills ``zt_out`` with the per-row CE.
+    cross-entropy w.r.t. the un-scaled GEMM output (``alpha_dev``, a one-element fp32 tensor, multiplies
+    ``alpha`` on the device), and fills ``zt_out`` with the per-row CE.
     """
     R, D = x.shape
     V = w.shape[0]
@@ -128,6 +130,7 @@ def gemm_lm(x: torch.Tensor, w: torch.Tensor, *, epi: int, targets: torch.Tensor
     args.epi = epi
     args.alpha, args.beta, args.inv_dim, args.eps = alpha, 0.0, inv_dim, eps
     args.rowss = _lib.ptr(rowss)
+    args.dscale_a = _lib.ptr(alpha_dev)
     t = targets.reshape(-1)
     if t.dtype != torch.int64:
         t = t.long()

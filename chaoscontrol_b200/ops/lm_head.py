@@ -18,8 +18,8 @@ from . import gemm as G
 from ._lib import f32, i64, vp
 
 _lib.register_sig("ccb_lmhead_lse", [vp, vp, vp, f32, vp, vp, vp, vp, i64, i64, i64, vp])
-_lib.register_sig("ccb_lmhead_train", [vp, vp, vp, f32, vp, vp, f32, vp, i64, vp, vp, i64, i64, i64, vp])
-_lib.register_sig("ccb_lmhead_dw", [vp, vp, vp, f32, vp, vp, f32, vp, vp, i64, i64, i64, i64, vp])
+_lib.register_sig("ccb_lmhead_train", [vp, vp, vp, f32, vp, vp, f32, vp, vp, i64, vp, vp, i64, i64, i64, vp])
+_lib.register_sig("ccb_lmhead_dw", [vp, vp, vp, f32, vp, vp, f32, vp, vp, vp, i64, i64, i64, i64, vp])
 
 EPS = 1e-6
 
@@ -62,7 +62,7 @@ def general_row_chunk(R: int) -> int:
     return min(R, 128 * sms)
 
 
-def _train_general(x, rowss, W_f, t, gscale, rowweight, eps, lse, want_dw=True):
+def _train_general(x, rowss, W_f, t, gscale, rowweight, eps, lse, want_dw=True, gscale_dev=None):
     """Chunked LM-head backward from GEMM epilogues.  Per row chunk: ``g = (softmax - onehot) *
     scale`` is produced by the logits GEMM's epilogue as a bf16 ``[rows, V]`` tile (bounded by the
     chunk, never the full ``[R, V]``), then ``dX = RMSNorm-backward(g @ W')`` and
@@ -85,7 +85,7 @@ def _train_general(x, rowss, W_f, t, gscale, rowweight, eps, lse, want_dw=True):
         ssc = rowss[r0:r1] if rowss is not None else None
         g = G.gemm_lm(xc, W_f, epi=G.EPI_CE_GRAD, targets=t[r0:r1], rowss=ssc, inv_dim=1.0 / D, eps=eps,
                       lse=lse[r0:r1], rowweight=rowweight[r0:r1] if rowweight is not None else None,
-                      alpha=gscale, out=gbuf[: r1 - r0], zt_out=loss[r0:r1])
+                      alpha=gscale, alpha_dev=gscale_dev, out=gbuf[: r1 - r0], zt_out=loss[r0:r1])
         if rowss is not None:
             G.gemm(g, W_f, b_mn=True, epi=G.EPI_RMSBWD, r1=xc, rowss=ssc, inv_dim=1.0 / D, eps=eps,
                    out=dX[r0:r1])
@@ -222,8 +222,11 @@ ONE_SWEEP = True      # module switch: lse + dX in one vocabulary sweep (see lm_
 def lm_head_train(x, rowss, W_f, targets, *, gscale: float, rowweight=None, eps: float = EPS,
                   row_chunks: Optional[int] = None, lse: Optional[torch.Tensor] = None,
                   one_sweep: Optional[bool] = None, allow_materialized: bool = False,
-                  want_dw: bool = True):
+                  want_dw: bool = True, gscale_dev: Optional[torch.Tensor] = None):
     """Loss and both gradients.  Returns ``(loss_rows, lse, dX bf16, dW_f_partials fp32 [C,V,D])``.
+
+    ``gscale_dev``: a one-element fp32 tensor that multiplies ``gscale`` (the gradient that
+    arrives from further up), read on the device.
 
     ``want_dw=False`` skips the weight-gradient kernel and returns ``None`` in its
     place: test-time training adapts recurrence parameters only and needs ``dX``
@@ -244,9 +247,11 @@ def lm_head_train(x, rowss, W_f, targets, *, gscale: float, rowweight=None, eps:
     R, D = x.shape
     V = W_f.shape[0]
     if (not fused_supported(x, W_f) or (_few_rows(R) and one_sweep is None)) and general_supported(x, W_f):
-        return _train_general(x, rowss, W_f, _prep(x, rowss, W_f, targets), gscale, rowweight, eps, lse, want_dw)
+        return _train_general(x, rowss, W_f, _prep(x, rowss, W_f, targets), gscale, rowweight, eps, lse, want_dw, gscale_dev)
     if not fused_supported(x, W_f):
         _refuse_unless_allowed(x, W_f, allow_materialized, "lm_head_train")
+        if gscale_dev is not None:
+            gscale = gscale * float(gscale_dev)
         lr, lse, dX, dW = lm_head_reference(x, rowss, W_f, targets, gscale=gscale,
                                             rowweight=rowweight, eps=eps)
         return lr, lse, dX.to(x.dtype), dW.unsqueeze(0)
@@ -259,7 +264,7 @@ def lm_head_train(x, rowss, W_f, targets, *, gscale: float, rowweight=None, eps:
     dX = torch.empty_like(x)
     L = _lib.lib()
     _lib.check(L.ccb_lmhead_train(x.data_ptr(), W_f.data_ptr(), _lib.ptr(rowss), eps, t.data_ptr(),
-                                  _lib.ptr(rowweight), gscale, lse.data_ptr(),
+                                  _lib.ptr(rowweight), gscale, _lib.ptr(gscale_dev), lse.data_ptr(),
                                   1 if lse_given else (2 if (ONE_SWEEP if one_sweep is None else one_sweep) else 0),
                                   loss.data_ptr(), dX.data_ptr(), R, V, D, _lib.stream_ptr()),
                "lmhead_train")
@@ -268,6 +273,6 @@ def lm_head_train(x, rowss, W_f, targets, *, gscale: float, rowweight=None, eps:
     C = row_chunks or default_row_chunks(R, V)
     part = torch.empty(C, V, D, dtype=torch.float32, device=dev)
     _lib.check(L.ccb_lmhead_dw(x.data_ptr(), W_f.data_ptr(), _lib.ptr(rowss), eps, t.data_ptr(),
-                               _lib.ptr(rowweight), gscale, lse.data_ptr(), part.data_ptr(), C, R, V,
+                               _lib.ptr(rowweight), gscale, _lib.ptr(gscale_dev), lse.data_ptr(), part.data_ptr(), C, R, V,
                                D, _lib.stream_ptr()), "lmhead_dw")
     return loss, lse, dX, part

@@ -135,3 +135,23 @@ def test_lmhead_one_sweep_matches_two_sweeps_and_the_reference(wscale, peak, epi
         return float((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-12))
     assert rel(dX1, rdX) < 2e-2 and rel(dX1, dX2) < 2e-2, (rel(dX1, rdX), rel(dX1, dX2))
     assert rel(p1.sum(0), rdW) < 2e-2 and rel(p1.sum(0), p2.sum(0)) < 1e-2
+
+
+@pytest.mark.parametrize("R,D,V", [(4096 + 77, 256, 512), (130, 256, 1024), (301, 384, 640)])
+@pytest.mark.parametrize("up", [1.0, -0.37, 3e-6, 0.0])
+def test_upstream_gradient_scales_inside_the_kernels(R, D, V, up):
+    """Both gradients of ``up * loss`` against autograd through 32-bit logits.  The gradient tile of a row is rounded to
+    bf16 once (relative 2^-8 an element) and so are the results; the sums over the vocabulary and the rows average the
+    first out, so the 2-norm differs by less than 1e-2."""
+    from chaoscontrol_b200.kernels import fused_linear_cross_entropy
+    g = torch.Generator(device="cuda").manual_seed(R)
+    x = torch.randn(R, D, generator=g, device="cuda").bfloat16().requires_grad_(True)
+    W = (torch.randn(V, D, generator=g, device="cuda") * 0.1).bfloat16().requires_grad_(True)
+    t = torch.randint(0, V, (R,), generator=g, device="cuda")
+    gx, gW = torch.autograd.grad(fused_linear_cross_entropy(x, W, t, reduction="sum") * up, (x, W))
+    (only,) = torch.autograd.grad(fused_linear_cross_entropy(x, W.detach(), t, reduction="sum") * up, (x,))
+    xf, Wf = x.detach().float().requires_grad_(True), W.detach().float().requires_grad_(True)
+    rx, rW = torch.autograd.grad(torch.nn.functional.cross_entropy(xf @ Wf.t(), t, reduction="sum") * up, (xf, Wf))
+    assert torch.equal(only, gx)
+    for a, b in ((gx, rx), (gW, rW)):
+        assert (a.float() - b).norm() <= 1e-2 * b.norm()

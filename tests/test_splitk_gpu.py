@@ -18,19 +18,18 @@ def test_splitk_reduce(S, N, K, dt, fold):
     part = torch.randn(S, N, K, generator=g, device="cuda")
     W = torch.randn(N, K, generator=g, device="cuda").bfloat16() if fold else None
     cs = torch.randn(K, generator=g, device="cuda").bfloat16() if fold else None
-    scale = torch.randn((), generator=g, device="cuda") if fold else None
-    out, dcol = splitk_reduce(part, colscale=cs, W=W, scale=scale, out_dtype=dt)
-    p64, f = part.double(), scale.double() if fold else 1.0
+    out, dcol = splitk_reduce(part, colscale=cs, W=W, out_dtype=dt)
+    p64 = part.double()
     c64 = cs.double() if fold else torch.ones(K, device="cuda", dtype=torch.float64)
-    ref = p64.sum(0) * f * c64
+    ref = p64.sum(0) * c64
     # S + 3 roundings of fp32 on the sum of magnitudes, then the rounding of the stored type: half a unit in the
     # last place is 2^-8 of the value for bf16's 8 significant bits
     rnd = 2.0 ** -8 if dt is torch.bfloat16 else 2.0 ** -24
-    bound = (S + 3) * 2.0 ** -24 * (p64.abs().sum(0) * f * c64).abs() + rnd * ref.abs()
+    bound = (S + 3) * 2.0 ** -24 * (p64.abs().sum(0) * c64).abs() + rnd * ref.abs()
     assert out.dtype == dt and ((out.double() - ref).abs() <= bound + 1e-30).all()
     if fold:
-        terms = p64.sum(0) * f * W.double()
-        mag = (p64.abs().sum(0) * abs(f) * W.double().abs()).sum(0)
+        terms = p64.sum(0) * W.double()
+        mag = (p64.abs().sum(0) * W.double().abs()).sum(0)
         assert ((dcol.double() - terms.sum(0)).abs() <=
                 (S + N + 4) * 2.0 ** -24 * mag + rnd * terms.sum(0).abs() + 1e-30).all()
     else:
