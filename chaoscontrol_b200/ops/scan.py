@@ -172,15 +172,20 @@ class _SsmScanFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, decay, update, h0):
         B, T, D = update.shape
-        states = torch.empty(B, T, D, dtype=torch.float32, device=update.device)
         h0c = None if h0 is None else h0.float().contiguous()
+        lowp = update.dtype != torch.float32
+        # the 32-bit states are kept for backward; 16-bit results are rounded from them in the same pass
+        keep = not lowp or any(ctx.needs_input_grad)
+        states = torch.empty(B, T, D, dtype=torch.float32, device=update.device) if keep else None
+        out = torch.empty_like(update) if lowp else None
         _lib.check(_lib.lib().ccb_plain_scan_fwd(decay.data_ptr(), _DT_CODE[decay.dtype], update.data_ptr(),
-                                                 _DT_CODE[update.dtype], _lib.ptr(h0c), states.data_ptr(),
-                                                 B, T, D, _lib.stream_ptr()), "plain_scan_fwd")
-        ctx.save_for_backward(decay, states, h0c if h0c is not None else torch.empty(0))
+                                                 _DT_CODE[update.dtype], _lib.ptr(h0c), _lib.ptr(states),
+                                                 _lib.ptr(out), B, T, D, _lib.stream_ptr()), "plain_scan_fwd")
+        if keep:
+            ctx.save_for_backward(decay, states, h0c if h0c is not None else torch.empty(0))
         ctx.has_h0 = h0 is not None
         ctx.update_dtype = update.dtype
-        return states.to(update.dtype)
+        return out if lowp else states
 
     @staticmethod
     def backward(ctx, g):

@@ -197,3 +197,43 @@ def test_time_tiled_scan_keeps_infinite_states(bad):
     for a, b in zip(*out):
         assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
     assert (out[0][2][0, 3].isinf() if bad == float("inf") else out[0][2][0, 3].isnan())
+
+
+# steps: one, off and on a warp's 8 and a block's 64; channels: odd (one to a lane) and even (two), off and on 32 / 64
+@pytest.mark.parametrize("B,T,D", [(1, 1, 1), (2, 7, 33), (3, 8, 64), (1, 64, 66), (2, 65, 130), (1, 200, 31), (5, 129, 96)])
+@pytest.mark.parametrize("ddt,udt", [_COMBOS[0], _COMBOS[2], _COMBOS[3], _COMBOS[5]], ids=lambda d: str(d).replace("torch.", ""))
+@pytest.mark.parametrize("shift", [0, 1])
+def test_ssm_scan_tiles_against_64_bits(B, T, D, ddt, udt, shift):
+    """``shift``: operands that start one element off, so that no row starts on a pair's boundary.  Decays reach above
+    one and below zero and a state may be infinite: the sums are those of a serial loop."""
+    g = torch.Generator(device="cuda").manual_seed(B * T * D)
+    n = B * T * D
+    mk = lambda dt, f: f(torch.rand(n + shift, generator=g, device="cuda")).to(dt)[shift:].view(B, T, D)
+    decay, update = mk(ddt, lambda r: r * 1.5 - 0.4), mk(udt, lambda r: r - 0.5)
+    h0 = torch.randn(B, D, generator=g, device="cuda")
+    go = torch.randn(B, T, D, generator=g, device="cuda").to(udt)
+    ins = [t.detach().requires_grad_(True) for t in (decay, update, h0)]
+    out = S.ssm_scan(*ins)
+    got = torch.autograd.grad(out, ins, go)
+    with torch.no_grad():
+        assert torch.equal(S.ssm_scan(decay, update, h0), out)
+    d64, u64, h64, g64 = (t.double() for t in (decay, update, h0, go))
+    s, mag, sts, mags = h64, h64.abs(), [], []
+    for t in range(T):
+        s = d64[:, t] * s + u64[:, t]
+        mag = d64[:, t].abs() * mag + u64[:, t].abs()
+        sts.append(s); mags.append(mag)
+    rnd = {torch.float32: 2.0 ** -24, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
+    fp = (T + 4) * 2.0 ** -24                       # every step rounds once, on sums of magnitudes `mag`
+    tiny = 2.0 ** -24                               # fp16's smallest step
+    st, mg = torch.stack(sts, 1), torch.stack(mags, 1)
+    assert ((out.double() - st).abs() <= rnd[udt] * st.abs() + fp * mg + tiny).all()
+    c, cm = torch.zeros_like(h64), torch.zeros_like(h64)
+    prev, pm = torch.cat([h64[:, None], st[:, :-1]], 1), torch.cat([h64[:, None].abs(), mg[:, :-1]], 1)
+    for t in reversed(range(T)):
+        gg, gm = g64[:, t] + c, g64[:, t].abs() + cm
+        assert ((got[1][:, t].double() - gg).abs() <= rnd[udt] * gg.abs() + fp * gm + tiny).all()
+        ref = gg * prev[:, t]
+        assert ((got[0][:, t].double() - ref).abs() <= rnd[ddt] * ref.abs() + 2 * fp * gm * pm[:, t] + tiny).all()
+        c, cm = gg * d64[:, t], gm * d64[:, t].abs()
+    assert ((got[2].double() - c).abs() <= 2.0 ** -23 * c.abs() + fp * cm).all()
