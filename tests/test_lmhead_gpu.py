@@ -155,3 +155,28 @@ def test_upstream_gradient_scales_inside_the_kernels(R, D, V, up):
     assert torch.equal(only, gx)
     for a, b in ((gx, rx), (gW, rW)):
         assert (a.float() - b).norm() <= 1e-2 * b.norm()
+
+
+@pytest.mark.parametrize("nparts", [1, 15, 16, 17, 64, 65, 130])
+@pytest.mark.parametrize("M", [1, 31, 33, 300])
+def test_lse_combine_partials(nparts, M):
+    """Merging (max, sum) pairs, empty ones (sum 0 under any maximum) among them, against 64 bits: each merge rounds the
+    sum and a power of two, and log2 of the sum is taken once."""
+    g = torch.Generator(device="cuda").manual_seed(nparts * M)
+    part = torch.stack([torch.randn(nparts, M, generator=g, device="cuda") * 30,
+                        torch.rand(nparts, M, generator=g, device="cuda") * 100 + 1e-3], -1).contiguous()
+    if nparts > 1:
+        part[::3, ::2, 1] = 0.0
+        part[::3, ::2, 0] = 1e4
+        part[1, :, 1] = 5.0                      # never all empty
+    zt = torch.randn(M, generator=g, device="cuda")
+    lse, loss = torch.empty(M, device="cuda"), torch.empty(M, device="cuda")
+    _lib.check(_lib.lib().ccb_lse_combine(part.data_ptr(), nparts, M, zt.data_ptr(), lse.data_ptr(), loss.data_ptr(),
+                                          _lib.stream_ptr()), "lse_combine")
+    p64 = part.double()
+    ln2 = 0.6931471805599453
+    z = torch.where(p64[..., 1] > 0, p64[..., 0] * ln2 + p64[..., 1].clamp_min(1e-300).log(), float("-inf"))
+    ref = torch.logsumexp(z, 0)
+    tol = (nparts + 8) * 2.0 ** -23 + 2.0 ** -23 * ref.abs()
+    assert ((lse.double() - ref).abs() <= tol).all()
+    assert ((loss.double() - (ref - zt.double())).abs() <= tol + 2.0 ** -23 * zt.abs().double()).all()
