@@ -130,3 +130,41 @@ def test_layer_and_fused_norm_gpu():
     # without the producer tag the layer quantises on its own and agrees
     out2 = layer(h.detach().clone())
     assert _rel(out2, out) < 3e-2   # re-quantising the bf16-rounded row moves a few codes
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("R,K", [(1, 128), (17, 128), (9, 256), (33, 384), (8, 512), (5, 640), (100, 1024), (7, 2048)])
+@pytest.mark.parametrize("norm", [False, True])
+def test_quant_rows_segments(R, K, norm):
+    """Row quantiser at the edges of its lane and segment split: scales to rounding, codes within one step of the exact
+    quotient (e4m3 keeps 3 fraction bits: half a step is 2^-4 of the value, or 2^-10 below the smallest normal)."""
+    g = torch.Generator(device="cuda").manual_seed(R + K)
+    x = torch.randn(R, K, generator=g, device="cuda").bfloat16()
+    w = (torch.rand(K, generator=g, device="cuda") + 0.5).bfloat16() if norm else None
+    qa, inv, y = FB.quant_rows(x, norm_weight=w, want_normed=norm)
+    v = x.double()
+    if norm:
+        ri = torch.rsqrt(v.square().mean(-1, keepdim=True) + 1e-6)
+        v = v * ri * w.double()
+        assert torch.allclose(inv.double(), ri.squeeze(1), rtol=1e-5)
+        assert ((y.double() - v).abs() <= (2.0 ** -8 + 1e-5) * v.abs()).all()
+    scale = v.view(R, K // 128, 128).abs().amax(-1).clamp_min(1e-12) / 448.0
+    assert torch.allclose(qa.s_t.double().t(), scale, rtol=2e-5)
+    quo = (v.view(R, K // 128, 128) / scale.unsqueeze(-1)).view(R, K)
+    assert ((qa.q.double() - quo).abs() <= (2.0 ** -4 + 1e-4) * quo.abs() + 2.0 ** -10 * 1.001).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,K", [(8, 128), (130, 128), (129, 100), (256, 200), (384, 264), (7, 9)])
+def test_quant_blocks_edges(N, K):
+    """Ragged blocks, sizes in eights (vector kernel) and not: the transposed codes are the codes, and each is within
+    half a step of the exact quotient."""
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    w = torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    q, qt, s = FB.quant_blocks(w)
+    assert torch.equal(q.t().contiguous().view(torch.uint8), qt.view(torch.uint8))
+    nb, kb = s.shape
+    pad = torch.nn.functional.pad(w.double(), (0, kb * 128 - K, 0, nb * 128 - N)).view(nb, 128, kb, 128)
+    assert torch.allclose(s.double(), pad.abs().amax(dim=(1, 3)).clamp_min(1e-12) / 448.0, rtol=1e-6)
+    quo = (pad / s.double()[:, None, :, None]).view(nb * 128, kb * 128)[:N, :K]
+    assert ((q.double() - quo).abs() <= (2.0 ** -4 + 1e-4) * quo.abs() + 2.0 ** -10 * 1.001).all()
