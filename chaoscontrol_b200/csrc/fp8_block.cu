@@ -24,6 +24,7 @@
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "ccb_api.h"
 #include "ptx.cuh"
@@ -202,7 +203,12 @@ constexpr int FB_STAGES = 5;
 constexpr int FB_SLOTS = 4;                                  // TMEM accumulator ring (4 x 128 columns)
 constexpr int FB_EPI_WARPS = 8;
 constexpr int FB_THREADS = 64 + 32 * FB_EPI_WARPS;
-constexpr int FB_BAR_OFF = 2 * FB_STAGES * FB_STAGE;
+// bf16 results leave through shared memory and TMA stores: each epilogue warp stages its 32 rows x 64 columns
+// (128-byte rows, swizzled).  Storing them from registers, a row to a lane, cost 32 half-used sectors an
+// instruction: 65 536 x 256 x 1024 and its input gradient took 116 us, staged 101.
+constexpr int FB_STG = 32 * 128;
+constexpr int FB_STG_OFF = 2 * FB_STAGES * FB_STAGE;
+constexpr int FB_BAR_OFF = FB_STG_OFF + FB_EPI_WARPS * FB_STG;
 constexpr int FB_SMEM = 1024 + FB_BAR_OFF + 512;
 
 struct FbArgs {
@@ -212,14 +218,14 @@ struct FbArgs {
   long long sb_so, sb_sk;
   void* C;
   long long ldc;
-  int out_fp32;
+  int out_fp32, tma_store;
   const __nv_bfloat16* bias;
   int* status;
 };
 
 __global__ void __launch_bounds__(FB_THREADS, 1)
 fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                      const FbArgs p) {
+                      const __grid_constant__ CUtensorMap tmC, const FbArgs p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -304,6 +310,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const int q = warp & 3;                    // TMEM lane quadrant
     const int part = (warp - 2) >> 2;          // columns [64 * part, 64 * part + 64) of the tile
     const int row_in_tile = q * 32 + lane;
+    uint8_t* my_stage = smem + FB_STG_OFF + (warp - 2) * FB_STG;
     uint32_t n_slot = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
@@ -341,17 +348,39 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         if (lane == 0) mbar_arrive(&tempty_bar[slot]);
       }
       if (!ok) break;
-      if (row_ok) {
+      if (p.bias != nullptr) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int n = n0 + part * 64 + h * 32;
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (n + i < p.N) out[h][i] += __bfloat162float(__ldg(p.bias + n + i));
+        }
+      }
+      if (p.tma_store) {
+        if (lane == 0) tma_store_wait_read<0>();           // this warp's last store has left the staging rows
+        __syncwarp();
+        uint8_t* srow = my_stage + lane * 128;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int h = j >> 2, e = (j & 3) * 8;
+          *reinterpret_cast<uint4*>(srow + (j ^ (lane & 7)) * 16) =
+              make_uint4(pack_bf16x2(out[h][e], out[h][e + 1]), pack_bf16x2(out[h][e + 2], out[h][e + 3]),
+                         pack_bf16x2(out[h][e + 4], out[h][e + 5]), pack_bf16x2(out[h][e + 6], out[h][e + 7]));
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        const int col = n0 + part * 64, row = m0 + q * 32;
+        if (lane == 0 && col < p.N && row < p.M) {          // the store clips rows and columns past the end
+          tma_store_3d(&tmC, my_stage, col, row, 0);
+          tma_store_commit();
+        }
+      } else if (row_ok) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int n = n0 + part * 64 + h * 32;
           const int nvalid = p.N - n;
           if (nvalid <= 0) continue;
-          if (p.bias != nullptr) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (i < nvalid) out[h][i] += __bfloat162float(p.bias[n + i]);
-          }
           if (p.out_fp32) {
             float* dst = reinterpret_cast<float*>(p.C) + (long long)m * p.ldc + n;
             if (nvalid >= 32) {
@@ -384,6 +413,9 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
       }
     }
+    // this warp's stores must have left shared memory and landed
+    if (p.tma_store && lane == 0) tma_store_wait_all<0>();
+    __syncwarp();
   }
 
   tc_fence_before_sync();
@@ -449,6 +481,11 @@ extern "C" int ccb_fp8_block_gemm(const void* A8, const float* sa_t, const void*
   if (make_tmap_u8_3d(&tmA, A8, (uint64_t)K, (uint64_t)M, 1, (uint64_t)K, 0, 128, FB_BM)) return -1;
   if (make_tmap_u8_3d(&tmB, B8, (uint64_t)K, (uint64_t)N, 1, (uint64_t)K, 0, 128, FB_BN)) return -1;
   FbArgs p;
+  // rows and base are on 16-byte boundaries wherever torch allocated the output itself
+  CUtensorMap tmC;
+  memset(&tmC, 0, sizeof(tmC));
+  p.tma_store = !out_fp32 && ((uintptr_t)C & 15) == 0 ? 1 : 0;
+  if (p.tma_store && make_tmap_bf16_3d(&tmC, C, (uint64_t)N, (uint64_t)M, 1, (uint64_t)ldc, 0, 64, 32)) return -1;
   p.M = (int)M; p.N = (int)N; p.K = (int)K;
   p.kblocks = (int)(K / 128);
   p.tiles_m = (int)((M + FB_BM - 1) / FB_BM);
@@ -459,7 +496,7 @@ extern "C" int ccb_fp8_block_gemm(const void* A8, const float* sa_t, const void*
   p.status = ccb_status_ptr();
   const long long total = (long long)p.tiles_m * p.tiles_n;
   const int grid = (int)(total < ccb_num_sms() ? total : ccb_num_sms());
-  fp8_block_gemm_kernel<<<grid, FB_THREADS, FB_SMEM, (cudaStream_t)stream>>>(tmA, tmB, p);
+  fp8_block_gemm_kernel<<<grid, FB_THREADS, FB_SMEM, (cudaStream_t)stream>>>(tmA, tmB, tmC, p);
   count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("fp8_block_gemm launch: %s", cudaGetErrorString(e));
