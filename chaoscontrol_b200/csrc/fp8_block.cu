@@ -199,7 +199,6 @@ fp8_quant_blocks_kernel(const __nv_bfloat16* __restrict__ w, uint8_t* __restrict
 // ---------------------------------------------------------------------------
 constexpr int FB_BM = 128, FB_BN = 128, FB_BK = 128;        // one-byte elements: 128 per swizzle row
 constexpr int FB_STAGE = FB_BM * FB_BK;                      // 16 KiB per operand tile
-constexpr int FB_STAGES = 5;
 constexpr int FB_SLOTS = 4;                                  // TMEM accumulator ring (4 x 128 columns)
 constexpr int FB_EPI_WARPS = 8;
 constexpr int FB_THREADS = 64 + 32 * FB_EPI_WARPS;
@@ -207,12 +206,25 @@ constexpr int FB_THREADS = 64 + 32 * FB_EPI_WARPS;
 // (128-byte rows, swizzled).  Storing them from registers, a row to a lane, cost 32 half-used sectors an
 // instruction: 65 536 x 256 x 1024 and its input gradient took 116 us, staged 101.
 constexpr int FB_STG = 32 * 128;
-constexpr int FB_STG_OFF = 2 * FB_STAGES * FB_STAGE;
-constexpr int FB_BAR_OFF = FB_STG_OFF + FB_EPI_WARPS * FB_STG;
-constexpr int FB_SMEM = 1024 + FB_BAR_OFF + 512;
+// RES: the weight tiles of a CTA's columns stay in shared memory (up to 128 KiB) while it walks the rows, and only
+// activations stream, a k-block to a stage; a row block's stages serve all of the CTA's column tiles.  With both
+// operands streaming, every 128 x 128 tile drags 2 x 128 x K bytes through the L2 -> SM path.  Events, cold L2,
+// streaming / resident in us at 65 536 rows: K x N = 256 x 1024 55 / 46, 512 x 1024 89 / 73, 384 x 640 50 / 46,
+// 1024 x 1024 155 / 146, 1024 x 256 50 / 46.
+template <int RES>
+struct FbCfg {
+  static constexpr int STAGES = RES ? 4 : 5;
+  static constexpr int RES_TILES = RES ? 8 : 0;              // 16 KiB weight tiles kept
+  static constexpr int A_OFF = RES_TILES * FB_STAGE;
+  static constexpr int STG_OFF = A_OFF + STAGES * (RES ? 1 : 2) * FB_STAGE;
+  static constexpr int BAR_OFF = STG_OFF + FB_EPI_WARPS * FB_STG;
+  static constexpr int SMEM = 1024 + BAR_OFF + 512;
+  static_assert(SMEM <= 227 * 1024, "exceeds the per-CTA shared memory limit");
+};
 
 struct FbArgs {
   int M, N, K, kblocks, tiles_m, tiles_n;
+  int nt, groups;           // RES: column tiles of a CTA, groups of CTAs that split the columns
   const float* sa_t;        // [K/128, M]
   const float* sb;          // scale of (output column block j, k block kb) at sb[j * sb_so + kb * sb_sk]
   long long sb_so, sb_sk;
@@ -223,27 +235,56 @@ struct FbArgs {
   int* status;
 };
 
+// Work of a CTA: row blocks w, w + nw, ... and, in each, column tiles [nt0, nt1); without RES one tile at a time.
+struct FbWalk {
+  int unit, step, units, nt0, nt1;
+};
+template <int RES>
+__device__ __forceinline__ FbWalk fb_walk(const FbArgs& p) {
+  FbWalk w;
+  if (RES) {
+    const int g = (int)blockIdx.x % p.groups;
+    w.unit = (int)blockIdx.x / p.groups;
+    w.step = (int)gridDim.x / p.groups;
+    w.units = p.tiles_m;
+    w.nt0 = g * p.nt;
+    w.nt1 = min(p.tiles_n, w.nt0 + p.nt);
+  } else {
+    w.unit = blockIdx.x;
+    w.step = gridDim.x;
+    w.units = p.tiles_m * p.tiles_n;
+    w.nt0 = 0;
+    w.nt1 = 1;
+  }
+  return w;
+}
+
+template <int RES>
 __global__ void __launch_bounds__(FB_THREADS, 1)
 fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmC, const FbArgs p) {
+  using Cfg = FbCfg<RES>;
+  constexpr int STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* sA = smem;
-  uint8_t* sB = smem + FB_STAGES * FB_STAGE;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + FB_BAR_OFF);
-  uint64_t* empty_bar = full_bar + FB_STAGES;
-  uint64_t* tfull_bar = empty_bar + FB_STAGES;
+  uint8_t* sA = smem + Cfg::A_OFF;
+  uint8_t* sB = RES ? smem : smem + STAGES * FB_STAGE;      // RES: tile (nt, kb) at ((nt - nt0) * kblocks + kb)
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Cfg::BAR_OFF);
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* tfull_bar = empty_bar + STAGES;
   uint64_t* tempty_bar = tfull_bar + FB_SLOTS;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + FB_SLOTS);
+  uint64_t* bres_bar = tempty_bar + FB_SLOTS;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bres_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int total_tiles = p.tiles_m * p.tiles_n;
+  const FbWalk wk = fb_walk<RES>(p);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < FB_STAGES; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
+    for (int i = 0; i < STAGES; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
     for (int i = 0; i < FB_SLOTS; ++i) { mbar_init(&tfull_bar[i], 1); mbar_init(&tempty_bar[i], FB_EPI_WARPS); }
+    mbar_init(bres_bar, 1);
     *abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmA);
@@ -263,14 +304,20 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-        const int m0 = (tile / p.tiles_n) * FB_BM, n0 = (tile % p.tiles_n) * FB_BN;
+      if (RES && wk.unit < wk.units) {
+        mbar_arrive_expect_tx(bres_bar, (uint32_t)((wk.nt1 - wk.nt0) * p.kblocks * FB_STAGE));
+        for (int nt = wk.nt0; nt < wk.nt1; ++nt)
+          for (int kb = 0; kb < p.kblocks; ++kb)
+            tma_load_3d(sB + ((nt - wk.nt0) * p.kblocks + kb) * FB_STAGE, &tmB, bres_bar, kb * FB_BK, nt * FB_BN, 0);
+      }
+      for (int u = wk.unit; u < wk.units && ok; u += wk.step) {
+        const int m0 = (RES ? u : u / p.tiles_n) * FB_BM, n0 = RES ? 0 : (u % p.tiles_n) * FB_BN;
         for (int kb = 0; kb < p.kblocks; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status)) { ok = false; break; }
-          mbar_arrive_expect_tx(&full_bar[stage], 2 * FB_STAGE);
+          mbar_arrive_expect_tx(&full_bar[stage], (RES ? 1 : 2) * FB_STAGE);
           tma_load_3d(sA + stage * FB_STAGE, &tmA, &full_bar[stage], kb * FB_BK, m0, 0);
-          tma_load_3d(sB + stage * FB_STAGE, &tmB, &full_bar[stage], kb * FB_BK, n0, 0);
-          if (++stage == FB_STAGES) { stage = 0; phase ^= 1u; }
+          if (!RES) tma_load_3d(sB + stage * FB_STAGE, &tmB, &full_bar[stage], kb * FB_BK, n0, 0);
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
       if (!ok) {
@@ -282,27 +329,34 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc = make_idesc_f8(FB_BM, FB_BN, 0, 0);
-      int stage = 0;
-      uint32_t phase = 0, n_slot = 0;
+      uint32_t n_slot = 0, n_ld = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-        for (int kb = 0; kb < p.kblocks; ++kb, ++n_slot) {
-          const int slot = n_slot % FB_SLOTS;
-          const uint32_t sph = (n_slot / FB_SLOTS) & 1u;
-          if (!mbar_wait(&tempty_bar[slot], sph ^ 1u, abort_flag, p.status)) { ok = false; break; }
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t a_base = smem_u32(sA + stage * FB_STAGE);
-          const uint32_t b_base = smem_u32(sB + stage * FB_STAGE);
+      if (RES && wk.unit < wk.units) {
+        ok = mbar_wait(bres_bar, 0u, abort_flag, p.status);
+        tc_fence_after_sync();
+      }
+      for (int u = wk.unit; u < wk.units && ok; u += wk.step, n_ld += (uint32_t)p.kblocks) {
+        for (int nt = wk.nt0; nt < wk.nt1 && ok; ++nt) {
+          for (int kb = 0; kb < p.kblocks; ++kb, ++n_slot) {
+            const int slot = n_slot % FB_SLOTS;
+            const uint32_t sph = (n_slot / FB_SLOTS) & 1u;
+            const uint32_t ld = n_ld + (uint32_t)kb;
+            const int stage = (int)(ld % STAGES);
+            if (!mbar_wait(&tempty_bar[slot], sph ^ 1u, abort_flag, p.status)) { ok = false; break; }
+            // a row block's stages arrive once and serve every column tile (more than one only while all fit the ring)
+            if (nt == wk.nt0 && !mbar_wait(&full_bar[stage], (ld / STAGES) & 1u, abort_flag, p.status)) { ok = false; break; }
+            tc_fence_after_sync();
+            const uint32_t a_base = smem_u32(sA + stage * FB_STAGE);
+            const uint32_t b_base = smem_u32(sB + (RES ? (nt - wk.nt0) * p.kblocks + kb : stage) * FB_STAGE);
 #pragma unroll
-          for (int k = 0; k < FB_BK / 32; ++k) {
-            const uint64_t adesc = make_smem_desc(a_base + k * 32, 16, 1024);
-            const uint64_t bdesc = make_smem_desc(b_base + k * 32, 16, 1024);
-            umma_f8(tmem_base + (uint32_t)(slot * FB_BN), adesc, bdesc, idesc, k > 0 ? 1u : 0u);
+            for (int k = 0; k < FB_BK / 32; ++k) {
+              const uint64_t adesc = make_smem_desc(a_base + k * 32, 16, 1024);
+              const uint64_t bdesc = make_smem_desc(b_base + k * 32, 16, 1024);
+              umma_f8(tmem_base + (uint32_t)(slot * FB_BN), adesc, bdesc, idesc, k > 0 ? 1u : 0u);
+            }
+            if (nt == wk.nt1 - 1) umma_commit(&empty_bar[stage]);
+            umma_commit(&tfull_bar[slot]);
           }
-          umma_commit(&empty_bar[stage]);
-          umma_commit(&tfull_bar[slot]);
-          if (++stage == FB_STAGES) { stage = 0; phase ^= 1u; }
         }
       }
     }
@@ -310,11 +364,31 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const int q = warp & 3;                    // TMEM lane quadrant
     const int part = (warp - 2) >> 2;          // columns [64 * part, 64 * part + 64) of the tile
     const int row_in_tile = q * 32 + lane;
-    uint8_t* my_stage = smem + FB_STG_OFF + (warp - 2) * FB_STG;
+    uint8_t* my_stage = smem + Cfg::STG_OFF + (warp - 2) * FB_STG;
     uint32_t n_slot = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-      const int m0 = (tile / p.tiles_n) * FB_BM, n0 = (tile % p.tiles_n) * FB_BN;
+    // The two block scales of a k-block do not depend on its accumulator: they are requested AHEAD k-blocks early,
+    // across tiles.  Fetched as the k-block began, their L2 latency was the k-block's time: 1470 cycles against 256
+    // of tensor work (streaming, 65 536 rows: 256 x 1024 66 us -> 55, 1024 x 1024 171 -> 155).
+    constexpr int AHEAD = 3;
+    float sca[AHEAD], scb[AHEAD];
+    int fu = wk.unit, fnt = wk.nt0, fkb = 0;                 // the k-block whose scales are fetched next
+    auto fetch_scales = [&](int i) {
+      sca[i] = scb[i] = 0.f;
+      if (fu >= wk.units) return;
+      const int fm = (RES ? fu : fu / p.tiles_n) * FB_BM + row_in_tile, fn = RES ? fnt : fu % p.tiles_n;
+      if (fm < p.M) sca[i] = __ldg(p.sa_t + (long long)fkb * p.M + fm);
+      scb[i] = __ldg(p.sb + (long long)fn * p.sb_so + (long long)fkb * p.sb_sk);
+      if (++fkb == p.kblocks) {
+        fkb = 0;
+        if (++fnt == wk.nt1) { fnt = wk.nt0; fu += wk.step; }
+      }
+    };
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) fetch_scales(i);
+    for (int u = wk.unit; u < wk.units && ok; u += wk.step)
+    for (int nt = wk.nt0; nt < wk.nt1; ++nt) {
+      const int m0 = (RES ? u : u / p.tiles_n) * FB_BM, n0 = (RES ? nt : u % p.tiles_n) * FB_BN;
       const int m = m0 + row_in_tile;
       const bool row_ok = m < p.M;
       float out[2][32];
@@ -325,24 +399,25 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       for (int kb = 0; kb < p.kblocks; ++kb, ++n_slot) {
         const int slot = n_slot % FB_SLOTS;
         const uint32_t sph = (n_slot / FB_SLOTS) & 1u;
-        // the two block scales do not depend on the accumulator: fetch before waiting
-        const float sc = (row_ok ? __ldg(p.sa_t + (long long)kb * p.M + m) : 0.f) *
-                         __ldg(p.sb + (long long)(n0 / FB_BN) * p.sb_so + (long long)kb * p.sb_sk);
+        const float sc = sca[0] * scb[0];
+#pragma unroll
+        for (int i = 0; i + 1 < AHEAD; ++i) { sca[i] = sca[i + 1]; scb[i] = scb[i + 1]; }
+        fetch_scales(AHEAD - 1);
         {
           const bool w = mbar_wait(&tfull_bar[slot], sph, abort_flag, p.status);
           if (!__all_sync(0xffffffffu, w)) { ok = false; break; }
         }
         tc_fence_after_sync();
         const uint32_t t_addr = tmem_base + (uint32_t)(slot * FB_BN + part * 64) + ((uint32_t)(q * 32) << 16);
+        uint32_t r[2][32];
+        __syncwarp();
+        tmem_ld32(t_addr, r[0]);
+        tmem_ld32(t_addr + 32, r[1]);
+        tmem_ld_wait();
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t r[32];
-          __syncwarp();
-          tmem_ld32(t_addr + h * 32, r);
-          tmem_ld_wait();
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int i = 0; i < 32; ++i) out[h][i] = fmaf(__uint_as_float(r[i]), sc, out[h][i]);
-        }
+          for (int i = 0; i < 32; ++i) out[h][i] = fmaf(__uint_as_float(r[h][i]), sc, out[h][i]);
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty_bar[slot]);
@@ -426,6 +501,24 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   }
 }
 
+template <int RES>
+static int launch_block_gemm(int grid, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
+                             const FbArgs& p, cudaStream_t stream) {
+  static bool attr_set[16] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!attr_set[dev & 15]) {
+    cudaError_t e = cudaFuncSetAttribute(fp8_block_gemm_kernel<RES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         FbCfg<RES>::SMEM);
+    if (e != cudaSuccess) return set_error("cudaFuncSetAttribute(fp8_block_gemm): %s", cudaGetErrorString(e));
+    attr_set[dev & 15] = true;
+  }
+  fp8_block_gemm_kernel<RES><<<grid, FB_THREADS, FbCfg<RES>::SMEM, stream>>>(tmA, tmB, tmC, p);
+  count_launch();
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : set_error("fp8_block_gemm launch: %s", cudaGetErrorString(e));
+}
+
 }  // namespace ccb
 
 using namespace ccb;
@@ -469,14 +562,6 @@ extern "C" int ccb_fp8_block_gemm(const void* A8, const float* sa_t, const void*
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (K % 128 != 0) return set_error("ccb_fp8_block_gemm: K must be a multiple of 128 (got %lld)", (long long)K);
   if ((out_fp32 ? ldc % 4 : ldc % 8) != 0) return set_error("ccb_fp8_block_gemm: output rows must be 16-byte aligned");
-  static bool attr_set[16] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!attr_set[dev & 15]) {
-    cudaError_t e = cudaFuncSetAttribute(fp8_block_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM);
-    if (e != cudaSuccess) return set_error("cudaFuncSetAttribute(fp8_block_gemm): %s", cudaGetErrorString(e));
-    attr_set[dev & 15] = true;
-  }
   CUtensorMap tmA, tmB;
   if (make_tmap_u8_3d(&tmA, A8, (uint64_t)K, (uint64_t)M, 1, (uint64_t)K, 0, 128, FB_BM)) return -1;
   if (make_tmap_u8_3d(&tmB, B8, (uint64_t)K, (uint64_t)N, 1, (uint64_t)K, 0, 128, FB_BN)) return -1;
@@ -495,9 +580,17 @@ extern "C" int ccb_fp8_block_gemm(const void* A8, const float* sa_t, const void*
   p.bias = (const __nv_bfloat16*)bias;
   p.status = ccb_status_ptr();
   const long long total = (long long)p.tiles_m * p.tiles_n;
-  const int grid = (int)(total < ccb_num_sms() ? total : ccb_num_sms());
-  fp8_block_gemm_kernel<<<grid, FB_THREADS, FB_SMEM, (cudaStream_t)stream>>>(tmA, tmB, tmC, p);
-  count_launch();
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : set_error("fp8_block_gemm launch: %s", cudaGetErrorString(e));
+  const int sms = ccb_num_sms();
+  // Resident weights: column tiles of a CTA as many as fit, and as leave every CTA at least two row blocks; more
+  // than one only while the row block fits the activation ring.  Fewer tiles than SMs: one tile a CTA.
+  int nt = p.kblocks <= 4 ? FbCfg<1>::RES_TILES / p.kblocks : 1;
+  if (nt > total / (2 * sms)) nt = (int)(total / (2 * sms));
+  if (nt < 1) nt = 1;
+  p.nt = nt;
+  p.groups = (p.tiles_n + nt - 1) / nt;
+  if (p.kblocks <= FbCfg<1>::RES_TILES && total > sms && p.groups <= sms) {
+    const long long walkers = sms / p.groups < p.tiles_m ? sms / p.groups : p.tiles_m;
+    return launch_block_gemm<1>((int)(walkers * p.groups), tmA, tmB, tmC, p, (cudaStream_t)stream);
+  }
+  return launch_block_gemm<0>((int)(total < sms ? total : sms), tmA, tmB, tmC, p, (cudaStream_t)stream);
 }

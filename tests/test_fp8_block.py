@@ -168,3 +168,29 @@ def test_quant_blocks_edges(N, K):
     assert torch.allclose(s.double(), pad.abs().amax(dim=(1, 3)).clamp_min(1e-12) / 448.0, rtol=1e-6)
     quo = (pad / s.double()[:, None, :, None]).view(nb * 128, kb * 128)[:N, :K]
     assert ((q.double() - quo).abs() <= (2.0 ** -4 + 1e-4) * quo.abs() + 2.0 ** -10 * 1.001).all()
+
+
+# more tiles than SMs: resident weights.  One, two, four and eight column tiles to a CTA, a last group that is not
+# full, a ragged last row and column tile, the deepest resident contraction and the first that streams
+@pytest.mark.gpu
+@pytest.mark.parametrize("R,K,N", [(19000, 128, 384), (40000, 256, 1024), (20011, 256, 640), (39000, 512, 264),
+                                   (26000, 384, 520), (19100, 1024, 256), (19100, 1152, 136)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_block_gemm_resident_weights(R, K, N, out_dtype):
+    """Against 64-bit products of the same 8-bit operands: products of e4m3 values are exact in fp32, so the
+    difference is K fp32 additions (and the rounding of a bf16 result)."""
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    qa, _, _ = FB.quant_rows(torch.randn(R, K, generator=g, device="cuda").bfloat16())
+    q, _, s = FB.quant_blocks((torch.randn(N, K, generator=g, device="cuda") * 0.1).bfloat16())
+    bias = torch.randn(N, generator=g, device="cuda").bfloat16()
+    out = FB.block_gemm(qa, q, s, sb_strides=(s.shape[1], 1), bias=bias, out_dtype=out_dtype)
+    from chaoscontrol_b200.ops import _lib
+    _lib.assert_ok()
+    a = (qa.q.double().view(R, K // 128, 128) * qa.s_t.double().t().unsqueeze(-1)).view(R, K)
+    nb = s.shape[0]
+    pad = torch.nn.functional.pad(q.double(), (0, 0, 0, nb * 128 - N)).view(nb, 128, K // 128, 128)
+    w = (pad * s.double()[:, None, :, None]).view(nb * 128, K)[:N]
+    ref, mag = a @ w.t() + bias.double(), a.abs() @ w.abs().t() + bias.double().abs()
+    rnd = 2.0 ** -8 if out_dtype is torch.bfloat16 else 0.0
+    assert ((out.double() - ref).abs() <= (K + 8) * 2.0 ** -24 * mag + rnd * ref.abs()).all()
+    assert torch.equal(out, FB.block_gemm(qa, q, s, sb_strides=(s.shape[1], 1), bias=bias, out_dtype=out_dtype))
