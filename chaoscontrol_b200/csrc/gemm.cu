@@ -965,7 +965,10 @@ static int launch_gemm(const CcbGemmArgs* a, cudaStream_t stream) {
         p.epi == CCB_EPI_ROWSCALE_SILU || p.f8)
       return set_error("ccb_gemm: shape not eligible for the resident-B layout (dispatch error)");
   }
-  if (g_gemm_pdl) {
+  // Launched as a programmatic dependent, a kernel sets up its barriers, tensor memory and descriptors under the
+  // tail of the one before it.  That is worth its extra launch attribute where SMs are free for it, i.e. in chains
+  // of small products (the fifteen above 131 -> 128 us, eager 174 -> 157).
+  if (g_gemm_pdl || 2 * total <= ccb_num_sms()) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(GEMM_THREADS);
@@ -1050,8 +1053,16 @@ extern "C" int ccb_gemm(const CcbGemmArgs* a, void* stream_) {
     return launch_gemm<256, 0, 0, 1>(a, stream);
   }
   if (a->epi < 0 || a->epi > CCB_EPI_RMSBWD) return set_error("ccb_gemm: unknown epilogue %lld", (long long)a->epi);
-  // 128-wide tiles only where the problem has a single narrow N tile to fill.
-  const bool narrow = a->N <= 128 && a->epi == CCB_EPI_STORE;
+  // 128-wide tiles where the problem has a single narrow N tile to fill, or where 256-wide ones would leave at
+  // least half of the SMs without any: such a launch is one tile's latency, and half a tile loads, multiplies and
+  // drains faster (fifteen Newton-Schulz products of 16 matrices 256 x 256: 172 -> 131 us on the device; layer
+  // backward at 512 rows of 256: 129 -> 113).  The row reductions of RESID_SS and RMSBWD want a row in one tile.
+  const long long tiles256 = (long long)a->batch * (a->splits < 1 ? 1 : a->splits) * ((a->M + 127) / 128) *
+                             ((a->N + 255) / 256);
+  const bool few = 2 * tiles256 <= ccb_num_sms() && !a->a_fp8 &&
+                   (a->epi == CCB_EPI_STORE || a->epi == CCB_EPI_ROWSCALE || a->epi == CCB_EPI_ROWSCALE_SILU ||
+                    a->epi == CCB_EPI_DSILU);
+  const bool narrow = (a->N <= 128 && a->epi == CCB_EPI_STORE) || few;
   if (narrow) {
     switch (key) {
       case 0: return launch_gemm<128, 0, 0>(a, stream);
