@@ -74,6 +74,8 @@ typedef struct CcbGemmArgs {
 } CcbGemmArgs;
 
 int ccb_gemm(const CcbGemmArgs* args, void* stream);
+// Split-K factor for C [m, n] = A^T B over k rows (both MN-major); tall: for 256-row tiles, 0 = not worth it.
+int64_t ccb_gemm_wgrad_splits(int64_t m, int64_t n, int64_t k, int64_t tall);
 
 // lse[m] = ln sum_v exp(logits[m, v]) from the LSE_PART partials ([nparts, M] float2);
 // loss[m] = lse[m] - zt[m] when both pointers are given.

@@ -93,22 +93,32 @@ constexpr int BRES_KBLOCKS = 4;
 // either CTA's late stage stalls both; on these memory-bound shapes that costs more than the saved weight
 // traffic.  Kept behind ccb_gemm_pair_resident (default off), like the plain pair mode.
 
-template <int BN, int CG = 1, int BRES = 0>
+// TALL (weight gradients): a tile is 256 rows, its halves in the two accumulators, and each B tile is loaded once
+// for both.  A weight gradient reads both operands over all rows and is bound by the L2 -> SM path, where 128 x 256
+// tiles read B once per 128 rows of A: dWp of a 256-wide layer at 131 072 rows drags 805 MB of operands, 537 in
+// 256 x 256 tiles.  Measured, events and cold L2, 128 / 256 rows in us: dWp [1024, 256] 95 / 82 at 131 072 rows and
+// 289 / 227 at 524 288, dW [256, 512] 64 / 59 and 165 / 148, [256, 256] at 524 288 89 / 74.  The GEMMs with a row
+// epilogue lose (K = 512 residual 67 / 89, RMSNorm backward K = 1024 107 / 151): their next tile's MMAs would wait
+// for the drain, while a weight gradient has one tile a CTA.
+template <int BN, int CG = 1, int BRES = 0, int TALL = 0>
 struct GemmCfg {
   static_assert(BRES == 0 || BRES == 1 || (BRES == 2 && CG == 2), "BRES 2 (K <= 512 resident) needs a CTA pair");
   static constexpr int B_ROWS = BN / CG;                  // rows of the B tile this CTA stages
   static constexpr int B_STAGE_BYTES = B_ROWS * BK * 2;
   static constexpr int RES_KBLOCKS = BRES == 2 ? 8 : BRES_KBLOCKS;   // k-blocks of the resident tile
+  static_assert(!TALL || (CG == 1 && BRES == 0 && BN == 256), "256-row tiles: streaming, one CTA");
+  static constexpr int A_TILE_BYTES = (TALL ? 2 : 1) * A_STAGE_BYTES;
   static constexpr int STAGES = BRES ? ((CG == 2 && BRES == 1) ? 8 : 4) : ((BN == 256 && CG == 1) ? 3 : 4);
   static constexpr int TMEM_COLS = 2 * BN;   // 512 or 256: powers of two
-  static constexpr int STG_BUFS = BRES ? 1 : STG_BUFS_PER_WARP;
+  static constexpr int STG_BUFS = (BRES || TALL) ? 1 : STG_BUFS_PER_WARP;
   static constexpr int A_OFF = BRES ? RES_KBLOCKS * B_STAGE_BYTES : 0;
-  static constexpr int STG_OFF = BRES ? A_OFF + STAGES * A_STAGE_BYTES : STAGES * (A_STAGE_BYTES + B_STAGE_BYTES);
+  static constexpr int STG_OFF = BRES ? A_OFF + STAGES * A_STAGE_BYTES : STAGES * (A_TILE_BYTES + B_STAGE_BYTES);
   static constexpr int BAR_OFF = STG_OFF + EPI_WARPS * STG_BUFS * STG_BUF_BYTES;
   static constexpr int XCH_OFF = BAR_OFF + 256;     // per-row partials exchanged between warps
-  // the resident layout has no room for alignment slack: its kernel checks that the dynamic
+  // the resident and tall layouts have no room for alignment slack: its kernel checks that the dynamic
   // shared-memory window starts on a 1 KiB boundary (it does when the kernel has no static shared memory)
-  static constexpr int SMEM_BYTES = (BRES ? 0 : 1024) + XCH_OFF + 2 * EPI_PARTS * BM * 4;
+  static constexpr bool ALIGNED_BASE = BRES || TALL;
+  static constexpr int SMEM_BYTES = (ALIGNED_BASE ? 0 : 1024) + XCH_OFF + 2 * EPI_PARTS * BM * 4;
   static_assert(2 * STAGES * 8 + 56 <= 256, "barrier block overflows its 256 bytes");
   static_assert(SMEM_BYTES <= 227 * 1024, "tile configuration exceeds the per-CTA shared memory limit");
 };
@@ -192,12 +202,13 @@ __device__ __forceinline__ float gemm_ex2(float x) {
 // LM = 1 compiles the LM-head epilogues (LSE_PART, CE_GRAD) instead of the trunk set.
 // EPI_T >= 0 fixes the epilogue at compile time (the hot trunk epilogues: no dispatch, less
 // code, fewer live registers in the chunk loop); EPI_T = -1 reads it from the arguments.
-template <int BN, int A_MN, int B_MN, int LM, int EPI_T, int CG, int BRES>
+template <int BN, int A_MN, int B_MN, int LM, int EPI_T, int CG, int BRES, int TALL>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmC2,
             const GemmKArgs p) {
-  using Cfg = GemmCfg<BN, CG, BRES>;
+  using Cfg = GemmCfg<BN, CG, BRES, TALL>;
+  static_assert(!TALL || (A_MN == 1 && B_MN == 1 && EPI_T == CCB_EPI_STORE), "256-row tiles: weight gradients");
   static_assert(CG == 1 || (A_MN == 0 && LM == 0), "CTA pairs: K-major A, trunk epilogues");
   static_assert(BRES == 0 || (A_MN == 0 && LM == 0), "resident B: K-major A, trunk epilogues");
   static_assert(BRES == 0 || EPI_T != CCB_EPI_ROWSCALE_SILU, "resident B has one staging buffer per warp: one output");
@@ -206,21 +217,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   // epilogues of both CTAs report to); the pair walks tiles of BM * CG rows together
   const uint32_t cta_rank = (CG == 2) ? cluster_ctarank() : 0u;
   const int walker = (int)blockIdx.x / CG, n_walkers = (int)gridDim.x / CG;
-  constexpr int BM_TILE = BM * CG;
+  constexpr int BM_TILE = BM * (TALL ? 2 : CG);
   const int epi_k = (EPI_T >= 0) ? EPI_T : p.epi;
   constexpr int STAGES = Cfg::STAGES;
   constexpr int B_STAGE_BYTES = Cfg::B_STAGE_BYTES;
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = BRES ? smem_raw
+  uint8_t* smem = Cfg::ALIGNED_BASE ? smem_raw
                        : reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                     ~static_cast<uintptr_t>(1023));
-  if (BRES && (smem_u32(smem) & 1023u) != 0u) {   // the swizzled tiles need a 1 KiB aligned base
+  if (Cfg::ALIGNED_BASE && (smem_u32(smem) & 1023u) != 0u) {   // the swizzled tiles need a 1 KiB aligned base
     if (threadIdx.x == 0) atomicCAS(p.status, CCB_OK, CCB_ERR_BAD_SHAPE);
     return;
   }
   uint8_t* sA = smem + Cfg::A_OFF;
-  uint8_t* sB = BRES ? smem : smem + STAGES * A_STAGE_BYTES;     // resident: k-block kb at sB + kb * B_STAGE_BYTES
+  uint8_t* sB = BRES ? smem : smem + STAGES * Cfg::A_TILE_BYTES;     // resident: k-block kb at sB + kb * B_STAGE_BYTES
   uint8_t* sStage = smem + Cfg::STG_OFF;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Cfg::BAR_OFF);
   uint64_t* empty_bar = full_bar + STAGES;
@@ -316,7 +327,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         for (int hn = 0; hn <= p.pair && ok; ++hn, t.n0 += BN)
         for (int kb = t.kb0; kb < t.kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status)) { ok = false; break; }
-          uint8_t* a_dst = sA + stage * A_STAGE_BYTES;
+          uint8_t* a_dst = sA + stage * Cfg::A_TILE_BYTES;
           uint8_t* b_dst = sB + stage * B_STAGE_BYTES;
           if (A_MN == 0 && CG == 1 && !p.pair && (p.l2pf & 1)) {
             // the same k-block of the tile after next: into L2 now, so that its load is an L2 hit
@@ -355,12 +366,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             if (++stage == STAGES) { stage = 0; phase ^= 1u; }
             continue;
           }
-          mbar_arrive_expect_tx(&full_bar[stage], A_STAGE_BYTES + B_STAGE_BYTES);
+          mbar_arrive_expect_tx(&full_bar[stage], Cfg::A_TILE_BYTES + B_STAGE_BYTES);
           if (A_MN == 0) {
             tma_load_3d(a_dst, &tmA, &full_bar[stage], kb * p.bk, t.m0, t.b);
+            if (TALL) tma_load_3d(a_dst + A_STAGE_BYTES, &tmA, &full_bar[stage], kb * p.bk, t.m0 + BM, t.b);
           } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j)
+            for (int j = 0; j < (TALL ? 2 : 1) * BM / 64; ++j)
               tma_load_3d(a_dst + j * 8192, &tmA, &full_bar[stage], t.m0 + 64 * j, kb * BK, t.b);
           }
           if (B_MN == 0) {
@@ -383,7 +395,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
     if (lane == 0 && cta_rank == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(BM_TILE, BN, A_MN, B_MN);
+      constexpr uint32_t idesc = make_idesc_bf16(BM * CG, BN, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -394,16 +406,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       }
       for (int tile = walker; tile < total_tiles && ok; tile += n_walkers, ++it) {
         TileCoord t = decode_tile(p, tile, BN, BM_TILE);
-        const int acc = p.pair ? 0 : (it & 1);
-        const uint32_t acc_phase = (uint32_t)(p.pair ? it : (it >> 1)) & 1u;
+        const int acc = (TALL || p.pair) ? 0 : (it & 1);
+        const uint32_t acc_phase = (uint32_t)((TALL || p.pair) ? it : (it >> 1)) & 1u;
         if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_flag, p.status)) { ok = false; break; }
+        if (TALL && !mbar_wait(&tempty_bar[1], acc_phase ^ 1u, abort_flag, p.status)) { ok = false; break; }
         tc_fence_after_sync();
         for (int hn = 0; hn <= p.pair && ok; ++hn) {
         const uint32_t d_tmem = tmem_base + (uint32_t)((p.pair ? hn : acc) * BN);
         for (int kb = t.kb0; kb < t.kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint32_t a_base = smem_u32(sA + stage * A_STAGE_BYTES);
+          const uint32_t a_base = smem_u32(sA + stage * Cfg::A_TILE_BYTES);
           const uint32_t b_base = smem_u32(sB + (BRES ? (kb - t.kb0) : stage) * B_STAGE_BYTES);
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
@@ -417,12 +430,24 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             else if (p.f8) umma_f8(d_tmem, adesc, bdesc, p.idesc_f8, accum);   // 32 one-byte k per MMA
             else umma_bf16(d_tmem, adesc, bdesc, idesc, accum);           // 16 two-byte k per MMA
           }
+          if (TALL) {
+            // rows 128..255 of the tile against the same B tile, into the other accumulator
+#pragma unroll
+            for (int k = 0; k < BK / 16; ++k) {
+              const uint32_t a2 = a_base + A_STAGE_BYTES;
+              const uint64_t adesc = A_MN ? make_smem_desc(a2 + k * 2048, 8192, 1024) : make_smem_desc(a2 + k * 32, 16, 1024);
+              const uint64_t bdesc = B_MN ? make_smem_desc(b_base + k * 2048, 8192, 1024)
+                                          : make_smem_desc(b_base + k * 32, 16, 1024);
+              umma_bf16(d_tmem + BN, adesc, bdesc, idesc, (kb > t.kb0 || k > 0) ? 1u : 0u);
+            }
+          }
           // stage reusable once these MMAs retire (in both CTAs of a pair)
           if (CG == 2) umma_commit_cg2(&empty_bar[stage]); else umma_commit(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
         }
         if (ok) { if (CG == 2) umma_commit_cg2(&tfull_bar[acc]); else umma_commit(&tfull_bar[acc]); }
+        if (TALL && ok) umma_commit(&tfull_bar[1]);
       }
     }
   } else {
@@ -445,11 +470,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       xphase ^= 1u;
       return __all_sync(0xffffffffu, w);
     };
-    for (int tile = walker; tile < total_tiles && ok; tile += n_walkers, ++it) {
+    for (int tile = walker; tile < total_tiles && ok; tile += n_walkers, ++it)
+    for (int half = 0; half < (TALL ? 2 : 1); ++half) {          // TALL: rows 0..127, then 128..255 (it may lie past the end)
       TileCoord t = decode_tile(p, tile, BN, BM_TILE);
-      t.m0 += BM * (int)cta_rank;             // this CTA's 128 rows of the pair's tile
-      const int acc = p.pair ? 0 : (it & 1);
-      const uint32_t acc_phase = (uint32_t)(p.pair ? it : (it >> 1)) & 1u;
+      t.m0 += BM * (TALL ? half : (int)cta_rank);       // this CTA's 128 rows of the pair's tile
+      const int acc = TALL ? half : (p.pair ? 0 : (it & 1));
+      const uint32_t acc_phase = (uint32_t)((TALL || p.pair) ? it : (it >> 1)) & 1u;
       const uint32_t t_addr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(q * 32) << 16);
       const int m = t.m0 + row_in_tile;
       const bool row_ok = m < p.M;
@@ -534,7 +560,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const int t1 = tile + n_walkers;
         if (t1 < total_tiles) {
           TileCoord tn = decode_tile(p, t1, BN, BM_TILE);
-          const int mn = tn.m0 + BM * (int)cta_rank + row_in_tile;
+          const int mn = tn.m0 + BM * (TALL ? half : (int)cta_rank) + row_in_tile;
           if (mn < p.M) {
             for (int k = 0; k < nmine; k += 2) {
               const int n = tn.n0 + chunk_of(k) * 32;
@@ -813,14 +839,14 @@ static int g_gemm_dbg = 0;
 static int g_gemm_l2pf = -1;
 static int g_gemm_pdl = 0;
 
-template <int BN, int A_MN, int B_MN, int LM = 0, int EPI_T = -1, int CG = 1, int BRES = 0>
+template <int BN, int A_MN, int B_MN, int LM = 0, int EPI_T = -1, int CG = 1, int BRES = 0, int TALL = 0>
 static int launch_gemm(const CcbGemmArgs* a, cudaStream_t stream) {
-  using Cfg = GemmCfg<BN, CG, BRES>;
+  using Cfg = GemmCfg<BN, CG, BRES, TALL>;
   static bool attr_set[16] = {false};
   static int max_pairs[16] = {0};
   int dev = 0;
   cudaGetDevice(&dev);
-  auto kern = gemm_kernel<BN, A_MN, B_MN, LM, EPI_T, CG, BRES>;
+  auto kern = gemm_kernel<BN, A_MN, B_MN, LM, EPI_T, CG, BRES, TALL>;
   if (!attr_set[dev & 15]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg::SMEM_BYTES);
@@ -894,7 +920,8 @@ static int launch_gemm(const CcbGemmArgs* a, cudaStream_t stream) {
   p.tma_store = tma_ok ? 1 : 0;
   p.M = (int)a->M; p.N = (int)a->N; p.K = (int)a->K;
   p.batch = (int)a->batch;
-  p.tiles_m = (p.M + BM * CG - 1) / (BM * CG);
+  constexpr int tile_rows = BM * (TALL ? 2 : CG);
+  p.tiles_m = (p.M + tile_rows - 1) / tile_rows;
   p.tiles_n = (p.N + BN - 1) / BN;
   p.kblocks = (p.K + p.bk - 1) / p.bk;
   int splits = (int)(a->splits < 1 ? 1 : a->splits);
@@ -1038,6 +1065,28 @@ extern "C" int ccb_gemm_cta_group(int cg) {
   return old;
 }
 
+// Split-K factor of a weight gradient [m, n] over k rows: as many splits as leave one tile to an SM, every split
+// non-empty.  tall != 0: the factor for 256-row tiles, 0 where 128-row ones are the better choice.  256-row tiles
+// halve the tile count, so the partial sums that the second stage reads double (38 MB instead of 19): they pay from
+// 24 k-blocks a CTA on, in problems that are split over rows at all, and where no half tile would be empty.
+extern "C" int64_t ccb_gemm_wgrad_splits(int64_t m, int64_t n, int64_t k, int64_t tall) {
+  const int64_t kblocks = (k + 63) / 64, tiles_n = (n + 255) / 256, tiles128 = (m + 127) / 128 * tiles_n;
+  const int64_t sms = ccb_num_sms();
+  int64_t tiles = tiles128 < 1 ? 1 : tiles128;
+  if (tall) {
+    if ((m + 127) / 128 % 2 != 0 || sms / tiles < 4 || tiles / 2 * kblocks < 24 * sms) return 0;
+    tiles /= 2;
+  }
+  int64_t want = sms / tiles;
+  if (want < 1) want = 1;
+  if (want > kblocks) want = kblocks;
+  for (; want > 1; --want) {
+    const int64_t per = (kblocks + want - 1) / want;
+    if ((kblocks + per - 1) / per == want) break;
+  }
+  return want;
+}
+
 extern "C" int ccb_gemm(const CcbGemmArgs* a, void* stream_) {
   using namespace ccb;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
@@ -1163,7 +1212,13 @@ extern "C" int ccb_gemm(const CcbGemmArgs* a, void* stream_) {
     switch (key) {
       case 0: return launch_gemm<256, 0, 0>(a, stream);
       case 1: return launch_gemm<256, 0, 1>(a, stream);
-      case 3: return launch_gemm<256, 1, 1>(a, stream);
+      case 3: {
+        const int64_t splits = a->splits < 1 ? 1 : a->splits;
+        if (a->epi == CCB_EPI_STORE && a->batch == 1 && a->out_fp32 && a->Cin == nullptr && a->bias == nullptr &&
+            ccb_gemm_wgrad_splits(a->M, a->N, a->K, 1) == splits)
+          return launch_gemm<256, 1, 1, 0, CCB_EPI_STORE, 1, 0, 1>(a, stream);
+        return launch_gemm<256, 1, 1>(a, stream);
+      }
       default: break;
     }
   }

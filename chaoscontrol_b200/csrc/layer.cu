@@ -61,18 +61,9 @@ static CcbGemmArgs gemm_args(const void* A, int64_t lda, const void* B, int64_t 
   return a;
 }
 
-// Split-K factor of a weight gradient [m, n] over k rows: as many as leave one tile to an SM, every split
-// non-empty (the Python front end's pick_splits).
 static int64_t wgrad_splits(int64_t m, int64_t n, int64_t k) {
-  const int64_t tiles = ((m + 127) / 128) * ((n + 255) / 256), kblocks = (k + 63) / 64;
-  int64_t want = ccb_num_sms() / (tiles < 1 ? 1 : tiles);
-  if (want < 1) want = 1;
-  if (want > kblocks) want = kblocks;
-  for (; want > 1; --want) {
-    const int64_t per = (kblocks + want - 1) / want;
-    if ((kblocks + per - 1) / per == want) break;
-  }
-  return want;
+  const int64_t tall = ccb_gemm_wgrad_splits(m, n, k, 1);
+  return tall > 0 ? tall : ccb_gemm_wgrad_splits(m, n, k, 0);
 }
 
 static int64_t max64(int64_t a, int64_t b) { return a > b ? a : b; }

@@ -59,6 +59,7 @@ _SIGS = {
     "ccb_last_error": ([], C.c_char_p),
     "ccb_status_ptr": ([], vp),
     "ccb_gemm": ([C.POINTER(GemmArgs), vp], C.c_int),
+    "ccb_gemm_wgrad_splits": ([i64, i64, i64, i64], i64),
     "ccb_lse_combine": ([vp, i64, i64, vp, vp, vp, vp], C.c_int),
     "ccb_fp8_quant_rows": ([vp, i64, vp, f32, vp, vp, vp, vp, i64, i64, vp], C.c_int),
     "ccb_fp8_quant_blocks": ([vp, vp, vp, vp, i64, i64, vp], C.c_int),

@@ -219,7 +219,7 @@ class _BlockFP8LinearFn(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             xb = x2.to(torch.bfloat16).contiguous()
             if g2.is_cuda and _lib.available():
-                S = G.pick_splits(N, K, g2.shape[0])
+                S = G.wgrad_splits(N, K, g2.shape[0])
                 part = G.gemm(g2, xb, a_mn=True, b_mn=True, splits=S, out_dtype=torch.float32)
                 gw, _ = splitk_reduce(part, out_dtype=wdtype if wdtype == torch.bfloat16 else torch.float32)
             else:

@@ -23,7 +23,7 @@ from . import _lib
 from ._lib import (EPI_CE_GRAD, EPI_DSILU, EPI_LSE_PART, EPI_RESID_SS, EPI_RMSBWD, EPI_ROWSCALE,
                    EPI_ROWSCALE_SILU, EPI_STORE, GemmArgs)
 
-__all__ = ["gemm", "gemm_fp8", "gemm_lm", "gemm_reference", "pick_splits", "EPI_STORE", "EPI_ROWSCALE",
+__all__ = ["gemm", "gemm_fp8", "gemm_lm", "gemm_reference", "pick_splits", "wgrad_splits", "EPI_STORE", "EPI_ROWSCALE",
            "EPI_ROWSCALE_SILU", "EPI_RESID_SS", "EPI_DSILU", "EPI_RMSBWD", "EPI_LSE_PART", "EPI_CE_GRAD"]
 
 
@@ -41,6 +41,13 @@ def pick_splits(m: int, n: int, k: int, bn: int = 256) -> int:
             break
         want -= 1
     return want
+
+
+def wgrad_splits(m: int, n: int, k: int) -> int:
+    """:func:`pick_splits` for the tile height that the weight-gradient kernel takes: twice as many splits of
+    256-row tiles where the contraction is long enough for them."""
+    L = _lib.lib()
+    return int(L.ccb_gemm_wgrad_splits(m, n, k, 1) or L.ccb_gemm_wgrad_splits(m, n, k, 0))
 
 
 def _dims(a: torch.Tensor, b: torch.Tensor, a_mn: bool, b_mn: bool):

@@ -33,7 +33,7 @@ import torch
 
 from . import _lib
 from .gemm import (EPI_DSILU, EPI_RESID_SS, EPI_RMSBWD, EPI_ROWSCALE, EPI_ROWSCALE_SILU,
-                   EPI_STORE, gemm, pick_splits)
+                   EPI_STORE, gemm, wgrad_splits)
 from .scan import scan_fused_bwd, scan_fused_fwd, scan_fused_reference
 
 EPS = 1e-6
@@ -172,7 +172,7 @@ def _wgrad(dy: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
     """Split-K partials of ``dy^T @ x`` (``[S, N, K]`` fp32)."""
     M, N = dy.shape
     K = x.shape[1]
-    S = pick_splits(N, K, M) if dy.is_cuda else 1
+    S = wgrad_splits(N, K, M) if dy.is_cuda else 1
     out = gemm(dy, x, a_mn=True, b_mn=True, splits=S, out_dtype=torch.float32)
     return out if out.dim() == 3 else out.unsqueeze(0)
 

@@ -45,3 +45,20 @@ def test_few_tiles_batches_and_layouts(G_, M, N, K):
             _lib.assert_ok()
             tol = (2.0 ** -8 if dt is torch.bfloat16 else 0.0) * ref.abs() + 1e-5 * ref.abs().max()
             assert ((out.float() - ref).abs() <= tol).all()
+
+
+# contractions just above the line where a weight gradient takes 256-row tiles; ragged columns and k-blocks
+@pytest.mark.parametrize("M,N,K", [(1024, 256, 58000), (512, 248, 114000), (256, 256, 227400), (1536, 384, 19003)])
+def test_tall_weight_gradient_tiles(M, N, K):
+    """dW = A^T B over K rows against 64 bits: K fp32 additions of exact products, spread over the splits."""
+    S = G.wgrad_splits(M, N, K)
+    assert S == _lib.lib().ccb_gemm_wgrad_splits(M, N, K, 1) and S >= 4
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a, b = (torch.randn(K, n, generator=g, device="cuda").bfloat16() for n in (M, N))
+    part = G.gemm(a, b, a_mn=True, b_mn=True, splits=S, out_dtype=torch.float32)
+    _lib.assert_ok()
+    ref, mag = a.double().t() @ b.double(), a.double().abs().t() @ b.double().abs()
+    per = (K + S - 1) // S
+    assert ((part.double().sum(0) - ref).abs() <= per * 2.0 ** -24 * mag).all()
+    assert torch.equal(part, G.gemm(a, b, a_mn=True, b_mn=True, splits=S, out_dtype=torch.float32))
+    assert G.wgrad_splits(M, N, K // 2) == G.pick_splits(M, N, K // 2)      # below the line: 128-row tiles
