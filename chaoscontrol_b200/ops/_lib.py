@@ -60,6 +60,7 @@ _SIGS = {
     "ccb_status_ptr": ([], vp),
     "ccb_gemm": ([C.POINTER(GemmArgs), vp], C.c_int),
     "ccb_gemm_wgrad_splits": ([i64, i64, i64, i64], i64),
+    "ccb_newton_schulz": ([vp, vp, vp, vp, i64, i64, i64, i64, f32, f32, f32, vp], C.c_int),
     "ccb_lse_combine": ([vp, i64, i64, vp, vp, vp, vp], C.c_int),
     "ccb_fp8_quant_rows": ([vp, i64, vp, f32, vp, vp, vp, vp, i64, i64, vp], C.c_int),
     "ccb_fp8_quant_blocks": ([vp, vp, vp, vp, i64, i64, vp], C.c_int),

@@ -33,19 +33,31 @@ def _ns_torch(X: Tensor, steps: int) -> Tensor:
 
 
 def _ns_kernels(X: Tensor, steps: int) -> Tensor:
-    """Newton-Schulz on a normalised bf16 batch ``[G, r, c]`` with the tcgen05 GEMM.
+    """Newton-Schulz on a normalised bf16 batch ``[G, r, c]`` (also used as workspace): one launch for small
+    matrices, else :func:`_ns_products`; the arithmetic is the same."""
+    a, b, c = _NS_COEFFS
+    G, r, cdim = X.shape
+    k = min(r, cdim)
+    A = torch.empty(2, G, k, k, dtype=torch.bfloat16, device=X.device)
+    Y = torch.empty_like(X)
+    rc = _lib.lib().ccb_newton_schulz(X.data_ptr(), Y.data_ptr(), A[0].data_ptr(), A[1].data_ptr(), G, r, cdim, steps,
+                                      a, b, c, _lib.stream_ptr())
+    if rc > 0:
+        return _ns_products(X, Y, A[0], A[1], steps)
+    _lib.check(rc, "newton_schulz")
+    return Y if steps % 2 else X
+
+
+def _ns_products(X: Tensor, Y: Tensor, A: Tensor, B: Tensor, steps: int) -> Tensor:
+    """The iteration as separate tcgen05 GEMMs (``Y`` like ``X``, ``A`` and ``B`` ``[G, k, k]``: workspace).
 
     Wide / square matrices iterate ``X <- aX + (bA + cA^2) X`` with ``A = X X^T``;
     tall ones use ``A = X^T X`` and ``X <- aX + X (bA + cA^2)`` so nothing is ever
     transposed in memory.
     """
     a, b, c = _NS_COEFFS
-    G, r, cdim = X.shape
+    r, cdim = X.shape[1:]
     tall = r > cdim
-    k = cdim if tall else r
-    A = torch.empty(G, k, k, dtype=torch.bfloat16, device=X.device)
-    B = torch.empty_like(A)
-    Y = torch.empty_like(X)
     for _ in range(steps):
         if tall:
             kblocks = (r + 63) // 64
