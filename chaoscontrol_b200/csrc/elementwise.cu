@@ -81,8 +81,18 @@ __global__ void embed_fwd_kernel(const TokT* __restrict__ tok, const __nv_bfloat
 // ---------------------------------------------------------------------------
 constexpr int EMB_CH = 32;
 
-template <int VPL>   // uint4 vectors per lane: D = 256 * VPL
-__global__ void embed_bwd_runs_kernel(const long long* __restrict__ sorted_tok,
+// Sort keys: the token, or -1 / V for one below / above the table (its rows belong to no gradient; the order stays that
+// of the tokens).  Two bytes instead of eight leave a radix sort two passes instead of eight.
+template <typename TokT>
+__global__ void token_keys_kernel(const TokT* __restrict__ tok, short* __restrict__ key, long long R, int V) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < R; i += (long long)gridDim.x * blockDim.x) {
+    const long long t = (long long)tok[i];
+    key[i] = (short)(t < 0 ? -1 : (t < V ? t : V));
+  }
+}
+
+template <int VPL, typename TokT>   // VPL uint4 vectors per lane: D = 256 * VPL
+__global__ void embed_bwd_runs_kernel(const TokT* __restrict__ sorted_tok,
                                       const long long* __restrict__ perm,
                                       const __nv_bfloat16* __restrict__ dx,
                                       float* __restrict__ dE, float* __restrict__ slots,
@@ -95,10 +105,10 @@ __global__ void embed_bwd_runs_kernel(const long long* __restrict__ sorted_tok,
   const int lane = threadIdx.x & 31;
   const int n = (int)(p1 - p0);
   // one coalesced load of the chunk's tokens and row indices, handed round by shuffles
-  const long long my_tok = (lane < n) ? sorted_tok[p0 + lane] : -1;
+  const long long my_tok = (lane < n) ? (long long)sorted_tok[p0 + lane] : -1;
   const long long my_row = (lane < n) ? perm[p0 + lane] : 0;
-  const long long tok_before = (p0 > 0) ? sorted_tok[p0 - 1] : -1;
-  const long long tok_after = (p1 < R) ? sorted_tok[p1] : -1;
+  const long long tok_before = (p0 > 0) ? (long long)sorted_tok[p0 - 1] : -1;
+  const long long tok_after = (p1 < R) ? (long long)sorted_tok[p1] : -1;
   {
     // token boundaries: where a token's rows begin and end in the sorted order
     long long prev = __shfl_up_sync(0xffffffffu, my_tok, 1);
@@ -173,66 +183,96 @@ __global__ void embed_bwd_runs_kernel(const long long* __restrict__ sorted_tok,
   flush(cur, run_start, n);
 }
 
-// grid: V blocks of 16 warps.  Warp w adds the boundary slots k = w, w + 16, ... of the token's
-// chunk run in order (lane l owns columns [l * D/32, (l+1) * D/32)), then warp 0 adds the sixteen
-// warp sums in warp order: a fixed tree, wide enough that the most frequent token of a Zipf batch
-// (thousands of chunks) does not serialise behind one warp.
+// A token's boundary slots k = w, w + 16, ... are added by warp w in order (lane l owns columns
+// [l * D/32, (l+1) * D/32)) and the sixteen sums are added in warp order: a fixed tree, wide enough that the most
+// frequent token of a Zipf batch (thousands of chunks) does not serialise behind one warp.  Up to sixteen slots the
+// tree is a plain sum in slot order, which one warp does by itself.  So a block takes JOIN_TOKS tokens, a grid apart
+// so that neighbouring ids (frequent ones come together) spread over blocks: its warps take the short ones side by
+// side, then all of them each long one.  A block of sixteen warps per token, most of which had nothing to join,
+// took 44 us at 32 768 rows and V = 16 384; 10 now.
 // first_pos / last_pos come from stage 1; last_pos is -1 for tokens that do not occur.
-constexpr int EMB_JOIN_WARPS = 16;
+constexpr int EMB_JOIN_WARPS = 16, EMB_JOIN_TOKS = 32;
 template <int FPL>   // floats per lane: D = 32 * FPL
 __global__ void __launch_bounds__(EMB_JOIN_WARPS * 32)
 embed_bwd_join_kernel(const long long* __restrict__ first_pos, const long long* __restrict__ last_pos,
-                      const float* __restrict__ slots, float* __restrict__ dE, int D) {
-  const long long tk = blockIdx.x;
-  const long long e = last_pos[tk] + 1;
-  if (e <= 0) return;
-  const long long s = first_pos[tk];
-  const long long cs = s / EMB_CH, ce = (e - 1) / EMB_CH;
-  if (cs == ce) return;                       // one owner: stored by stage 1
+                      const float* __restrict__ slots, float* __restrict__ dE, int D, int V) {
   extern __shared__ float sm_join[];          // [EMB_JOIN_WARPS][D]
+  __shared__ long long s_first[EMB_JOIN_TOKS], s_n[EMB_JOIN_TOKS];     // first position; slots to add (0: none)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = lane * FPL;
-  const long long n = ce - cs + 1;            // slots to add: chunk cs (first or second slot), then first slots
-  const int first_slot = ((s % EMB_CH) == 0) ? 0 : 1;
-  float acc[FPL];
-#pragma unroll
-  for (int i = 0; i < FPL; ++i) acc[i] = 0.f;
-  auto slot_ptr = [&](long long k) {
-    return slots + ((cs + k) * 2 + (k == 0 ? first_slot : 0)) * (long long)D + c0;
-  };
-  long long k = warp;
-  for (; k + 3 * EMB_JOIN_WARPS < n; k += 4 * EMB_JOIN_WARPS) {
-    float4 t[4][FPL / 4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const float4* p = reinterpret_cast<const float4*>(slot_ptr(k + u * EMB_JOIN_WARPS));
-#pragma unroll
-      for (int i = 0; i < FPL / 4; ++i) t[u][i] = p[i];
+  if (threadIdx.x < EMB_JOIN_TOKS) {
+    const long long tk = (long long)blockIdx.x + (long long)threadIdx.x * gridDim.x;
+    long long s = 0, n = 0;
+    if (tk < V) {
+      const long long e = last_pos[tk] + 1;
+      if (e > 0) {
+        s = first_pos[tk];
+        const long long cs = s / EMB_CH, ce = (e - 1) / EMB_CH;
+        if (cs != ce) n = ce - cs + 1;        // one owner: stored by stage 1
+      }
     }
+    s_first[threadIdx.x] = s;
+    s_n[threadIdx.x] = n;
+  }
+  __syncthreads();
+  // slots of token j: chunk cs (first or second slot), then first slots
+  auto slot_ptr = [&](int j, long long k) {
+    const long long s = s_first[j], cs = s / EMB_CH;
+    return slots + ((cs + k) * 2 + (k == 0 && s % EMB_CH != 0 ? 1 : 0)) * (long long)D + c0;
+  };
+  float acc[FPL];
+  // adds slots k, k + step, ... in order, four in flight
+  auto add_slots = [&](int j, long long k, long long n, int step) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int i = 0; i < FPL; ++i) acc[i] = 0.f;
+    for (; k + 3 * step < n; k += 4 * step) {
+      float4 t[4][FPL / 4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4* p = reinterpret_cast<const float4*>(slot_ptr(j, k + u * step));
+#pragma unroll
+        for (int i = 0; i < FPL / 4; ++i) t[u][i] = p[i];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int i = 0; i < FPL / 4; ++i) {
+          acc[4 * i] += t[u][i].x; acc[4 * i + 1] += t[u][i].y;
+          acc[4 * i + 2] += t[u][i].z; acc[4 * i + 3] += t[u][i].w;
+        }
+    }
+    for (; k < n; k += step) {
+      const float4* p = reinterpret_cast<const float4*>(slot_ptr(j, k));
 #pragma unroll
       for (int i = 0; i < FPL / 4; ++i) {
-        acc[4 * i] += t[u][i].x; acc[4 * i + 1] += t[u][i].y;
-        acc[4 * i + 2] += t[u][i].z; acc[4 * i + 3] += t[u][i].w;
+        const float4 v = p[i];
+        acc[4 * i] += v.x; acc[4 * i + 1] += v.y; acc[4 * i + 2] += v.z; acc[4 * i + 3] += v.w;
       }
-  }
-  for (; k < n; k += EMB_JOIN_WARPS) {
-    const float4* p = reinterpret_cast<const float4*>(slot_ptr(k));
-#pragma unroll
-    for (int i = 0; i < FPL / 4; ++i) {
-      const float4 v = p[i];
-      acc[4 * i] += v.x; acc[4 * i + 1] += v.y; acc[4 * i + 2] += v.z; acc[4 * i + 3] += v.w;
     }
+  };
+  for (int j = warp; j < EMB_JOIN_TOKS; j += EMB_JOIN_WARPS) {
+    const long long n = s_n[j];
+    if (n == 0 || n > EMB_JOIN_WARPS) continue;
+    add_slots(j, 0, n, 1);
+    float4* o = reinterpret_cast<float4*>(dE + ((long long)blockIdx.x + (long long)j * gridDim.x) * D + c0);
+#pragma unroll
+    for (int i = 0; i < FPL / 4; ++i) o[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
   }
+  for (int j = 0; j < EMB_JOIN_TOKS; ++j) {
+    const long long n = s_n[j];
+    if (n <= EMB_JOIN_WARPS) continue;        // the same for the whole block
+    add_slots(j, warp, n, EMB_JOIN_WARPS);
 #pragma unroll
-  for (int i = 0; i < FPL; ++i) sm_join[warp * D + c0 + i] = acc[i];
-  __syncthreads();
-  for (int c = threadIdx.x; c < D; c += blockDim.x) {
-    float t = sm_join[c];
+    for (int i = 0; i < FPL; ++i) sm_join[warp * D + c0 + i] = acc[i];
+    __syncthreads();
+    const long long tk = (long long)blockIdx.x + (long long)j * gridDim.x;
+    for (int c = threadIdx.x; c < D; c += blockDim.x) {
+      float t = sm_join[c];
 #pragma unroll
-    for (int w = 1; w < EMB_JOIN_WARPS; ++w) t += sm_join[w * D + c];
-    dE[tk * D + c] = t;
+      for (int w = 1; w < EMB_JOIN_WARPS; ++w) t += sm_join[w * D + c];
+      dE[tk * D + c] = t;
+    }
+    __syncthreads();                          // before the next token's sums replace these
   }
 }
 
@@ -951,44 +991,60 @@ extern "C" int ccb_embed_fwd(const void* tok, int64_t tok_is_i64, const void* E,
 extern "C" int64_t ccb_embed_bwd_slots(int64_t R, int64_t D, int64_t V) {
   return ((R + EMB_CH - 1) / EMB_CH) * 2 * D + 4 * V;
 }
+// key[i] = the token, -1 below or V above the table; V < 32 768.
+extern "C" int ccb_token_keys(const void* tok, int64_t tok_is_i64, void* key_i16, int64_t R, int64_t V, void* stream) {
+  if (R <= 0) return 0;
+  if (V <= 0 || V > 32767) return set_error("ccb_token_keys: V=%lld does not fit 16-bit keys", (long long)V);
+  if (tok_is_i64)
+    token_keys_kernel<<<grid_for(R, 256), 256, 0, (cudaStream_t)stream>>>((const long long*)tok, (short*)key_i16, R, (int)V);
+  else
+    token_keys_kernel<<<grid_for(R, 256), 256, 0, (cudaStream_t)stream>>>((const int*)tok, (short*)key_i16, R, (int)V);
+  CCB_CHECK_LAUNCH("token_keys");
+  return 0;
+}
+
+template <int VPL, typename TokT>
+static int launch_embed_bwd(const TokT* st, const long long* pm, const __nv_bfloat16* g, float* dE, float* slots,
+                            long long* fp, long long* lp, int64_t R, int64_t V, cudaStream_t s) {
+  constexpr int D = 256 * VPL, wpb = 4;
+  const long long chunks = (R + EMB_CH - 1) / EMB_CH;
+  embed_bwd_runs_kernel<VPL, TokT><<<(unsigned)((chunks + wpb - 1) / wpb), wpb * 32, 0, s>>>(
+      st, pm, g, dE, slots, fp, lp, R, D, (int)V);
+  CCB_CHECK_LAUNCH("embed_bwd_runs");
+  constexpr int smem = EMB_JOIN_WARPS * D * (int)sizeof(float);
+  // sixteen [1024] strips are 64 KiB of shared memory: above the default limit, opt in
+  if (smem > 48 * 1024) cudaFuncSetAttribute(embed_bwd_join_kernel<D / 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  embed_bwd_join_kernel<D / 32><<<(unsigned)((V + EMB_JOIN_TOKS - 1) / EMB_JOIN_TOKS), EMB_JOIN_WARPS * 32, smem, s>>>(
+      fp, lp, slots, dE, D, (int)V);
+  CCB_CHECK_LAUNCH("embed_bwd_join");
+  return 0;
+}
+
+// sorted_tok: int64, or the 16-bit keys of ccb_token_keys (tok_bytes 8 / 2).
+extern "C" int ccb_embed_bwd_sorted_as(const void* sorted_tok, int64_t tok_bytes, const int64_t* perm, const void* dx,
+                                       float* dE, float* slots, int64_t R, int64_t D, int64_t V, void* stream) {
+  if (R <= 0) return 0;
+  if (slots == nullptr) return set_error("ccb_embed_bwd_sorted: the boundary-slot workspace is required");
+  if (tok_bytes != 8 && tok_bytes != 2) return set_error("ccb_embed_bwd_sorted: tokens of %lld bytes", (long long)tok_bytes);
+  if (D != 256 && D != 512 && D != 1024)
+    return set_error("ccb_embed_bwd_sorted: D=%lld unsupported (256, 512, 1024)", (long long)D);
+  cudaStream_t s = (cudaStream_t)stream;
+  const long long* pm = (const long long*)perm;
+  const __nv_bfloat16* g = (const __nv_bfloat16*)dx;
+  long long* fp = reinterpret_cast<long long*>(slots + (R + EMB_CH - 1) / EMB_CH * 2 * D);
+  long long* lp = fp + V;
+  cudaMemsetAsync(lp, 0xFF, sizeof(long long) * (size_t)V, s);      // -1: token does not occur
+  auto run = [&](auto* st) {
+    if (D == 256) return launch_embed_bwd<1>(st, pm, g, dE, slots, fp, lp, R, V, s);
+    if (D == 512) return launch_embed_bwd<2>(st, pm, g, dE, slots, fp, lp, R, V, s);
+    return launch_embed_bwd<4>(st, pm, g, dE, slots, fp, lp, R, V, s);
+  };
+  return tok_bytes == 8 ? run((const long long*)sorted_tok) : run((const short*)sorted_tok);
+}
 extern "C" int ccb_embed_bwd_sorted(const int64_t* sorted_tok, const int64_t* perm, const void* dx,
                                     float* dE, float* slots, int64_t R, int64_t D, int64_t V,
                                     void* stream) {
-  if (R <= 0) return 0;
-  if (slots == nullptr) return set_error("ccb_embed_bwd_sorted: the boundary-slot workspace is required");
-  const int wpb = 4;
-  const long long chunks = (R + EMB_CH - 1) / EMB_CH;
-  const unsigned grid = (unsigned)((chunks + wpb - 1) / wpb);
-  cudaStream_t s = (cudaStream_t)stream;
-  const long long* st = (const long long*)sorted_tok;
-  const long long* pm = (const long long*)perm;
-  const __nv_bfloat16* g = (const __nv_bfloat16*)dx;
-  long long* fp = reinterpret_cast<long long*>(slots + chunks * 2 * D);
-  long long* lp = fp + V;
-  cudaMemsetAsync(lp, 0xFF, sizeof(long long) * (size_t)V, s);      // -1: token does not occur
-  if (D == 256) {
-    embed_bwd_runs_kernel<1><<<grid, wpb * 32, 0, s>>>(st, pm, g, dE, slots, fp, lp, R, (int)D, (int)V);
-    CCB_CHECK_LAUNCH("embed_bwd_runs");
-    embed_bwd_join_kernel<8><<<(unsigned)V, EMB_JOIN_WARPS * 32, EMB_JOIN_WARPS * D * sizeof(float), s>>>(
-        fp, lp, slots, dE, (int)D);
-  } else if (D == 512) {
-    embed_bwd_runs_kernel<2><<<grid, wpb * 32, 0, s>>>(st, pm, g, dE, slots, fp, lp, R, (int)D, (int)V);
-    CCB_CHECK_LAUNCH("embed_bwd_runs");
-    embed_bwd_join_kernel<16><<<(unsigned)V, EMB_JOIN_WARPS * 32, EMB_JOIN_WARPS * D * sizeof(float), s>>>(
-        fp, lp, slots, dE, (int)D);
-  } else if (D == 1024) {
-    embed_bwd_runs_kernel<4><<<grid, wpb * 32, 0, s>>>(st, pm, g, dE, slots, fp, lp, R, (int)D, (int)V);
-    CCB_CHECK_LAUNCH("embed_bwd_runs");
-    // sixteen [1024] strips are 64 KiB of shared memory: above the default limit, opt in
-    cudaFuncSetAttribute(embed_bwd_join_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(EMB_JOIN_WARPS * 1024 * sizeof(float)));
-    embed_bwd_join_kernel<32><<<(unsigned)V, EMB_JOIN_WARPS * 32, EMB_JOIN_WARPS * D * sizeof(float), s>>>(
-        fp, lp, slots, dE, (int)D);
-  } else {
-    return set_error("ccb_embed_bwd_sorted: D=%lld unsupported (256, 512, 1024)", (long long)D);
-  }
-  CCB_CHECK_LAUNCH("embed_bwd_join");
-  return 0;
+  return ccb_embed_bwd_sorted_as(sorted_tok, 8, perm, dx, dE, slots, R, D, V, stream);
 }
 
 static int launch_colsum(const float* part, int64_t NB, int64_t K, void* out, int out_bf16, int64_t accumulate,

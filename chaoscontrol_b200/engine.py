@@ -81,9 +81,8 @@ class TrainEngine:
         B, Tn = inputs.shape
         R = B * Tn
         V = model.lm_head.weight.shape[0]
-        flat_in = inputs.reshape(-1)
         # token sort for the embedding backward: depends on the inputs only
-        sort_cache = torch.sort(flat_in.long(), stable=True)
+        sort_cache = T.token_sort(inputs, V) if model.dim in T.EMBED_BWD_DIMS else None
         x, ss = T.embed_fwd(inputs, a.param_view("embed.weight"))
         ws, ctxs = [], []
         for i in range(len(model.layers)):

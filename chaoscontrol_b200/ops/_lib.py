@@ -80,6 +80,8 @@ _SIGS = {
     "ccb_plain_scan_bwd": ([vp, i64, vp, vp, vp, i64, vp, vp, vp, i64, i64, i64, vp], C.c_int),
     "ccb_embed_fwd": ([vp, i64, vp, vp, vp, i64, i64, i64, vp], C.c_int),
     "ccb_embed_bwd_sorted": ([vp, vp, vp, vp, vp, i64, i64, i64, vp], C.c_int),
+    "ccb_embed_bwd_sorted_as": ([vp, i64, vp, vp, vp, vp, i64, i64, i64, vp], C.c_int),
+    "ccb_token_keys": ([vp, i64, vp, i64, i64, vp], C.c_int),
     "ccb_embed_bwd_slots": ([i64, i64, i64], C.c_int64),
     "ccb_lmhead_epilogue_parts": ([C.c_int], C.c_int),
     "ccb_gemm_cta_group": ([C.c_int], C.c_int),

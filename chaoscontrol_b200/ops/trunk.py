@@ -96,30 +96,46 @@ def embed_fwd(tokens: torch.Tensor, E: torch.Tensor):
     return x, (x.float() ** 2).sum(-1)
 
 
+EMBED_BWD_DIMS = (256, 512, 1024)      # widths of the sorted embedding-backward kernel
+
+
+def token_sort(tokens: torch.Tensor, V: int):
+    """``(sorted tokens, stable permutation)`` for :func:`embed_bwd`.  On the GPU 16-bit keys where the table allows."""
+    flat = tokens.reshape(-1)
+    if flat.is_cuda and V < 32768 and flat.dtype in (torch.int32, torch.int64) and flat.numel() > 0:
+        flat = flat.contiguous()
+        key = torch.empty(flat.numel(), dtype=torch.int16, device=flat.device)
+        _lib.check(_lib.lib().ccb_token_keys(flat.data_ptr(), int(flat.dtype == torch.int64), key.data_ptr(),
+                                             flat.numel(), V, _lib.stream_ptr()), "token_keys")
+        flat = key
+    else:
+        flat = flat.long()
+    return torch.sort(flat, stable=True)
+
+
 def embed_bwd(tokens: torch.Tensor, dx: torch.Tensor, V: int,
               sort_cache: Optional[tuple] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """fp32 ``[V, D]`` gradient of the embedding table (sum of the ``dx`` rows of each token).
 
     On the GPU the rows are added in a fixed order derived from the stably sorted token array, so
     the same batch gives the same bits on every run and on every replica."""
-    flat = tokens.reshape(-1).long()
     D = dx.shape[1]
     if out is not None:
         dE = out.zero_()
     else:
         dE = torch.zeros(V, D, dtype=torch.float32, device=dx.device)
-    if dx.is_cuda and D in (256, 512, 1024):
+    if dx.is_cuda and D in EMBED_BWD_DIMS:
         if sort_cache is None:
-            sort_cache = torch.sort(flat, stable=True)
+            sort_cache = token_sort(tokens, V)
         st, perm = sort_cache
         L = _lib.lib()
-        slots = torch.empty(int(L.ccb_embed_bwd_slots(flat.numel(), D, V)), dtype=torch.float32,
-                            device=dx.device)
-        _lib.check(L.ccb_embed_bwd_sorted(st.data_ptr(), perm.data_ptr(), dx.data_ptr(), dE.data_ptr(),
-                                          slots.data_ptr(), flat.numel(), D, V, _lib.stream_ptr()),
+        R = st.numel()
+        slots = torch.empty(int(L.ccb_embed_bwd_slots(R, D, V)), dtype=torch.float32, device=dx.device)
+        _lib.check(L.ccb_embed_bwd_sorted_as(st.data_ptr(), st.element_size(), perm.data_ptr(), dx.data_ptr(),
+                                             dE.data_ptr(), slots.data_ptr(), R, D, V, _lib.stream_ptr()),
                    "embed_bwd")
         return dE
-    dE.index_add_(0, flat, dx.float())
+    dE.index_add_(0, tokens.reshape(-1).long(), dx.float())
     return dE
 
 

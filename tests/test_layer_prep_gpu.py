@@ -77,3 +77,22 @@ def _weights(rnd, D, F):
     lin = lambda n, k: rnd(n, k, k=k ** -0.5).bfloat16()
     return trunk.LayerWeights(Wp=lin(4 * D, D), Wo=lin(D, D), Wfc=lin(F, D), Wproj=lin(D, F), wn1=rnd(D).bfloat16(),
                           wn2=rnd(D).bfloat16(), log_a=rnd(D).bfloat16()).prepare()
+
+
+# tokens in one chunk, in sixteen and in seventeen (one warp / all warps of a block), vocabularies on both sides of
+# 16-bit keys, and ids outside the table, which no gradient takes
+@pytest.mark.parametrize("V,dt", [(31, torch.int64), (33, torch.int32), (32767, torch.int64), (32768, torch.int64),
+                                  (40000, torch.int32)])
+@pytest.mark.parametrize("D", [256, 512])
+def test_embed_bwd_token_widths(V, dt, D):
+    g = torch.Generator(device="cuda").manual_seed(V + D)
+    runs = [(0, 1), (1, 31), (2, 32 * 14), (5, 32 * 15 + 3), (7, 32 * 16 + 5), (V - 1, 2000), (-3, 40), (V, 33), (V + 70000, 9)]
+    tok = torch.cat([torch.full((n,), t, dtype=torch.int64) for t, n in runs]).cuda()
+    tok = tok[torch.randperm(tok.numel(), generator=g, device="cuda")].to(dt)
+    dx = torch.randn(tok.numel(), D, generator=g, device="cuda").bfloat16()
+    got = trunk.embed_bwd(tok, dx, V)
+    ok = (tok >= 0) & (tok < V)
+    ref = torch.zeros(V, D, dtype=torch.float64, device="cuda").index_add_(0, tok[ok].long(), dx[ok].double())
+    mag = torch.zeros(V, D, dtype=torch.float64, device="cuda").index_add_(0, tok[ok].long(), dx[ok].double().abs())
+    assert ((got.double() - ref).abs() <= 2048 * 2.0 ** -24 * mag).all()          # at most 2000 fp32 additions a row
+    assert torch.equal(got, trunk.embed_bwd(tok, dx, V, sort_cache=torch.sort(tok.long(), stable=True)))
