@@ -436,7 +436,7 @@ __global__ void colsum_kernel(const float* __restrict__ part, int NB, int K, OT*
   }
 }
 
-// W'[n,k] = W[n,k] * wn[k]  (bf16), the RMSNorm weight folded into a linear.
+// W'[n,k] = W[n,k] * wn[k]  (bf16), the RMSNorm weight folded into a linear; any width and alignment.
 __global__ void fold_colscale_kernel(const __nv_bfloat16* __restrict__ W,
                                      const __nv_bfloat16* __restrict__ wn,
                                      __nv_bfloat16* __restrict__ out, long long N, int K) {
@@ -444,6 +444,19 @@ __global__ void fold_colscale_kernel(const __nv_bfloat16* __restrict__ W,
   if (i >= N * K) return;
   const int k = (int)(i % K);
   out[i] = __float2bfloat16(__bfloat162float(W[i]) * __bfloat162float(wn[k]));
+}
+// The same in 16-byte vectors (an LM head of 16 384 x 256: 16 us an element a thread, under 8 like this).
+__global__ void __launch_bounds__(256)
+fold_colscale_vec_kernel(const uint4* __restrict__ W, const uint4* __restrict__ wn, uint4* __restrict__ out,
+                         long long n, int kv) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint4 w = __ldg(W + i), g = __ldg(wn + (int)(i % kv));
+  auto mul = [](uint32_t a, uint32_t b) {
+    const float2 x = unpack_bf16x2(a), y = unpack_bf16x2(b);
+    return pack_bf16x2(x.x * y.x, x.y * y.y);
+  };
+  out[i] = make_uint4(mul(w.x, g.x), mul(w.y, g.y), mul(w.z, g.z), mul(w.w, g.w));
 }
 
 // ---------------------------------------------------------------------------
@@ -1121,8 +1134,14 @@ extern "C" int ccb_colsum(const float* part, int64_t NB, int64_t K, float* out, 
 extern "C" int ccb_fold_colscale(const void* W, const void* wn, void* out, int64_t N, int64_t K,
                                  void* stream) {
   if (N * K <= 0) return 0;
-  fold_colscale_kernel<<<(unsigned)((N * K + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)W, (const __nv_bfloat16*)wn, (__nv_bfloat16*)out, N, (int)K);
+  if (K % 8 == 0 && (((uintptr_t)W | (uintptr_t)wn | (uintptr_t)out) & 15) == 0) {
+    const long long n = N * K / 8;
+    fold_colscale_vec_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        (const uint4*)W, (const uint4*)wn, (uint4*)out, n, (int)(K / 8));
+  } else {
+    fold_colscale_kernel<<<(unsigned)((N * K + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        (const __nv_bfloat16*)W, (const __nv_bfloat16*)wn, (__nv_bfloat16*)out, N, (int)K);
+  }
   CCB_CHECK_LAUNCH("fold_colscale");
   return 0;
 }

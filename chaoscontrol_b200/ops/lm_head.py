@@ -197,11 +197,13 @@ def lm_head_lse(x, rowss, W_f, targets, *, eps: float = EPS, want_entropy: bool 
 
 def default_row_chunks(R: int, V: int) -> int:
     """Row-chunk count for the dW kernel so (V/128 x chunks) work items divide
-    evenly over the SMs."""
+    evenly over the SMs: the fewest chunks that keep 97 % of them busy (the most
+    even count where none does), because every chunk writes a [V, D] partial that
+    the reduction reads back."""
     sms = _lib.lib().ccb_num_sms() if _lib.available() else 148
     vt = max(V // 128, 1)
     mt = (R + 127) // 128
-    best = 1
+    best, best_eff = 1, 0.0
     for c in range(1, min(mt, 64) + 1):
         per = (mt + c - 1) // c
         if (mt + per - 1) // per != c:
@@ -209,10 +211,10 @@ def default_row_chunks(R: int, V: int) -> int:
         items = vt * c
         waves = (items + sms - 1) // sms
         eff = items / (waves * sms)
-        if eff > 0.97 and c >= best:
-            best = c
-            if items >= 8 * sms:
-                break
+        if eff > best_eff:
+            best, best_eff = c, eff
+        if eff > 0.97 or items >= 8 * sms:
+            break
     return best
 
 
