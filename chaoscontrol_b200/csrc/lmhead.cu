@@ -84,12 +84,63 @@ struct LmHeadArgs {
   __nv_bfloat16* dX;        // [R, 256] out (TRAIN)
   const __nv_bfloat16* W;   // [V, 256] folded head weight (TRAIN1: target rows are gathered)
   float* dWpart;            // [row_chunks, V, 256] out (DW)
+  // split walk (LSE / TRAIN / TRAIN1): see LhWalk; null = whole m-tiles
+  float4* part_rows;        // [2 * grid, 128]
+  float* part_acc;          // [2 * grid, 128, 256] (training)
   int* status;
   // stage-isolation switches for bottleneck analysis (results are then wrong by design):
   // 1 = the gradient-sweep epilogue skips exp2 / pack / the shared-memory store of the g tile,
   // 2 = the second MMA (dX or dW accumulation) is not issued, 4 = the logits MMA is not issued
   int dbg;
 };
+
+// What a CTA works on, the same in every warp role: units of rows (an m-tile, or a (v-tile, row chunk) pair for dW)
+// and, in each, tiles [inner0, inner1) of the other operand.
+//
+// The sweeps over the vocabulary own an m-tile per unit, so 512 m-tiles on 148 SMs are 3.46 waves that take four, and
+// 71 leave half of the chip idle.  With a workspace the m-tile x v-tile steps are dealt out evenly instead: CTA i
+// takes steps [i * share, (i + 1) * share) of the flattened order, i.e. at most one partial m-tile at either end of
+// its range and whole ones between.  A partial m-tile's row sums and accumulators go to slot 2i or 2i + 1, and
+// lmhead_join_kernel adds the pieces of each m-tile in vocabulary order.  V = 16 384: gradient sweep with a given lse
+// at 512 m-tiles 865 -> 740 us and 11 for the join, one-sweep training at 256 m-tiles 476 -> 420 and 15, scoring at
+// 512 505 -> 490 and 9.
+struct LhWalk {
+  int mode_dw, n_vtiles, n_mtiles, per_chunk;
+  int unit, step, units;              // whole units
+  long long pos, end;                 // split walk (end > 0)
+  bool split, first;
+  int cta;
+  // the unit, its inner range and its slot (-1: whole); false when the CTA is done
+  __device__ __forceinline__ bool next(int& u, int& inner0, int& inner1, int& slot) {
+    slot = -1;
+    if (split) {
+      if (pos >= end) return false;
+      u = (int)(pos / n_vtiles);
+      inner0 = (int)(pos - (long long)u * n_vtiles);
+      const long long left = end - pos;
+      inner1 = left < n_vtiles - inner0 ? inner0 + (int)left : n_vtiles;
+      if (inner0 != 0 || inner1 != n_vtiles) slot = 2 * cta + (first ? 0 : 1);
+      first = false;
+      pos += inner1 - inner0;
+      return true;
+    }
+    if (unit >= units) return false;
+    u = unit;
+    unit += step;
+    if (mode_dw) {
+      inner0 = u / n_vtiles * per_chunk;
+      inner1 = min(n_mtiles, inner0 + per_chunk);
+    } else {
+      inner0 = 0;
+      inner1 = n_vtiles;
+    }
+    return true;
+  }
+};
+
+__host__ __device__ __forceinline__ long long lh_share(long long n_mtiles, long long n_vtiles, int grid) {
+  return (n_mtiles * n_vtiles + grid - 1) / grid;
+}
 
 struct LhBars {
   uint64_t res_full, res_empty;
@@ -166,7 +217,20 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
   // ---- work decomposition (identical in every role) -------------------------
   // LSE / TRAIN: unit = m-tile; inner = v-tiles (x sweeps).
   // DW: unit = (v-tile, row chunk); inner = m-tiles of the chunk.
-  const int n_units = (MODE == MODE_DW) ? p.n_vtiles * p.row_chunks : p.n_mtiles;
+  LhWalk walk;
+  walk.mode_dw = MODE == MODE_DW;
+  walk.n_vtiles = p.n_vtiles;
+  walk.n_mtiles = p.n_mtiles;
+  walk.per_chunk = p.mtiles_per_chunk;
+  walk.unit = blockIdx.x;
+  walk.step = gridDim.x;
+  walk.units = (MODE == MODE_DW) ? p.n_vtiles * p.row_chunks : p.n_mtiles;
+  walk.split = MODE != MODE_DW && p.part_rows != nullptr;
+  walk.first = true;
+  walk.cta = blockIdx.x;
+  const long long share = lh_share(p.n_mtiles, p.n_vtiles, gridDim.x), n_steps = (long long)p.n_mtiles * p.n_vtiles;
+  walk.pos = share * blockIdx.x;
+  walk.end = walk.pos + share < n_steps ? walk.pos + share : n_steps;
   constexpr bool IS_TRAIN = (MODE == MODE_TRAIN) || (MODE == MODE_TRAIN1);
   constexpr bool FUSED1 = (MODE == MODE_TRAIN1);
   // Scoring keeps the unit's X tile in tensor memory and feeds it to the logits MMA from there:
@@ -198,18 +262,9 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
       uint32_t res_phase = 0;
       uint32_t n_stg = 0;
       bool ok = true;
-      for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
-        int res_row, inner0, inner1;
-        if (MODE == MODE_DW) {
-          const int vt = unit % p.n_vtiles, ch = unit / p.n_vtiles;
-          res_row = vt * LH_VT;
-          inner0 = ch * p.mtiles_per_chunk;
-          inner1 = min(p.n_mtiles, inner0 + p.mtiles_per_chunk);
-        } else {
-          res_row = unit * LH_ROWS;
-          inner0 = 0;
-          inner1 = p.n_vtiles;
-        }
+      int unit, inner0, inner1, slot;
+      while (ok && walk.next(unit, inner0, inner1, slot)) {
+        const int res_row = (MODE == MODE_DW) ? unit % p.n_vtiles * LH_VT : unit * LH_ROWS;
         const CUtensorMap* tmRes = (MODE == MODE_DW) ? &tmW : &tmX;
         const CUtensorMap* tmStg = (MODE == MODE_DW) ? &tmX : &tmW;
         if (!TA) {
@@ -281,13 +336,8 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         return true;
       };
 
-      for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
-        int inner0 = 0, inner1 = p.n_vtiles;
-        if (MODE == MODE_DW) {
-          const int ch = unit / p.n_vtiles;
-          inner0 = ch * p.mtiles_per_chunk;
-          inner1 = min(p.n_mtiles, inner0 + p.mtiles_per_chunk);
-        }
+      int unit, inner0, inner1, slot;
+      while (ok && walk.next(unit, inner0, inner1, slot)) {
         if (!TA) {
           if (!mbar_wait(&bars->res_full, res_phase, abort_flag, p.status)) { ok = false; break; }
         }
@@ -399,15 +449,10 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
       return true;
     };
 
-    for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
-      int inner0 = 0, inner1 = p.n_vtiles, v_unit0 = 0, ch = 0;
-      if (MODE == MODE_DW) {
-        const int vt = unit % p.n_vtiles;
-        ch = unit / p.n_vtiles;
-        v_unit0 = vt * LH_VT;
-        inner0 = ch * p.mtiles_per_chunk;
-        inner1 = min(p.n_mtiles, inner0 + p.mtiles_per_chunk);
-      }
+    int unit, inner0, inner1, slot;
+    while (ok && walk.next(unit, inner0, inner1, slot)) {
+      const int v_unit0 = (MODE == MODE_DW) ? unit % p.n_vtiles * LH_VT : 0, ch = unit / p.n_vtiles;
+      float4* prow = slot >= 0 ? p.part_rows + (long long)slot * LH_ROWS + row_in_tile : nullptr;   // partial m-tile
       // per-row constants (LSE / TRAIN: fixed for the unit; DW: reloaded per m-tile)
       int r = 0;
       bool row_ok = false;
@@ -740,17 +785,18 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
           if (!parts_sum(run_s * my_resc, s)) { ok = false; break; }
           const float lse2 = m + __log2f(s);
           c2 = lse2;
-          if (row_ok && part == 0) p.lse[r] = lse2 * LN2;
+          if (row_ok && part == 0 && !prow) p.lse[r] = lse2 * LN2;
           if (MODE == MODE_LSE) {
             // the target column lived in exactly one part
-            float t_all = 0.f;
+            float t_all = 0.f, e_tot = 0.f;
             if (!parts_sum(tacc, t_all)) { ok = false; break; }
-            if (row_ok && part == 0) p.loss[r] = lse2 * LN2 - t_all * rs;
-            if (p.entropy != nullptr) {
+            if (p.entropy != nullptr && !parts_sum(run_e * my_resc, e_tot)) { ok = false; break; }
+            if (prow) {
+              if (part == 0) *prow = make_float4(m, s, t_all, e_tot);
+            } else if (row_ok && part == 0) {
+              p.loss[r] = lse2 * LN2 - t_all * rs;
               // H = lse - E[logit],  E[logit] = rs * sum(p~ * raw) / sum(p~)
-              float e_tot = 0.f;
-              if (!parts_sum(run_e * my_resc, e_tot)) { ok = false; break; }
-              if (row_ok && part == 0) p.entropy[r] = lse2 * LN2 - rs * e_tot / s;
+              if (p.entropy != nullptr) p.entropy[r] = lse2 * LN2 - rs * e_tot / s;
             }
           }
         } else if (FUSED1) {
@@ -760,7 +806,9 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
           if (!parts_sum(zt, z_all)) { ok = false; break; }
           const float lg = __log2f(S);
           inv_s = 1.f / S;
-          if (row_ok && part == 0) {
+          if (prow) {
+            if (part == 0) *prow = make_float4(c2, S, z_all, 0.f);
+          } else if (row_ok && part == 0) {
             p.lse[r] = (c2 + lg) * LN2;
             p.loss[r] = (lg - z_all) * LN2;
           }
@@ -768,7 +816,11 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
           // per-row CE = -log p_target = -zt * ln2 (zt captured by exactly one warp of the row)
           float z_all = 0.f;
           if (!parts_sum(zt, z_all)) { ok = false; break; }
-          if (row_ok && part == 0) p.loss[r] = -z_all * LN2;
+          if (prow) {
+            if (part == 0) *prow = make_float4(0.f, 0.f, z_all, 0.f);
+          } else if (row_ok && part == 0) {
+            p.loss[r] = -z_all * LN2;
+          }
         }
       }
       if (!ok) break;
@@ -779,7 +831,21 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
           if (!wait_all(&bars->d2_full, n_d2 & 1u)) { ok = false; break; }
           tc_fence_after_sync();
           const uint32_t t2 = tmem_base + 256 + lane_addr;
-          if (IS_TRAIN) {
+          if (IS_TRAIN && prow) {
+            // a piece of the m-tile: the accumulator as it is
+            float* orow = p.part_acc + ((long long)slot * LH_ROWS + row_in_tile) * LH_D;
+            for (int c = 0; c < 8; ++c) {
+              uint32_t a[32];
+              __syncwarp();
+              tmem_ld32(t2 + c * 32, a);
+              tmem_ld_wait();
+              float4* o4 = reinterpret_cast<float4*>(orow + c * 32);
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                o4[j] = make_float4(__uint_as_float(a[j * 4]), __uint_as_float(a[j * 4 + 1]),
+                                    __uint_as_float(a[j * 4 + 2]), __uint_as_float(a[j * 4 + 3]));
+            }
+          } else if (IS_TRAIN) {
             // dx = q - x * (rs^2 / D) * sum_d q * x   (RMSNorm backward, weight folded)
             const __nv_bfloat16* xrow = p.X + (long long)r * LH_D;
             // TRAIN1: the accumulator holds sum_v p~ W'; q = (acc / S - W'[target]) * gs
@@ -881,6 +947,97 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
   }
 }
 
+// Joins the pieces of m-tiles that the split walk cut: one warp a row, pieces in vocabulary order.  Sixteen blocks
+// of eight rows for each boundary between two CTAs' ranges; those of a tile's first boundary do the work.
+// The pieces' own references (m: the maximum, or TRAIN1's fixed one) are brought to the largest of them.
+template <int MODE>
+__global__ void __launch_bounds__(256) lmhead_join_kernel(const LmHeadArgs p, int grid) {
+  const long long share = lh_share(p.n_mtiles, p.n_vtiles, grid), nv = p.n_vtiles;
+  const long long cut = ((blockIdx.x >> 4) + 1) * share;                // where CTA (blockIdx.x >> 4) + 1 begins
+  if (cut >= (long long)p.n_mtiles * nv) return;
+  const int unit = (int)(cut / nv);
+  if (cut == unit * nv || cut - share > unit * nv) return;              // between two tiles; not the tile's first
+  const int row = (blockIdx.x & 15) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int r = unit * LH_ROWS + row;
+  if (r >= p.R) return;
+  const int c_first = (int)(unit * nv / share), c_last = (int)(((unit + 1) * nv - 1) / share);
+  auto slot_of = [&](int c) -> long long { return 2 * c + (c * share >= unit * nv ? 0 : 1); };
+  const float rs = p.rowss ? rsqrtf(p.rowss[r] * p.inv_dim + p.eps) : 1.f;
+  const int tgt = (int)p.targets[r];
+  float M = -INFINITY;
+  if (MODE != MODE_TRAIN)
+    for (int c = c_first; c <= c_last; ++c) M = fmaxf(M, p.part_rows[slot_of(c) * LH_ROWS + row].x);
+  float S = 0.f, z = 0.f, e = 0.f, acc[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+  for (int c = c_first; c <= c_last; ++c) {
+    const long long slot = slot_of(c);
+    const float4 v = p.part_rows[slot * LH_ROWS + row];
+    const float w = MODE == MODE_TRAIN ? 1.f : ex2f(v.x - M);
+    S += v.y * w;
+    if (MODE == MODE_TRAIN1) {
+      // the piece that holds the target knows its logit relative to the piece's reference
+      const long long a = c * share > unit * nv ? c * share - unit * nv : 0, b = (c + 1) * share - unit * nv;
+      if (tgt / LH_VT >= a && tgt / LH_VT < b) z = v.z + v.x;
+    } else {
+      z += v.z;
+    }
+    e += v.w * w;
+    if (MODE != MODE_LSE) {
+      const float4* a4 = reinterpret_cast<const float4*>(p.part_acc + (slot * LH_ROWS + row) * LH_D + lane * 8);
+      const float4 a0 = __ldg(a4), a1 = __ldg(a4 + 1);
+      acc[0] += a0.x * w; acc[1] += a0.y * w; acc[2] += a0.z * w; acc[3] += a0.w * w;
+      acc[4] += a1.x * w; acc[5] += a1.y * w; acc[6] += a1.z * w; acc[7] += a1.w * w;
+    }
+  }
+  if (lane == 0) {
+    if (MODE == MODE_LSE) {
+      const float lse = (M + __log2f(S)) * LN2;
+      p.lse[r] = lse;
+      p.loss[r] = lse - z * rs;
+      if (p.entropy != nullptr) p.entropy[r] = lse - rs * e / S;
+    } else if (MODE == MODE_TRAIN1) {
+      p.lse[r] = (M + __log2f(S)) * LN2;
+      p.loss[r] = (M + __log2f(S) - z) * LN2;
+    } else {
+      p.loss[r] = -z * LN2;
+    }
+  }
+  if (MODE == MODE_LSE) return;
+  const float gscale = p.gscale_dev ? p.gscale * __ldg(p.gscale_dev) : p.gscale;
+  const float gs = gscale * (p.rowweight ? p.rowweight[r] : 1.f) * rs;
+  auto unpack = [](const uint4& u, float (&f)[8]) {
+    const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
+    f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+  };
+  if (MODE == MODE_TRAIN1) {
+    float wv[8];
+    unpack(__ldg(reinterpret_cast<const uint4*>(p.W + (long long)tgt * LH_D + lane * 8)), wv);
+    const float inv_s = 1.f / S;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = (acc[i] * inv_s - wv[i]) * gs;
+  }
+  float xv[8], dot = 0.f;
+  unpack(__ldg(reinterpret_cast<const uint4*>(p.X + (long long)r * LH_D + lane * 8)), xv);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) dot += acc[i] * xv[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+  const float coef = p.rowss ? dot * rs * rs * p.inv_dim : 0.f;
+  uint4 o;
+  o.x = pack_bf16x2(acc[0] - xv[0] * coef, acc[1] - xv[1] * coef); o.y = pack_bf16x2(acc[2] - xv[2] * coef, acc[3] - xv[3] * coef);
+  o.z = pack_bf16x2(acc[4] - xv[4] * coef, acc[5] - xv[5] * coef); o.w = pack_bf16x2(acc[6] - xv[6] * coef, acc[7] - xv[7] * coef);
+  *reinterpret_cast<uint4*>(p.dX + (long long)r * LH_D + lane * 8) = o;
+}
+
+// Whether the sweep over `n_mtiles` row tiles is split: where whole tiles would leave the SMs at least SPLIT_STEPS
+// v-tile steps short of even.
+constexpr int LH_SPLIT_STEPS = 16;
+static bool lh_split(long long n_mtiles, long long n_vtiles) {
+  const long long sms = ccb_num_sms(), waves = (n_mtiles + sms - 1) / sms;
+  return waves * n_vtiles - lh_share(n_mtiles, n_vtiles, (int)sms) >= LH_SPLIT_STEPS;
+}
+
 // Epilogue column parts: 2 = eight epilogue warps, 4 = sixteen; 0 = per mode, as measured on a B200
 // at 262 144 rows: the scoring sweep gains from sixteen warps (1.81 -> 1.77 ms), the training kernels
 // lose (7.76 -> 8.11 ms for the one-sweep kernel plus the dW kernel).
@@ -906,10 +1063,19 @@ static int launch_lmhead_p(const void* X, const void* W, LmHeadArgs& a, cudaStre
   if (make_tmap_bf16_3d(&tmW, W, LH_D, (uint64_t)a.V, 1, LH_D, 0, 64, 128)) return -1;
   a.status = ccb_status_ptr();
   a.dbg = g_lh_dbg;
-  const int units = (MODE == MODE_DW) ? a.n_vtiles * a.row_chunks : a.n_mtiles;
-  const int grid = units < ccb_num_sms() ? units : ccb_num_sms();
+  const bool split = MODE != MODE_DW && a.part_rows != nullptr;
+  const long long units = (MODE == MODE_DW) ? a.n_vtiles * a.row_chunks
+                                            : (split ? (long long)a.n_mtiles * a.n_vtiles : a.n_mtiles);
+  const int grid = (int)(units < ccb_num_sms() ? units : ccb_num_sms());
   kern<<<grid, lh_threads(PARTS), LH_SMEM, stream>>>(tmX, tmW, a);
   count_launch();
+  if (split) {
+    constexpr int JM = MODE == MODE_DW ? MODE_LSE : MODE;              // not instantiated for dW
+    if (grid > 1) {
+      lmhead_join_kernel<JM><<<(unsigned)((grid - 1) * 16), 256, 0, stream>>>(a, grid);
+      count_launch();
+    }
+  }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("lmhead launch: %s", cudaGetErrorString(e));
 }
@@ -972,10 +1138,21 @@ static int lmhead_common(LmHeadArgs& a, int64_t R, int64_t V, int64_t D, const f
   return 0;
 }
 
-// lse[r], loss[r] = CE of row r.  Forward only.
+// Floats of the workspace with which ccb_lmhead_lse (train 0) / ccb_lmhead_train (train 1, one vocabulary sweep)
+// deal the work out evenly over the SMs; 0 where whole row tiles do as well.
+extern "C" int64_t ccb_lmhead_work(int64_t R, int64_t V, int64_t D, int64_t train) {
+  if (R <= 0 || D != LH_D || V % LH_VT != 0 || !lh_split((R + LH_ROWS - 1) / LH_ROWS, V / LH_VT)) return 0;
+  return 2 * (int64_t)ccb_num_sms() * LH_ROWS * (4 + (train ? LH_D : 0));
+}
+static void lh_workspace(LmHeadArgs& a, float* work) {
+  a.part_rows = (float4*)work;
+  a.part_acc = work ? work + 2 * (int64_t)ccb_num_sms() * LH_ROWS * 4 : nullptr;
+}
+
+// lse[r], loss[r] = CE of row r.  Forward only.  work: ccb_lmhead_work floats, 16-byte aligned, or null.
 extern "C" int ccb_lmhead_lse(const void* X, const void* W, const float* rowss, float eps,
                               const int64_t* targets, float* lse, float* loss, float* entropy,
-                              int64_t R, int64_t V, int64_t D, void* stream) {
+                              float* work, int64_t R, int64_t V, int64_t D, void* stream) {
   LmHeadArgs a = {};
   int rc = lmhead_common(a, R, V, D, rowss, eps, targets);
   if (rc) return rc < 0 ? rc : 0;
@@ -983,6 +1160,7 @@ extern "C" int ccb_lmhead_lse(const void* X, const void* W, const float* rowss, 
   a.loss = loss;
   a.entropy = entropy;
   a.X = (const __nv_bfloat16*)X;      // rows are copied into tensor memory for the logits MMA
+  lh_workspace(a, work);
   return launch_lmhead<MODE_LSE>(X, W, a, (cudaStream_t)stream);
 }
 
@@ -991,8 +1169,8 @@ extern "C" int ccb_lmhead_lse(const void* X, const void* W, const float* rowss, 
 // 2 = one sweep with a fixed per-row reference (MODE_TRAIN1), lse[] is written.
 extern "C" int ccb_lmhead_train(const void* X, const void* W, const float* rowss, float eps,
                                 const int64_t* targets, const float* rowweight, float gscale,
-                                const float* gscale_dev, float* lse, int64_t lse_is_input, float* loss, void* dX, int64_t R,
-                                int64_t V, int64_t D, void* stream) {
+                                const float* gscale_dev, float* lse, int64_t lse_is_input, float* loss, void* dX, float* work,
+                                int64_t R, int64_t V, int64_t D, void* stream) {
   LmHeadArgs a = {};
   int rc = lmhead_common(a, R, V, D, rowss, eps, targets);
   if (rc) return rc < 0 ? rc : 0;
@@ -1005,6 +1183,7 @@ extern "C" int ccb_lmhead_train(const void* X, const void* W, const float* rowss
   a.X = (const __nv_bfloat16*)X;
   a.dX = (__nv_bfloat16*)dX;
   a.W = (const __nv_bfloat16*)W;
+  if (lse_is_input != 0) lh_workspace(a, work);        // one sweep: it may be split
   if (lse_is_input == 2) return launch_lmhead<MODE_TRAIN1>(X, W, a, (cudaStream_t)stream);
   return launch_lmhead<MODE_TRAIN>(X, W, a, (cudaStream_t)stream);
 }

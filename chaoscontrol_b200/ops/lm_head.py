@@ -17,8 +17,9 @@ from . import _lib
 from . import gemm as G
 from ._lib import f32, i64, vp
 
-_lib.register_sig("ccb_lmhead_lse", [vp, vp, vp, f32, vp, vp, vp, vp, i64, i64, i64, vp])
-_lib.register_sig("ccb_lmhead_train", [vp, vp, vp, f32, vp, vp, f32, vp, vp, i64, vp, vp, i64, i64, i64, vp])
+_lib.register_sig("ccb_lmhead_work", [i64, i64, i64, i64], i64)
+_lib.register_sig("ccb_lmhead_lse", [vp, vp, vp, f32, vp, vp, vp, vp, vp, i64, i64, i64, vp])
+_lib.register_sig("ccb_lmhead_train", [vp, vp, vp, f32, vp, vp, f32, vp, vp, i64, vp, vp, vp, i64, i64, i64, vp])
 _lib.register_sig("ccb_lmhead_dw", [vp, vp, vp, f32, vp, vp, f32, vp, vp, vp, i64, i64, i64, i64, vp])
 
 EPS = 1e-6
@@ -174,6 +175,12 @@ def _lse_materialized(x, rowss, W_f, targets, eps, want_entropy, max_logit_bytes
     return rows, lse
 
 
+def _split_work(x, W_f, train: bool):
+    """Workspace of an evenly dealt vocabulary sweep, or None where whole row tiles fill the SMs as well."""
+    n = int(_lib.lib().ccb_lmhead_work(x.shape[0], W_f.shape[0], x.shape[1], int(train)))
+    return torch.empty(n, dtype=torch.float32, device=x.device) if n else None
+
+
 def lm_head_lse(x, rowss, W_f, targets, *, eps: float = EPS, want_entropy: bool = False,
                 allow_materialized: bool = False):
     """Forward only: ``(loss_rows, lse)`` fp32 ``[R]`` (plus the softmax entropy
@@ -191,7 +198,7 @@ def lm_head_lse(x, rowss, W_f, targets, *, eps: float = EPS, want_entropy: bool 
     ent = torch.empty(R, dtype=torch.float32, device=x.device) if want_entropy else None
     _lib.check(_lib.lib().ccb_lmhead_lse(x.data_ptr(), W_f.data_ptr(), _lib.ptr(rowss), eps,
                                          t.data_ptr(), lse.data_ptr(), loss.data_ptr(), _lib.ptr(ent),
-                                         R, W_f.shape[0], D, _lib.stream_ptr()), "lmhead_lse")
+                                         _lib.ptr(_split_work(x, W_f, False)), R, W_f.shape[0], D, _lib.stream_ptr()), "lmhead_lse")
     return (loss, lse, ent) if want_entropy else (loss, lse)
 
 
@@ -268,8 +275,8 @@ def lm_head_train(x, rowss, W_f, targets, *, gscale: float, rowweight=None, eps:
     _lib.check(L.ccb_lmhead_train(x.data_ptr(), W_f.data_ptr(), _lib.ptr(rowss), eps, t.data_ptr(),
                                   _lib.ptr(rowweight), gscale, _lib.ptr(gscale_dev), lse.data_ptr(),
                                   1 if lse_given else (2 if (ONE_SWEEP if one_sweep is None else one_sweep) else 0),
-                                  loss.data_ptr(), dX.data_ptr(), R, V, D, _lib.stream_ptr()),
-               "lmhead_train")
+                                  loss.data_ptr(), dX.data_ptr(), _lib.ptr(_split_work(x, W_f, True)), R, V, D,
+                                  _lib.stream_ptr()), "lmhead_train")
     if not want_dw:
         return loss, lse, dX, None
     C = row_chunks or default_row_chunks(R, V)

@@ -180,3 +180,39 @@ def test_lse_combine_partials(nparts, M):
     tol = (nparts + 8) * 2.0 ** -23 + 2.0 ** -23 * ref.abs()
     assert ((lse.double() - ref).abs() <= tol).all()
     assert ((loss.double() - (ref - zt.double())).abs() <= tol + 2.0 ** -23 * zt.abs().double()).all()
+
+
+# row tiles: fewer than SMs, one more, several waves; vocabularies whose tiles divide the shares and not; a last row
+# tile that is not full
+@pytest.mark.parametrize("R,V", [(4096, 4096), (9000, 4352), (18944 + 60, 4096), (18944 + 128, 2304), (40000, 2560)])
+@pytest.mark.parametrize("norm", [False, True])
+def test_evenly_dealt_sweeps_match_whole_tiles(R, V, norm):
+    """The split walk against whole row tiles, kernel by kernel.  lse, loss and entropy differ by the order of fp32
+    sums; dX by that and one bf16 rounding."""
+    x, W, t, ss = _mk_d(R, V, 256, wscale=0.3, seed=7)
+    rowss = ss if norm else None
+    w = torch.rand(R, device="cuda")
+    L = _lib.lib()
+    assert L.ccb_lmhead_work(R, V, 256, 1) > 0
+    res = []
+    real = LH._split_work
+    for split in (True, False):
+        LH._split_work = real if split else (lambda *a: None)
+        try:
+            row = list(LH.lm_head_lse(x, rowss, W, t, want_entropy=True))
+            for kw in (dict(lse=row[1]), dict(one_sweep=True)):
+                l, z, dX, _ = LH.lm_head_train(x, rowss, W, t, gscale=0.5, rowweight=w, want_dw=False, **kw)
+                row += [l, z, dX]
+        finally:
+            LH._split_work = real
+        res.append(row)
+    _lib.assert_ok()
+    for i, (a, b) in enumerate(zip(*res)):
+        a, b = a.float(), b.float()
+        if a.dim() == 1:
+            assert (a - b).abs().max().item() <= 2e-4 * (1.0 + b.abs().max().item()), i
+        else:
+            assert (a - b).abs().max().item() <= 2.0 ** -7 * b.abs().max().item(), i
+            assert (a - b).norm() <= 2e-3 * b.norm(), i
+    again = LH.lm_head_train(x, rowss, W, t, gscale=0.5, rowweight=w, want_dw=False, one_sweep=True)
+    assert torch.equal(again[2], res[0][8])
