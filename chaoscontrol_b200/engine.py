@@ -9,10 +9,11 @@ what ``train_ssm_step`` runs when the model qualifies
 Kernel schedule of one step (L layers)::
 
     embed gather (+row ss)                                   1 launch
-    per layer fwd: 2 weight folds, 4 GEMMs, 1 scan           7 launches
-    LM head: fold, lse+dX kernel, dW kernel, split-K reduce  5 launches
-    per layer bwd: 4 dX GEMMs, 4 dW GEMMs + reduces, 1 scan  ~16 launches
-    embedding backward (sort + scatter-add)                  3 launches
+    per layer fwd: weight fold, 4 GEMMs, 1 scan              6 launches, one native call
+    LM head: fold, lse+dX kernel (+ join), dW kernel,
+             split-K reduce and column sum                   5-6 launches
+    per layer bwd: 4 dX GEMMs, 4 dW GEMMs + reduces, 1 scan  16 launches, one native call
+    embedding backward (keys, sort, runs, join)              4 launches and the sort's own
 """
 from __future__ import annotations
 
