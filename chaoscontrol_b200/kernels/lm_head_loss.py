@@ -57,10 +57,11 @@ class _RmsNormFn(torch.autograd.Function):
         gx = torch.empty_like(x2)
         nb = int(_lib.lib().ccb_rmsnorm_bwd_blocks(R))
         part = torch.empty(nb, D, dtype=torch.float32, device=x2.device)
-        gw = torch.empty(D, dtype=torch.float32, device=x2.device)
-        _lib.check(_lib.lib().ccb_rmsnorm_bwd(x2.data_ptr(), w.data_ptr(), go2.data_ptr(),
-                                              inv.data_ptr(), gx.data_ptr(), part.data_ptr(),
-                                              gw.data_ptr(), R, D, _lib.stream_ptr()), "rmsnorm_bwd")
+        gdt = torch.bfloat16 if ctx.wdtype == torch.bfloat16 else torch.float32
+        gw = torch.empty(D, dtype=gdt, device=x2.device)
+        _lib.check(_lib.lib().ccb_rmsnorm_bwd_as(x2.data_ptr(), w.data_ptr(), go2.data_ptr(), inv.data_ptr(),
+                                                 gx.data_ptr(), part.data_ptr(), gw.data_ptr(),
+                                                 int(gdt == torch.bfloat16), R, D, _lib.stream_ptr()), "rmsnorm_bwd")
         return gx.view(ctx.shp), gw.to(ctx.wdtype), None
 
 

@@ -104,6 +104,9 @@ _SIGS = {
     "ccb_rmsnorm_fwd": ([vp, vp, vp, vp, vp, vp, i64, i64, f32, vp], C.c_int),
     "ccb_rmsnorm_bwd_blocks": ([i64], i64),
     "ccb_rmsnorm_bwd": ([vp, vp, vp, vp, vp, vp, vp, i64, i64, vp], C.c_int),
+    "ccb_rmsnorm_bwd_as": ([vp, vp, vp, vp, vp, vp, vp, i64, i64, i64, vp], C.c_int),
+    "ccb_colsum_bf16_blocks": ([i64, i64], i64),
+    "ccb_colsum_bf16": ([vp, i64, i64, vp, vp, i64, vp], C.c_int),
     "ccb_muon_momentum": ([vp, vp, vp, vp, i64, i64, f32, i64, vp], C.c_int),
     "ccb_muon_normalize": ([vp, vp, i64, i64, f32, vp], C.c_int),
     "ccb_muon_apply": ([vp, vp, i64, f32, f32, vp], C.c_int),

@@ -163,10 +163,12 @@ class _RmsNormQuantFn(torch.autograd.Function):
             gx = torch.empty_like(x2)
             nb = int(_lib.lib().ccb_rmsnorm_bwd_blocks(R))
             part = torch.empty(nb, D, dtype=torch.float32, device=x2.device)
-            gw = torch.empty(D, dtype=torch.float32, device=x2.device)
-            _lib.check(_lib.lib().ccb_rmsnorm_bwd(x2.data_ptr(), w.data_ptr(), go2.data_ptr(), inv.data_ptr(),
-                                                  gx.data_ptr(), part.data_ptr(), gw.data_ptr(), R, D,
-                                                  _lib.stream_ptr()), "rmsnorm_bwd")
+            gdt = torch.bfloat16 if weight.dtype == torch.bfloat16 else torch.float32
+            gw = torch.empty(D, dtype=gdt, device=x2.device)
+            _lib.check(_lib.lib().ccb_rmsnorm_bwd_as(x2.data_ptr(), w.data_ptr(), go2.data_ptr(), inv.data_ptr(),
+                                                     gx.data_ptr(), part.data_ptr(), gw.data_ptr(),
+                                                     int(gdt == torch.bfloat16), R, D, _lib.stream_ptr()),
+                       "rmsnorm_bwd")
             return gx.view(ctx.shp), gw.to(weight.dtype), None
         xf, g = x2.float(), go2.float() * weight.to(torch.bfloat16).float()
         xn = xf * inv[:, None]
@@ -226,8 +228,24 @@ class _BlockFP8LinearFn(torch.autograd.Function):
                 gw = g2.float().t() @ xb.float()
             gw = gw.to(wdtype)
         if has_bias and ctx.needs_input_grad[2]:
-            gb = g2.float().sum(0).to(wdtype)
+            gb = _bias_grad(g2, wdtype)
         return gx, gw, gb, None
+
+
+def _bias_grad(g: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """Column sums of a contiguous bf16 ``[R, N]`` in ``dtype``."""
+    if _use_kernels(g) and g.numel() > 0:
+        R, N = g.shape
+        L = _lib.lib()
+        odt = torch.bfloat16 if dtype == torch.bfloat16 else torch.float32
+        part = torch.empty(L.ccb_colsum_bf16_blocks(R, N), N, dtype=torch.float32, device=g.device)
+        out = torch.empty(N, dtype=odt, device=g.device)
+        rc = L.ccb_colsum_bf16(g.data_ptr(), R, N, part.data_ptr(), out.data_ptr(), int(odt == torch.bfloat16),
+                               _lib.stream_ptr())
+        if rc <= 0:
+            _lib.check(rc, "colsum_bf16")
+            return out.to(dtype)
+    return g.float().sum(0).to(dtype)
 
 
 def _dequant_t(qt: torch.Tensor, s: torch.Tensor, N: int, K: int) -> torch.Tensor:

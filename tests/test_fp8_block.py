@@ -194,3 +194,17 @@ def test_block_gemm_resident_weights(R, K, N, out_dtype):
     rnd = 2.0 ** -8 if out_dtype is torch.bfloat16 else 0.0
     assert ((out.double() - ref).abs() <= (K + 8) * 2.0 ** -24 * mag + rnd * ref.abs()).all()
     assert torch.equal(out, FB.block_gemm(qa, q, s, sb_strides=(s.shape[1], 1), bias=bias, out_dtype=out_dtype))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("R,N", [(1, 8), (31, 256), (33, 264), (4097, 1024), (70001, 136), (50, 12)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+def test_bias_gradient_column_sums(R, N, dt):
+    """R fp32 additions a column in a fixed order, rounded once (N = 12: the PyTorch statement)."""
+    g = torch.Generator(device="cuda").manual_seed(R + N)
+    x = torch.randn(R, N, generator=g, device="cuda").bfloat16()
+    got = FB._bias_grad(x, dt)
+    ref, mag = x.double().sum(0), x.double().abs().sum(0)
+    rnd = 2.0 ** -8 if dt is torch.bfloat16 else 0.0
+    assert got.dtype == dt and ((got.double() - ref).abs() <= (R + 1) * 2.0 ** -24 * mag + rnd * ref.abs()).all()
+    assert torch.equal(got, FB._bias_grad(x, dt))
