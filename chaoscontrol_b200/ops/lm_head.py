@@ -176,7 +176,8 @@ def _lse_materialized(x, rowss, W_f, targets, eps, want_entropy, max_logit_bytes
 
 
 def _split_work(x, W_f, train: bool):
-    """Workspace of an evenly dealt vocabulary sweep, or None where whole row tiles fill the SMs as well."""
+    """Workspace of an evenly dealt vocabulary sweep, or None where whole row tiles fill the SMs as well.
+    The caller keeps the tensor until the kernels that use it have been launched."""
     n = int(_lib.lib().ccb_lmhead_work(x.shape[0], W_f.shape[0], x.shape[1], int(train)))
     return torch.empty(n, dtype=torch.float32, device=x.device) if n else None
 
@@ -196,9 +197,10 @@ def lm_head_lse(x, rowss, W_f, targets, *, eps: float = EPS, want_entropy: bool 
     lse = torch.empty(R, dtype=torch.float32, device=x.device)
     loss = torch.empty(R, dtype=torch.float32, device=x.device)
     ent = torch.empty(R, dtype=torch.float32, device=x.device) if want_entropy else None
+    work = _split_work(x, W_f, False)
     _lib.check(_lib.lib().ccb_lmhead_lse(x.data_ptr(), W_f.data_ptr(), _lib.ptr(rowss), eps,
                                          t.data_ptr(), lse.data_ptr(), loss.data_ptr(), _lib.ptr(ent),
-                                         _lib.ptr(_split_work(x, W_f, False)), R, W_f.shape[0], D, _lib.stream_ptr()), "lmhead_lse")
+                                         _lib.ptr(work), R, W_f.shape[0], D, _lib.stream_ptr()), "lmhead_lse")
     return (loss, lse, ent) if want_entropy else (loss, lse)
 
 
@@ -272,10 +274,11 @@ def lm_head_train(x, rowss, W_f, targets, *, gscale: float, rowweight=None, eps:
     loss = torch.empty(R, dtype=torch.float32, device=dev)
     dX = torch.empty_like(x)
     L = _lib.lib()
+    work = _split_work(x, W_f, True)
     _lib.check(L.ccb_lmhead_train(x.data_ptr(), W_f.data_ptr(), _lib.ptr(rowss), eps, t.data_ptr(),
                                   _lib.ptr(rowweight), gscale, _lib.ptr(gscale_dev), lse.data_ptr(),
                                   1 if lse_given else (2 if (ONE_SWEEP if one_sweep is None else one_sweep) else 0),
-                                  loss.data_ptr(), dX.data_ptr(), _lib.ptr(_split_work(x, W_f, True)), R, V, D,
+                                  loss.data_ptr(), dX.data_ptr(), _lib.ptr(work), R, V, D,
                                   _lib.stream_ptr()), "lmhead_train")
     if not want_dw:
         return loss, lse, dX, None
