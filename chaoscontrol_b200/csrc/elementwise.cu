@@ -959,10 +959,11 @@ __global__ void sgd_kernel(__nv_bfloat16* __restrict__ p, const float* __restric
 // itself, 26 us for the 511 rows of an evaluation chunk whose logits GEMM takes 12; 4 us with this split.
 constexpr int LSC_WARPS = 16;
 __device__ __forceinline__ void lse_merge(float2& a, const float2 v) {
-  // a partial whose sum is zero or not a number adds nothing, whatever its maximum
-  if (v.y > 0.f) {
+  // An empty partial (sum zero) adds nothing, whatever its maximum.  Every other one is merged, so that a sum that is
+  // not a number (a NaN logit, or an infinite one: the tile's own inf - inf) makes the row's result one as well.
+  if (v.y != 0.f) {
     const float m = fmaxf(a.x, v.x);
-    a.y = (a.y > 0.f ? a.y * exp2f(a.x - m) : 0.f) + v.y * exp2f(v.x - m);
+    a.y = (a.y != 0.f ? a.y * exp2f(a.x - m) : 0.f) + v.y * exp2f(v.x - m);
     a.x = m;
   }
 }

@@ -662,13 +662,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             for (int i = 0; i < 32; ++i)
               if (i < nvalid) mx = fmaxf(mx, v[i]);
             const float new_m = fmaxf(run_m, mx * lm_c1);
+            // while every logit so far is -inf their sum is zero, not the NaN of inf - inf
+            const float ref = new_m == -INFINITY ? 0.f : new_m;
             float sacc = 0.f;
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
-              if (i < nvalid) sacc += gemm_ex2(fmaf(v[i], lm_c1, -new_m));
+              if (i < nvalid) sacc += gemm_ex2(fmaf(v[i], lm_c1, -ref));
               if (i == tl) { lm_zt = v[i] * rs; lm_hit = true; }
             }
-            run_s = run_s * gemm_ex2(run_m - new_m) + sacc;
+            run_s = run_s * gemm_ex2(run_m - ref) + sacc;
             run_m = new_m;
             return;   // nothing is stored per column
           }

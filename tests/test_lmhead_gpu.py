@@ -216,3 +216,51 @@ def test_evenly_dealt_sweeps_match_whole_tiles(R, V, norm):
             assert (a - b).norm() <= 2e-3 * b.norm(), i
     again = LH.lm_head_train(x, rowss, W, t, gscale=0.5, rowweight=w, want_dw=False, one_sweep=True)
     assert torch.equal(again[2], res[0][8])
+
+
+@pytest.mark.parametrize("nparts", [2, 17, 130])
+@pytest.mark.parametrize("bad", [(float("inf"), float("nan")), (3.0, float("nan")), (float("-inf"), float("nan"))])
+def test_lse_combine_lets_a_broken_partial_through(nparts, bad):
+    """A tile that held an infinite or NaN logit arrives with a NaN sum: the row's lse and loss are NaN, wherever the
+    partial stands and whether or not the others are empty; rows without one are untouched."""
+    M = nparts + 40
+    g = torch.Generator(device="cuda").manual_seed(nparts)
+    part = torch.stack([torch.randn(nparts, M, generator=g, device="cuda"),
+                        torch.rand(nparts, M, generator=g, device="cuda") + 0.5], -1).contiguous()
+    clean = part.clone()
+    for i in range(nparts):
+        part[i, i] = torch.tensor(bad)           # row i: the i-th partial
+    part[:, nparts, 1] = 0.0                     # only the broken one is not empty
+    part[nparts // 2, nparts] = torch.tensor(bad)
+    zt = torch.zeros(M, device="cuda")
+
+    def combine(p):
+        lse, loss = torch.empty(M, device="cuda"), torch.empty(M, device="cuda")
+        _lib.check(_lib.lib().ccb_lse_combine(p.data_ptr(), nparts, M, zt.data_ptr(), lse.data_ptr(), loss.data_ptr(),
+                                              _lib.stream_ptr()), "lse_combine")
+        return lse, loss
+    for a, b in zip(combine(part), combine(clean)):
+        assert a[: nparts + 1].isnan().all()
+        assert b.isfinite().all() and torch.equal(a[nparts + 1:], b[nparts + 1:])
+
+
+@pytest.mark.parametrize("R,D", [(511, 256), (300, 384)])
+def test_infinite_logits_reach_the_loss(R, D):
+    """Scoring with a damaged head: a vocabulary row whose logit is +inf makes every loss non-finite, a whole tile of
+    -inf logits has probability zero and changes nothing else (against 32-bit logits of the other columns; tolerance of
+    the scoring tests)."""
+    V = 1024
+    g = torch.Generator(device="cuda").manual_seed(D)
+    x = (torch.rand(R, D, generator=g, device="cuda") + 0.5).bfloat16()          # positive: the overflow has one sign
+    W = (torch.randn(V, D, generator=g, device="cuda") * 0.05).bfloat16()
+    t = torch.randint(0, 256, (R,), generator=g, device="cuda")
+    up, down = W.clone(), W.clone()
+    up[700] = 3e38
+    down[256:512] = -3e38
+    loss, lse = LH.lm_head_lse(x, None, up, t)
+    assert not loss.isfinite().any() and not lse.isfinite().any()
+    loss, lse = LH.lm_head_lse(x, None, down, t)
+    _lib.assert_ok()
+    keep = torch.cat([W[:256], W[512:]])
+    rl, rlse, _, _ = LH.lm_head_reference(x, None, keep, t, want_grads=False)
+    assert torch.allclose(lse, rlse, rtol=1e-3, atol=2e-2) and torch.allclose(loss, rl, rtol=1e-3, atol=3e-2)
