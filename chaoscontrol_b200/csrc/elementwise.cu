@@ -277,8 +277,9 @@ embed_bwd_join_kernel(const long long* __restrict__ first_pos, const long long* 
 }
 
 // ---------------------------------------------------------------------------
-// Split-K reduction.  out[n,k] (+)= colscale[k] * sum_s part[s,n,k], stored as fp32 or bf16
-// (the parameter's own dtype, so no cast pass follows); when W is given also emits per-row-block
+// Split-K reduction.  out[n,k] (+)= colscale[k] * (scale *) sum_s part[s,n,k], stored as fp32 or bf16
+// (the parameter's own dtype, so no cast pass follows; `scale`, one fp32 value on the device, multiplies the fp32
+// sum); when W is given also emits per-row-block
 // partial column sums of sum[n,k] * W[n,k] (the gradient of an RMSNorm weight folded into W),
 // reduced by a second tiny kernel so the result is deterministic.
 //
@@ -307,7 +308,7 @@ template <int G, typename OT>
 __global__ void __launch_bounds__(128 * G)
 splitk_tile_kernel(const float* __restrict__ part, int S, long long split_stride, int N, int K,
                    const __nv_bfloat16* __restrict__ colscale, const __nv_bfloat16* __restrict__ W,
-                   OT* __restrict__ out, float* __restrict__ colpart) {
+                   const float* __restrict__ scale, OT* __restrict__ out, float* __restrict__ colpart) {
   __shared__ float4 join[G > 1 ? (G - 1) * 128 : 1];
   __shared__ float4 colj[128];
   const int slot = threadIdx.x & 127, g = threadIdx.x >> 7;
@@ -342,6 +343,10 @@ splitk_tile_kernel(const float* __restrict__ part, int S, long long split_stride
   if (g == 0) {
     float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
     if (ok) {
+      if (scale != nullptr) {
+        const float up = __ldg(scale);
+        acc.x *= up; acc.y *= up; acc.z *= up; acc.w *= up;
+      }
       if (W != nullptr) {
         const uint2 q = __ldg(reinterpret_cast<const uint2*>(W + o));
         const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y);
@@ -374,8 +379,9 @@ splitk_tile_kernel(const float* __restrict__ part, int S, long long split_stride
 template <typename OT>
 __global__ void splitk_reduce_kernel(const float* __restrict__ part, int S, long long split_stride,
                                      int N, int K, const __nv_bfloat16* __restrict__ colscale,
-                                     const __nv_bfloat16* __restrict__ W, OT* __restrict__ out,
-                                     int accumulate, float* __restrict__ colpart) {
+                                     const __nv_bfloat16* __restrict__ W, const float* __restrict__ scale,
+                                     OT* __restrict__ out, int accumulate, float* __restrict__ colpart) {
+  const float up = scale ? __ldg(scale) : 1.f;
   const int n0 = blockIdx.x * SPK_ROWS;
   for (int k = threadIdx.x; k < K; k += blockDim.x) {
     const float cs = colscale ? __bfloat162float(colscale[k]) : 1.f;
@@ -394,6 +400,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int S, long
           s += v0; s += v1; s += v2; s += v3;
         }
         for (; sp < S; ++sp) s += pp[(long long)sp * split_stride];
+        s *= up;
         const long long o = (long long)n * K + k;
         if (W) cacc += s * __bfloat162float(W[o]);
         const float val = s * cs;
@@ -1117,8 +1124,8 @@ static int launch_colsum(const float* part, int64_t NB, int64_t K, void* out, in
 
 template <typename OT>
 static int launch_splitk(const float* part, int64_t S, int64_t split_stride, int64_t N, int64_t K,
-                         const __nv_bfloat16* colscale, const __nv_bfloat16* W, OT* out, int64_t accumulate,
-                         float* colpart, cudaStream_t s) {
+                         const __nv_bfloat16* colscale, const __nv_bfloat16* W, const float* scale, OT* out,
+                         int64_t accumulate, float* colpart, cudaStream_t s) {
   const unsigned nb = (unsigned)((N + SPK_ROWS - 1) / SPK_ROWS);
   const uintptr_t wide = (uintptr_t)part | (uintptr_t)out;                  // 16-byte accesses
   const uintptr_t half = (uintptr_t)colscale | (uintptr_t)W;                // 8-byte accesses
@@ -1127,30 +1134,30 @@ static int launch_splitk(const float* part, int64_t S, int64_t split_stride, int
   if (tile) {
     const dim3 grid(nb, (unsigned)((K + SPK_COLS - 1) / SPK_COLS));
     // groups: each keeps at least four partials, so that its loads are in flight together
-    if (S <= 4) splitk_tile_kernel<1, OT><<<grid, 128, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out, colpart);
-    else if (S <= 8) splitk_tile_kernel<2, OT><<<grid, 256, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out, colpart);
-    else if (S <= 24) splitk_tile_kernel<4, OT><<<grid, 512, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out, colpart);
-    else splitk_tile_kernel<8, OT><<<grid, 1024, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out, colpart);
+    if (S <= 4) splitk_tile_kernel<1, OT><<<grid, 128, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out, colpart);
+    else if (S <= 8) splitk_tile_kernel<2, OT><<<grid, 256, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out, colpart);
+    else if (S <= 24) splitk_tile_kernel<4, OT><<<grid, 512, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out, colpart);
+    else splitk_tile_kernel<8, OT><<<grid, 1024, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out, colpart);
   } else {
-    splitk_reduce_kernel<OT><<<nb, 256, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, out,
+    splitk_reduce_kernel<OT><<<nb, 256, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out,
                                                 (int)accumulate, colpart);
   }
   CCB_CHECK_LAUNCH("splitk_reduce");
   return 0;
 }
 
-// `out` and `colsum_out` are fp32, or bf16 with out_bf16.
+// `out` and `colsum_out` are fp32, or bf16 with out_bf16; `scale` (device, may be null) multiplies the sums.
 extern "C" int ccb_splitk_reduce_as(const float* part, int64_t S, int64_t split_stride, int64_t N, int64_t K,
-                                    const void* colscale, const void* W, void* out, int64_t out_bf16,
-                                    int64_t accumulate, float* colpart, void* colsum_out,
+                                    const void* colscale, const void* W, const float* scale, void* out,
+                                    int64_t out_bf16, int64_t accumulate, float* colpart, void* colsum_out,
                                     int64_t colsum_accumulate, void* stream) {
   if (N <= 0 || K <= 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   const __nv_bfloat16* cs = (const __nv_bfloat16*)colscale;
   const __nv_bfloat16* w = (const __nv_bfloat16*)W;
   float* cp = W ? colpart : nullptr;
-  const int rc = out_bf16 ? launch_splitk(part, S, split_stride, N, K, cs, w, (__nv_bfloat16*)out, accumulate, cp, s)
-                          : launch_splitk(part, S, split_stride, N, K, cs, w, (float*)out, accumulate, cp, s);
+  const int rc = out_bf16 ? launch_splitk(part, S, split_stride, N, K, cs, w, scale, (__nv_bfloat16*)out, accumulate, cp, s)
+                          : launch_splitk(part, S, split_stride, N, K, cs, w, scale, (float*)out, accumulate, cp, s);
   if (rc) return rc;
   if (cp && colsum_out)
     return launch_colsum(cp, (N + SPK_ROWS - 1) / SPK_ROWS, K, colsum_out, (int)out_bf16, colsum_accumulate, s);
@@ -1161,7 +1168,7 @@ extern "C" int ccb_splitk_reduce(const float* part, int64_t S, int64_t split_str
                                  int64_t K, const void* colscale, const void* W, float* out,
                                  int64_t accumulate, float* colpart, float* colsum_out,
                                  int64_t colsum_accumulate, void* stream) {
-  return ccb_splitk_reduce_as(part, S, split_stride, N, K, colscale, W, out, 0, accumulate, colpart,
+  return ccb_splitk_reduce_as(part, S, split_stride, N, K, colscale, W, nullptr, out, 0, accumulate, colpart,
                               colsum_out, colsum_accumulate, stream);
 }
 

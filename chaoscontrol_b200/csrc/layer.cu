@@ -19,8 +19,8 @@ int ccb_scan_bwd(const void* P, int64_t ldp, const float* log_a, const float* h0
                  const float* dhT, const float* rowss, float inv_dim, float eps, void* dP, int64_t lddp,
                  float* dloga_part, float* dh0, int64_t B, int64_t T, int64_t D, int64_t la_bstride, void* stream);
 int ccb_splitk_reduce_as(const float* part, int64_t S, int64_t split_stride, int64_t N, int64_t K, const void* colscale,
-                         const void* W, void* out, int64_t out_bf16, int64_t accumulate, float* colpart,
-                         void* colsum_out, int64_t colsum_accumulate, void* stream);
+                         const void* W, const float* scale, void* out, int64_t out_bf16, int64_t accumulate,
+                         float* colpart, void* colsum_out, int64_t colsum_accumulate, void* stream);
 int ccb_colsum_as(const float* part, int64_t NB, int64_t K, void* out, int64_t out_bf16, int64_t accumulate, void* stream);
 
 typedef struct CcbLayerArgs {
@@ -93,7 +93,7 @@ static int wgrad(const void* dy, int64_t N, const void* x, int64_t K, int64_t R,
   a.splits = wgrad_splits(N, K, R);
   a.c_split = a.splits > 1 ? N * K : 0;
   if (int rc = ccb_gemm(&a, s)) return rc;
-  return ccb_splitk_reduce_as(part, a.splits, N * K, N, K, wn, W, out, out_bf16, 0, colpart, dwn, 0, s);
+  return ccb_splitk_reduce_as(part, a.splits, N * K, N, K, wn, W, nullptr, out, out_bf16, 0, colpart, dwn, 0, s);
 }
 
 }  // namespace ccb

@@ -75,7 +75,7 @@ struct LmHeadArgs {
   const long long* targets; // [R]
   const float* rowweight;   // [R] or null
   float gscale;             // d loss / d (per-row CE), e.g. 1/R
-  const float* gscale_dev;  // optional device scalar that multiplies gscale (an upstream gradient)
+  const float* gscale_dev;  // optional device scalar that multiplies dX as it is rounded (an upstream gradient)
   float* lse;               // [R] natural-log lse (out in LSE/TRAIN, in for DW)
   float* loss;              // [R] per-row CE (out, LSE/TRAIN)
   float* entropy;           // [R] softmax entropy in nats (out, LSE; optional)
@@ -410,7 +410,7 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
     const int row_in_tile = q * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     float* xchg = reinterpret_cast<float*>(smem + LH_OFF_X);     // [PARTS][128]
-    const float gscale = p.gscale_dev ? p.gscale * __ldg(p.gscale_dev) : p.gscale;
+    const float up = p.gscale_dev ? __ldg(p.gscale_dev) : 1.f;
     uint32_t n_d1 = 0, n_g = 0, n_d2 = 0, n_x = 0, n_xt = 0;
     bool ok = true;
     // Every wait below is made warp-uniform, so the warp-collective TMEM loads
@@ -465,7 +465,7 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         c1 = rs * LOG2E;
         tgt = row_ok ? (int)p.targets[r] : -1;
         const float w = (row_ok && p.rowweight) ? p.rowweight[r] : 1.f;
-        gs = row_ok ? gscale * w * rs : 0.f;
+        gs = row_ok ? p.gscale * w * rs : 0.f;
         if (need_lse) c2 = row_ok ? p.lse[r] * LOG2E : 0.f;
       };
       if (MODE != MODE_DW) load_row(unit, MODE == MODE_TRAIN && p.skip_lse);
@@ -530,7 +530,7 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         };
         auto scale_of = [&](const RawRow& x, float& rsv) -> float {
           rsv = p.rowss ? rsqrtf(x.ss * p.inv_dim + p.eps) : 1.f;
-          return gscale * x.w * rsv;
+          return p.gscale * x.w * rsv;
         };
         RawRow wraw = {0.f, INFINITY, 0.f, -1}, graw[NG];
         if (writer) wraw = fetch_raw(inner0 * LH_ROWS + row_in_tile);
@@ -903,10 +903,10 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
                   const float2 f0 = unpack_bf16x2(qv.x), f1 = unpack_bf16x2(qv.y),
                                f2 = unpack_bf16x2(qv.z), f3 = unpack_bf16x2(qv.w);
                   uint4 o;
-                  o.x = pack_bf16x2(__uint_as_float(a[j * 8 + 0]) - f0.x * coef, __uint_as_float(a[j * 8 + 1]) - f0.y * coef);
-                  o.y = pack_bf16x2(__uint_as_float(a[j * 8 + 2]) - f1.x * coef, __uint_as_float(a[j * 8 + 3]) - f1.y * coef);
-                  o.z = pack_bf16x2(__uint_as_float(a[j * 8 + 4]) - f2.x * coef, __uint_as_float(a[j * 8 + 5]) - f2.y * coef);
-                  o.w = pack_bf16x2(__uint_as_float(a[j * 8 + 6]) - f3.x * coef, __uint_as_float(a[j * 8 + 7]) - f3.y * coef);
+                  o.x = pack_bf16x2((__uint_as_float(a[j * 8 + 0]) - f0.x * coef) * up, (__uint_as_float(a[j * 8 + 1]) - f0.y * coef) * up);
+                  o.y = pack_bf16x2((__uint_as_float(a[j * 8 + 2]) - f1.x * coef) * up, (__uint_as_float(a[j * 8 + 3]) - f1.y * coef) * up);
+                  o.z = pack_bf16x2((__uint_as_float(a[j * 8 + 4]) - f2.x * coef) * up, (__uint_as_float(a[j * 8 + 5]) - f2.y * coef) * up);
+                  o.w = pack_bf16x2((__uint_as_float(a[j * 8 + 6]) - f3.x * coef) * up, (__uint_as_float(a[j * 8 + 7]) - f3.y * coef) * up);
                   o4[j] = o;
                 }
               }
@@ -1004,8 +1004,8 @@ __global__ void __launch_bounds__(256) lmhead_join_kernel(const LmHeadArgs p, in
     }
   }
   if (MODE == MODE_LSE) return;
-  const float gscale = p.gscale_dev ? p.gscale * __ldg(p.gscale_dev) : p.gscale;
-  const float gs = gscale * (p.rowweight ? p.rowweight[r] : 1.f) * rs;
+  const float up = p.gscale_dev ? __ldg(p.gscale_dev) : 1.f;
+  const float gs = p.gscale * (p.rowweight ? p.rowweight[r] : 1.f) * rs;
   auto unpack = [](const uint4& u, float (&f)[8]) {
     const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
     f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
@@ -1025,8 +1025,10 @@ __global__ void __launch_bounds__(256) lmhead_join_kernel(const LmHeadArgs p, in
   for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
   const float coef = p.rowss ? dot * rs * rs * p.inv_dim : 0.f;
   uint4 o;
-  o.x = pack_bf16x2(acc[0] - xv[0] * coef, acc[1] - xv[1] * coef); o.y = pack_bf16x2(acc[2] - xv[2] * coef, acc[3] - xv[3] * coef);
-  o.z = pack_bf16x2(acc[4] - xv[4] * coef, acc[5] - xv[5] * coef); o.w = pack_bf16x2(acc[6] - xv[6] * coef, acc[7] - xv[7] * coef);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = (acc[i] - xv[i] * coef) * up;
+  o.x = pack_bf16x2(acc[0], acc[1]); o.y = pack_bf16x2(acc[2], acc[3]);
+  o.z = pack_bf16x2(acc[4], acc[5]); o.w = pack_bf16x2(acc[6], acc[7]);
   *reinterpret_cast<uint4*>(p.dX + (long long)r * LH_D + lane * 8) = o;
 }
 
@@ -1167,6 +1169,9 @@ extern "C" int ccb_lmhead_lse(const void* X, const void* W, const float* rowss, 
 // lse, per-row loss and dX (gradient w.r.t. the un-normalised hidden state).
 // lse_is_input: 0 = two sweeps (lse, then gradient); 1 = lse[] is read, gradient sweep only;
 // 2 = one sweep with a fixed per-row reference (MODE_TRAIN1), lse[] is written.
+// gscale_dev (may be null) multiplies dX in fp32 as it is rounded.  It stays out of the bf16 gradient tile: p - onehot is
+// near -1 or small there, but -1/R of a mean loss rounds by the same factor in every row, up to 2^-8, which no sum
+// averages out.
 extern "C" int ccb_lmhead_train(const void* X, const void* W, const float* rowss, float eps,
                                 const int64_t* targets, const float* rowweight, float gscale,
                                 const float* gscale_dev, float* lse, int64_t lse_is_input, float* loss, void* dX, float* work,
@@ -1191,7 +1196,7 @@ extern "C" int ccb_lmhead_train(const void* X, const void* W, const float* rowss
 // dWpart[row_chunks, V, D] fp32: partial gradients of W' = W_lm * w_norm.
 extern "C" int ccb_lmhead_dw(const void* X, const void* W, const float* rowss, float eps,
                              const int64_t* targets, const float* rowweight, float gscale,
-                             const float* gscale_dev, const float* lse, float* dWpart, int64_t row_chunks, int64_t R,
+                             const float* lse, float* dWpart, int64_t row_chunks, int64_t R,
                              int64_t V, int64_t D, void* stream) {
   LmHeadArgs a = {};
   int rc = lmhead_common(a, R, V, D, rowss, eps, targets);
@@ -1205,7 +1210,6 @@ extern "C" int ccb_lmhead_dw(const void* X, const void* W, const float* rowss, f
                      (long long)row_chunks, a.row_chunks);
   a.rowweight = rowweight;
   a.gscale = gscale;
-  a.gscale_dev = gscale_dev;
   a.lse = const_cast<float*>(lse);
   a.dWpart = dWpart;
   a.X = (const __nv_bfloat16*)X;

@@ -93,10 +93,11 @@ class _LinearCeFn(torch.autograd.Function):
     def backward(ctx, gtotal, _gl):
         x, weight, targets, lse, rw = ctx.saved_tensors
         roww = rw.float().contiguous() if ctx.has_w else None
-        # the upstream gradient rides in the kernels' own scale: no pass over dX or dW to multiply it in
+        # the upstream gradient is multiplied in where each result is rounded: no pass over dX or dW for it
+        up = gtotal.float()
         _, _, dX, part = LH.lm_head_train(x, None, weight, targets, gscale=1.0, rowweight=roww, lse=lse,
-                                          gscale_dev=gtotal.float(), want_dw=ctx.needs_input_grad[1])
-        dW = splitk_reduce(part, out_dtype=weight.dtype)[0] if part is not None else None
+                                          gscale_dev=up, want_dw=ctx.needs_input_grad[1])
+        dW = splitk_reduce(part, out_dtype=weight.dtype, scale=up)[0] if part is not None else None
         return dX, dW, None, None
 
 

@@ -91,7 +91,7 @@ _SIGS = {
     "ccb_lmhead_debug": ([C.c_int], C.c_int),
     "ccb_lmhead_deep_ring": ([C.c_int], C.c_int),
     "ccb_splitk_reduce": ([vp, i64, i64, i64, i64, vp, vp, vp, i64, vp, vp, i64, vp], C.c_int),
-    "ccb_splitk_reduce_as": ([vp, i64, i64, i64, i64, vp, vp, vp, i64, i64, vp, vp, i64, vp], C.c_int),
+    "ccb_splitk_reduce_as": ([vp, i64, i64, i64, i64, vp, vp, vp, vp, i64, i64, vp, vp, i64, vp], C.c_int),
     "ccb_colsum": ([vp, i64, i64, vp, i64, vp], C.c_int),
     "ccb_colsum_as": ([vp, i64, i64, vp, i64, i64, vp], C.c_int),
     "ccb_fold_colscale": ([vp, vp, vp, i64, i64, vp], C.c_int),

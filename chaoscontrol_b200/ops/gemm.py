@@ -65,7 +65,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
          cin: Optional[torch.Tensor] = None, r1: Optional[torch.Tensor] = None,
          r2: Optional[torch.Tensor] = None, rowss: Optional[torch.Tensor] = None,
          inv_dim: float = 0.0, eps: float = 1e-6, c2: Optional[torch.Tensor] = None,
-         ss_out: Optional[torch.Tensor] = None, ss_atomic: bool = False) -> torch.Tensor:
+         ss_out: Optional[torch.Tensor] = None, ss_atomic: bool = False,
+         alpha_dev: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``alpha_dev`` (``EPI_STORE`` on a CUDA device): a one-element fp32 tensor that multiplies ``alpha``."""
+    if alpha_dev is not None and (epi != EPI_STORE or not a.is_cuda):
+        raise ValueError("gemm: alpha_dev is an operand of the CUDA store epilogue")
     if not a.is_cuda:
         return _gemm_cpu(a, b, a_mn=a_mn, b_mn=b_mn, out=out, out_dtype=out_dtype, splits=splits,
                          epi=epi, alpha=alpha, beta=beta, cin=cin, r1=r1, r2=r2, rowss=rowss,
@@ -110,6 +114,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     args.out_fp32 = int(out.dtype == torch.float32)
     args.ss_atomic = int(ss_atomic)
     args.alpha, args.beta, args.inv_dim, args.eps = alpha, beta, inv_dim, eps
+    args.dscale_a = _lib.ptr(alpha_dev)
     _lib.check(_lib.lib().ccb_gemm(C.byref(args), _lib.stream_ptr()), "gemm")
     return out
 
@@ -117,15 +122,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
 def gemm_lm(x: torch.Tensor, w: torch.Tensor, *, epi: int, targets: torch.Tensor,
             rowss: Optional[torch.Tensor], inv_dim: float, eps: float, lse: Optional[torch.Tensor] = None,
             rowweight: Optional[torch.Tensor] = None, alpha: float = 1.0,
-            alpha_dev: Optional[torch.Tensor] = None,
             out: Optional[torch.Tensor] = None, zt_out: Optional[torch.Tensor] = None):
     """LM-head epilogues on ``logits = rs * (x @ w.T)`` (``x`` ``[R, D]``, ``w`` ``[V, D]``, bf16, CUDA).
 
     ``EPI_LSE_PART`` returns ``(partials [2 * ceil(V / 256), R, 2] fp32, zt [R])``: log2-domain
     ``(max, sum)`` per half tile and the target logit; no logits are written.
     ``EPI_CE_GRAD`` returns the bf16 ``[R, V]`` gradient of the summed, ``alpha * rowweight``-weighted
-    cross-entropy w.r.t. the un-scaled GEMM output (``alpha_dev``, a one-element fp32 tensor, multiplies
-    ``alpha`` on the device), and fills ``zt_out`` with the per-row CE.
+    cross-entropy w.r.t. the un-scaled GEMM output, and fills ``zt_out`` with the per-row CE.
     """
     R, D = x.shape
     V = w.shape[0]
@@ -137,7 +140,6 @@ def gemm_lm(x: torch.Tensor, w: torch.Tensor, *, epi: int, targets: torch.Tensor
     args.epi = epi
     args.alpha, args.beta, args.inv_dim, args.eps = alpha, 0.0, inv_dim, eps
     args.rowss = _lib.ptr(rowss)
-    args.dscale_a = _lib.ptr(alpha_dev)
     t = targets.reshape(-1)
     if t.dtype != torch.int64:
         t = t.long()

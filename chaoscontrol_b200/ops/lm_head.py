@@ -20,7 +20,7 @@ from ._lib import f32, i64, vp
 _lib.register_sig("ccb_lmhead_work", [i64, i64, i64, i64], i64)
 _lib.register_sig("ccb_lmhead_lse", [vp, vp, vp, f32, vp, vp, vp, vp, vp, i64, i64, i64, vp])
 _lib.register_sig("ccb_lmhead_train", [vp, vp, vp, f32, vp, vp, f32, vp, vp, i64, vp, vp, vp, i64, i64, i64, vp])
-_lib.register_sig("ccb_lmhead_dw", [vp, vp, vp, f32, vp, vp, f32, vp, vp, vp, i64, i64, i64, i64, vp])
+_lib.register_sig("ccb_lmhead_dw", [vp, vp, vp, f32, vp, vp, f32, vp, vp, i64, i64, i64, i64, vp])
 
 EPS = 1e-6
 
@@ -67,7 +67,7 @@ def _train_general(x, rowss, W_f, t, gscale, rowweight, eps, lse, want_dw=True, 
     """Chunked LM-head backward from GEMM epilogues.  Per row chunk: ``g = (softmax - onehot) *
     scale`` is produced by the logits GEMM's epilogue as a bf16 ``[rows, V]`` tile (bounded by the
     chunk, never the full ``[R, V]``), then ``dX = RMSNorm-backward(g @ W')`` and
-    ``dW' += g^T @ X`` are two more tcgen05 GEMMs."""
+    ``dW' += g^T @ X`` are two more tcgen05 GEMMs.  ``gscale_dev`` multiplies ``dX`` as it is rounded."""
     R, D = x.shape
     V = W_f.shape[0]
     if lse is None:
@@ -86,12 +86,16 @@ def _train_general(x, rowss, W_f, t, gscale, rowweight, eps, lse, want_dw=True, 
         ssc = rowss[r0:r1] if rowss is not None else None
         g = G.gemm_lm(xc, W_f, epi=G.EPI_CE_GRAD, targets=t[r0:r1], rowss=ssc, inv_dim=1.0 / D, eps=eps,
                       lse=lse[r0:r1], rowweight=rowweight[r0:r1] if rowweight is not None else None,
-                      alpha=gscale, alpha_dev=gscale_dev, out=gbuf[: r1 - r0], zt_out=loss[r0:r1])
-        if rowss is not None:
+                      alpha=gscale, out=gbuf[: r1 - r0], zt_out=loss[r0:r1])
+        if rowss is None:
+            G.gemm(g, W_f, b_mn=True, out=dX[r0:r1], alpha_dev=gscale_dev)
+        elif gscale_dev is None:
             G.gemm(g, W_f, b_mn=True, epi=G.EPI_RMSBWD, r1=xc, rowss=ssc, inv_dim=1.0 / D, eps=eps,
                    out=dX[r0:r1])
         else:
-            G.gemm(g, W_f, b_mn=True, out=dX[r0:r1])
+            dx32 = G.gemm(g, W_f, b_mn=True, epi=G.EPI_RMSBWD, r1=xc, rowss=ssc, inv_dim=1.0 / D, eps=eps,
+                          out_dtype=torch.float32)
+            dX[r0:r1] = dx32 * gscale_dev
         if not want_dw:
             continue
         Sc = min(S, G.pick_splits(V, D, r1 - r0))
@@ -236,8 +240,9 @@ def lm_head_train(x, rowss, W_f, targets, *, gscale: float, rowweight=None, eps:
                   want_dw: bool = True, gscale_dev: Optional[torch.Tensor] = None):
     """Loss and both gradients.  Returns ``(loss_rows, lse, dX bf16, dW_f_partials fp32 [C,V,D])``.
 
-    ``gscale_dev``: a one-element fp32 tensor that multiplies ``gscale`` (the gradient that
-    arrives from further up), read on the device.
+    ``gscale_dev``: a one-element fp32 tensor (the gradient that arrives from further up), read on
+    the device, that multiplies ``dX`` in fp32 as it is rounded.  The partials of ``dW_f`` do not
+    carry it: hand it to their reduction (``trunk.splitk_reduce(..., scale=)``).
 
     ``want_dw=False`` skips the weight-gradient kernel and returns ``None`` in its
     place: test-time training adapts recurrence parameters only and needs ``dX``
@@ -261,10 +266,10 @@ def lm_head_train(x, rowss, W_f, targets, *, gscale: float, rowweight=None, eps:
         return _train_general(x, rowss, W_f, _prep(x, rowss, W_f, targets), gscale, rowweight, eps, lse, want_dw, gscale_dev)
     if not fused_supported(x, W_f):
         _refuse_unless_allowed(x, W_f, allow_materialized, "lm_head_train")
-        if gscale_dev is not None:
-            gscale = gscale * float(gscale_dev)
         lr, lse, dX, dW = lm_head_reference(x, rowss, W_f, targets, gscale=gscale,
                                             rowweight=rowweight, eps=eps)
+        if gscale_dev is not None:
+            dX = dX * gscale_dev
         return lr, lse, dX.to(x.dtype), dW.unsqueeze(0)
     t = _prep(x, rowss, W_f, targets)
     dev = x.device
@@ -285,6 +290,6 @@ def lm_head_train(x, rowss, W_f, targets, *, gscale: float, rowweight=None, eps:
     C = row_chunks or default_row_chunks(R, V)
     part = torch.empty(C, V, D, dtype=torch.float32, device=dev)
     _lib.check(L.ccb_lmhead_dw(x.data_ptr(), W_f.data_ptr(), _lib.ptr(rowss), eps, t.data_ptr(),
-                               _lib.ptr(rowweight), gscale, _lib.ptr(gscale_dev), lse.data_ptr(), part.data_ptr(), C, R, V,
-                               D, _lib.stream_ptr()), "lmhead_dw")
+                               _lib.ptr(rowweight), gscale, lse.data_ptr(), part.data_ptr(), C, R, V, D,
+                               _lib.stream_ptr()), "lmhead_dw")
     return loss, lse, dX, part

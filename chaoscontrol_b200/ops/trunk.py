@@ -141,13 +141,15 @@ def embed_bwd(tokens: torch.Tensor, dx: torch.Tensor, V: int,
 
 def splitk_reduce(part: torch.Tensor, *, colscale: Optional[torch.Tensor] = None,
                   W: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-                  dcol_out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.float32):
+                  dcol_out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.float32,
+                  scale: Optional[torch.Tensor] = None):
     """Sum split-K partials ``[S, N, K]`` (or ``[N, K]``).
 
     Returns ``(dW [N,K], dcol [K] or None)`` with
     ``dW = colscale * sum`` and ``dcol = sum_n sum[n,k] * W[n,k]`` -- the
     gradients of ``W`` and of the RMSNorm weight folded into it.  Results are fp32;
-    ``out_dtype=torch.bfloat16`` rounds them once, as they are stored.
+    ``out_dtype=torch.bfloat16`` rounds them once, as they are stored.  ``scale``, a one-element
+    fp32 tensor, multiplies the fp32 sums.
     """
     if part.dim() == 2:
         part = part.unsqueeze(0)
@@ -165,12 +167,14 @@ def splitk_reduce(part: torch.Tensor, *, colscale: Optional[torch.Tensor] = None
             dcol = dcol_out if dcol_out is not None else torch.empty(K, dtype=out_dtype, device=part.device)
             assert dcol.dtype == out_dtype
         _lib.check(_lib.lib().ccb_splitk_reduce_as(part.data_ptr(), S, part.stride(0), N, K,
-                                                   _lib.ptr(colscale), _lib.ptr(W), out.data_ptr(),
+                                                   _lib.ptr(colscale), _lib.ptr(W), _lib.ptr(scale), out.data_ptr(),
                                                    int(out_dtype == torch.bfloat16), 0,
                                                    _lib.ptr(colpart), _lib.ptr(dcol), 0,
                                                    _lib.stream_ptr()), "splitk_reduce")
         return out, dcol
     s = part.float().sum(0)
+    if scale is not None:
+        s = s * scale
     dcol = (s * W.float()).sum(0).to(out_dtype) if W is not None else None
     if colscale is not None:
         s = s * colscale.float()[None, :]

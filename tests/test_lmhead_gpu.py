@@ -264,3 +264,37 @@ def test_infinite_logits_reach_the_loss(R, D):
     keep = torch.cat([W[:256], W[512:]])
     rl, rlse, _, _ = LH.lm_head_reference(x, None, keep, t, want_grads=False)
     assert torch.allclose(lse, rlse, rtol=1e-3, atol=2e-2) and torch.allclose(loss, rl, rtol=1e-3, atol=3e-2)
+
+
+@pytest.mark.parametrize("R,D", [(1020, 256), (4080, 256), (1020, 384), (4080, 384)])
+def test_mean_loss_gradients_keep_their_precision_at_every_row_count(R, D):
+    """1/1020 and 1/4080 lie almost half a unit in the last place from the next bf16 value.  Rounding a result to bf16
+    leaves a 2-norm error of about 0.42 * 2^-8 = 0.0016 (uniform in the unit, mantissas spread over their logarithm), the
+    gradient tile's own rounding a little more; a scale rounded in every row alike would add 0.0035."""
+    from chaoscontrol_b200.kernels import fused_linear_cross_entropy
+    V = 2048
+    g = torch.Generator(device="cuda").manual_seed(R + D)
+    x = torch.randn(R, D, generator=g, device="cuda").bfloat16().requires_grad_(True)
+    W = (torch.randn(V, D, generator=g, device="cuda") * 0.1).bfloat16().requires_grad_(True)
+    t = torch.randint(0, V, (R,), generator=g, device="cuda")
+    gx, gW = torch.autograd.grad(fused_linear_cross_entropy(x, W, t), (x, W))
+    xd, Wd = x.detach().double().requires_grad_(True), W.detach().double().requires_grad_(True)
+    rx, rW = torch.autograd.grad(torch.nn.functional.cross_entropy(xd @ Wd.t(), t), (xd, Wd))
+    for a, b in ((gx, rx), (gW, rW)):
+        assert float((a.double() - b).norm() / b.norm()) <= 0.0025
+
+
+@pytest.mark.parametrize("R,D,norm", [(300, 256, True), (300, 384, True), (300, 384, False), (4096 + 77, 256, True),
+                                      (18944 + 60, 256, True)])
+def test_device_scale_is_applied_to_dx_and_left_out_of_the_partials(R, D, norm):
+    """``gscale_dev`` against the same call without it: a power of two commutes with every rounding, so dX is exactly that
+    much larger; the weight partials are the same bits.  Every path: few rows, general, whole row tiles, split sweep."""
+    x, W, t, ss = _mk_d(R, 1024, D, wscale=0.3, seed=11)
+    rowss = ss if norm else None
+    _, lse = LH.lm_head_lse(x, rowss, W, t)
+    up = torch.full((), 0.25, device="cuda")
+    for kw in (dict(lse=lse), dict()):
+        a = LH.lm_head_train(x, rowss, W, t, gscale=0.5, **kw)
+        b = LH.lm_head_train(x, rowss, W, t, gscale=0.5, gscale_dev=up, **kw)
+        _lib.assert_ok()
+        assert torch.equal(b[2].float(), a[2].float() * 0.25) and torch.equal(b[3], a[3])

@@ -34,3 +34,15 @@ def test_splitk_reduce(S, N, K, dt, fold):
                 (S + N + 4) * 2.0 ** -24 * mag + rnd * terms.sum(0).abs() + 1e-30).all()
     else:
         assert dcol is None
+
+
+@pytest.mark.parametrize("S,N,K", [(1, 8, 64), (30, 64, 256), (30, 5, 10)])
+def test_splitk_reduce_scale(S, N, K):
+    """A device scale multiplies the fp32 sums before anything is rounded: exact for a power of two."""
+    g = torch.Generator(device="cuda").manual_seed(S)
+    part = torch.randn(S, N, K, generator=g, device="cuda")
+    W = torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    up = torch.full((), -0.5, device="cuda")
+    for dt in (torch.float32, torch.bfloat16):
+        for a, b in zip(splitk_reduce(part, W=W, out_dtype=dt, scale=up), splitk_reduce(part, W=W, out_dtype=dt)):
+            assert torch.equal(a, b * -0.5)
