@@ -229,9 +229,12 @@ class LayerWeights:
         """:meth:`prepare` as one kernel launch; False (nothing done) for operands it does not take.
         ``parts``: the four projections, to be packed as well."""
         ops = [self.Wfc, self.wn1, self.wn2, self.log_a, *(parts if parts is not None else [self.Wp])]
-        if not all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() for t in ops):
+        if not _plain_bf16(*ops):
             return False
         F_, D = self.Wfc.shape
+        mats = [(t, (D, D)) for t in parts] if parts is not None else [(self.Wp, (4 * D, D))]
+        if not _shaped((self.wn1, (D,)), (self.wn2, (D,)), (self.log_a, (D,)), *mats):
+            return False
         dev = self.Wfc.device
         Wp = torch.empty(4 * D, D, dtype=torch.bfloat16, device=dev) if parts is not None else None
         Wp_f = torch.empty(4 * D, D, dtype=torch.bfloat16, device=dev)
@@ -338,6 +341,16 @@ def _plain_bf16(*ts) -> bool:
     return all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() for t in ts)
 
 
+def _shaped(*pairs) -> bool:
+    """The native layer calls take addresses and the sizes of one layer: every (tensor, shape) has to be as they say.
+    Anything else goes through the step-by-step form, whose operations check (or broadcast) what they are given."""
+    return all(tuple(t.shape) == shape for t, shape in pairs)
+
+
+def _layer_shaped(w: "LayerWeights", D: int, F_: int) -> bool:
+    return _shaped((w.Wp_f, (4 * D, D)), (w.Wfc_f, (F_, D)), (w.Wo, (D, D)), (w.Wproj, (D, F_)), (w.log_a32, (D,)))
+
+
 def _plain_f32(*ts) -> bool:
     return all(t is None or (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()) for t in ts)
 
@@ -359,7 +372,8 @@ def _layer_forward_native(x, ss1, w, B, T, h0, save):
     """:func:`layer_forward` as one native call; None when an operand is not plain."""
     R, D = x.shape
     F_ = w.Wfc.shape[0]
-    if not (R == B * T and R > 0 and D % 8 == 0 and F_ % 8 == 0 and w.log_a32.dim() == 1 and
+    if not (R == B * T and R > 0 and D % 8 == 0 and F_ % 8 == 0 and _layer_shaped(w, D, F_) and
+            _shaped((ss1, (R,))) and
             _plain_bf16(x, w.Wp_f, w.Wfc_f, w.Wo, w.Wproj) and _plain_f32(ss1, w.log_a32, h0)):
         return None
     dev = x.device
@@ -384,12 +398,14 @@ def _layer_backward_native(dx3, ctx, w, B, T, dhT, want_dh0, outs, grad_dtype):
     R, D = ctx.x.shape
     F_ = ctx.F
     if not (_plain_bf16(dx3, w.Wp_f, w.Wfc_f, w.Wo, w.Wproj, w.Wp, w.Wfc, w.wn1, w.wn2) and
-            _plain_f32(w.log_a32, dhT) and dx3.shape == ctx.x.shape):
+            _plain_f32(w.log_a32, dhT) and dx3.shape == ctx.x.shape and _layer_shaped(w, D, F_) and
+            _shaped((w.Wp, (4 * D, D)), (w.Wfc, (F_, D)), (w.wn1, (D,)), (w.wn2, (D,)))):
         return None
     dev = dx3.device
+    shapes = ((4 * D, D), (D, D), (F_, D), (D, F_), (D,), (D,), (D,))      # in the order of _GRAD_KEYS
     if outs:
         if grad_dtype != torch.float32 or any(k not in outs for k in _GRAD_KEYS) or not _plain_f32(
-                *(outs[k] for k in _GRAD_KEYS)):
+                *(outs[k] for k in _GRAD_KEYS)) or not _shaped(*((outs[k], s) for k, s in zip(_GRAD_KEYS, shapes))):
             return None
         g = [outs[k] for k in _GRAD_KEYS]
     elif grad_dtype in (torch.float32, torch.bfloat16):
