@@ -255,6 +255,11 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
     return smem + (st < 2 ? LH_OFF_STG + st * LH_TILE : LH_OFF_RES);
   };
   const int n_sweeps = (MODE == MODE_TRAIN && DEEP == 0 && !p.skip_lse) ? 2 : 1;
+  // One-sweep training takes every row's numerators against the maximum of its first 32 logits.  A piece of an m-tile
+  // that begins elsewhere computes that tile's logits first, one step without a second MMA, so that all pieces of a row
+  // share the reference and saturate and flush where the whole row would.  (A piece's own first 32 logits may lie far
+  // below its others: unused words, a damaged stretch of the head.)  Only the first piece of a CTA can begin elsewhere.
+  auto ref_step = [](int inner0) { return FUSED1 && inner0 > 0 ? 1 : 0; };
 
   if (warp == 0) {
     // =========================== TMA producer ================================
@@ -276,7 +281,8 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
           res_phase ^= 1u;
         }
         for (int sw = 0; sw < n_sweeps && ok; ++sw) {
-          for (int it = inner0; it < inner1; ++it, ++n_stg) {
+          for (int i = inner0 - ref_step(inner0); i < inner1; ++i, ++n_stg) {
+            const int it = FUSED1 && i < inner0 ? 0 : i;
             const int s = (int)(n_stg % NSTG);
             const uint32_t ph = (n_stg / NSTG) & 1u;
             if (!mbar_wait(&bars->stg_empty[s], ph ^ 1u, abort_flag, p.status)) { ok = false; break; }
@@ -350,7 +356,7 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
           const bool second = (MODE == MODE_DW) || (IS_TRAIN && sw == n_sweeps - 1);
           int prev_stage = -1;
           bool prev_first = true;
-          for (int it = inner0; it < inner1; ++it) {
+          for (int it = inner0 - ref_step(inner0); it < inner1; ++it) {
             const int s = (int)(n_stg % NSTG);
             const uint32_t sph = (n_stg / NSTG) & 1u;
             ++n_stg;
@@ -380,7 +386,7 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
               }
             }
             umma_commit(&bars->d1_full[b]);
-            if (!second) {
+            if (!second || (FUSED1 && it < inner0)) {
               umma_commit(&bars->stg_empty[s]);
             } else {
               if (prev_stage >= 0) {
@@ -620,7 +626,7 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
       for (int sw = 0; sw < n_sweeps && ok; ++sw) {
         const bool second = (MODE == MODE_DW) || (IS_TRAIN && sw == n_sweeps - 1);
         float run_m = -INFINITY, run_s = 0.f, run_e = 0.f, tacc = 0.f, zt = 0.f;
-        for (int it = inner0; it < inner1 && ok; ++it) {
+        for (int it = inner0 - ref_step(inner0); it < inner1 && ok; ++it) {
           const int b = ONEBUF ? 0 : (n_d1 & 1);
           const uint32_t dph = ONEBUF ? (n_d1 & 1u) : ((n_d1 >> 1) & 1u);
           ++n_d1;
@@ -673,10 +679,8 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
             if (lane == 0) mbar_arrive(&bars->d1_empty[b]);
           } else {
             // ---- sweep 2 / DW: g tile -> shared memory ------------------------
-            const uint32_t gph = n_g & 1u;
-            ++n_g;
-            if (FUSED1 && it == inner0) {
-              // per-row reference: max of the unit's first 32 logits (every warp reads the same
+            if (FUSED1 && it == inner0 - ref_step(inner0)) {
+              // per-row reference: max of the row's first 32 logits (every warp reads the same
               // 32 columns, so all parts of a row agree without an exchange)
               uint32_t a0[32];
               __syncwarp();
@@ -686,7 +690,15 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
 #pragma unroll
               for (int i = 1; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(a0[i]));
               c2 = fmaf(mx, c1, LH_REF_MARGIN);
+              if (it < inner0) {                     // the reference step: nothing else of this tile is wanted
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->d1_empty[b]);
+                continue;
+              }
             }
+            const uint32_t gph = n_g & 1u;
+            ++n_g;
             // all of this warp's groups are requested before any is used: one TMEM round trip
             // per tile on the path between the two MMAs
             uint32_t ah[NG][32];
@@ -949,7 +961,7 @@ lmhead_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
 
 // Joins the pieces of m-tiles that the split walk cut: one warp a row, pieces in vocabulary order.  Sixteen blocks
 // of eight rows for each boundary between two CTAs' ranges; those of a tile's first boundary do the work.
-// The pieces' own references (m: the maximum, or TRAIN1's fixed one) are brought to the largest of them.
+// Scoring brings the pieces' sums from their own maxima to the largest of them; the training pieces share a reference.
 template <int MODE>
 __global__ void __launch_bounds__(256) lmhead_join_kernel(const LmHeadArgs p, int grid) {
   const long long share = lh_share(p.n_mtiles, p.n_vtiles, grid), nv = p.n_vtiles;
@@ -965,7 +977,7 @@ __global__ void __launch_bounds__(256) lmhead_join_kernel(const LmHeadArgs p, in
   const float rs = p.rowss ? rsqrtf(p.rowss[r] * p.inv_dim + p.eps) : 1.f;
   const int tgt = (int)p.targets[r];
   float M = -INFINITY;
-  if (MODE != MODE_TRAIN)
+  if (MODE == MODE_LSE)
     for (int c = c_first; c <= c_last; ++c) M = fmaxf(M, p.part_rows[slot_of(c) * LH_ROWS + row].x);
   float S = 0.f, z = 0.f, e = 0.f, acc[8];
 #pragma unroll
@@ -973,21 +985,16 @@ __global__ void __launch_bounds__(256) lmhead_join_kernel(const LmHeadArgs p, in
   for (int c = c_first; c <= c_last; ++c) {
     const long long slot = slot_of(c);
     const float4 v = p.part_rows[slot * LH_ROWS + row];
-    const float w = MODE == MODE_TRAIN ? 1.f : ex2f(v.x - M);
+    const float w = MODE == MODE_LSE ? ex2f(v.x - M) : 1.f;
     S += v.y * w;
-    if (MODE == MODE_TRAIN1) {
-      // the piece that holds the target knows its logit relative to the piece's reference
-      const long long a = c * share > unit * nv ? c * share - unit * nv : 0, b = (c + 1) * share - unit * nv;
-      if (tgt / LH_VT >= a && tgt / LH_VT < b) z = v.z + v.x;
-    } else {
-      z += v.z;
-    }
+    z += v.z;                                  // the target's logit, zero in the pieces that do not hold it
     e += v.w * w;
+    if (MODE == MODE_TRAIN1) M = v.x;          // the reference, the same in every piece
     if (MODE != MODE_LSE) {
       const float4* a4 = reinterpret_cast<const float4*>(p.part_acc + (slot * LH_ROWS + row) * LH_D + lane * 8);
       const float4 a0 = __ldg(a4), a1 = __ldg(a4 + 1);
-      acc[0] += a0.x * w; acc[1] += a0.y * w; acc[2] += a0.z * w; acc[3] += a0.w * w;
-      acc[4] += a1.x * w; acc[5] += a1.y * w; acc[6] += a1.z * w; acc[7] += a1.w * w;
+      acc[0] += a0.x; acc[1] += a0.y; acc[2] += a0.z; acc[3] += a0.w;
+      acc[4] += a1.x; acc[5] += a1.y; acc[6] += a1.z; acc[7] += a1.w;
     }
   }
   if (lane == 0) {
@@ -997,8 +1004,9 @@ __global__ void __launch_bounds__(256) lmhead_join_kernel(const LmHeadArgs p, in
       p.loss[r] = lse - z * rs;
       if (p.entropy != nullptr) p.entropy[r] = lse - rs * e / S;
     } else if (MODE == MODE_TRAIN1) {
-      p.lse[r] = (M + __log2f(S)) * LN2;
-      p.loss[r] = (M + __log2f(S) - z) * LN2;
+      const float lg = __log2f(S);
+      p.lse[r] = (M + lg) * LN2;
+      p.loss[r] = (lg - z) * LN2;
     } else {
       p.loss[r] = -z * LN2;
     }

@@ -298,3 +298,30 @@ def test_device_scale_is_applied_to_dx_and_left_out_of_the_partials(R, D, norm):
         b = LH.lm_head_train(x, rowss, W, t, gscale=0.5, gscale_dev=up, **kw)
         _lib.assert_ok()
         assert torch.equal(b[2].float(), a[2].float() * 0.25) and torch.equal(b[3], a[3])
+
+
+@pytest.mark.parametrize("R,V", [(4096, 4096), (18944 + 128, 2304)])
+def test_split_one_sweep_keeps_the_rows_own_reference(R, V, epilogue_parts):
+    """Bands of logits 200 nats below the rest wherever a piece of a row tile may begin (the first 32 words of every
+    vocabulary tile but the first).  The row's reference, the maximum of its first 32 logits, is ordinary; every piece
+    has to use it.  lse and loss as in the other one-sweep test, dX against whole row tiles."""
+    x, W, t, _ = _mk_d(R, V, 256, wscale=0.05, seed=13)
+    x[:, 0] = 8.0
+    W[:, 0] = 0.0
+    low = torch.arange(V, device="cuda").view(-1, 128)[1:, :32].reshape(-1)
+    W[low, 0] = -25.0
+    t = torch.where((t >= 128) & (t % 128 < 32), t + 32, t)
+    assert _lib.lib().ccb_lmhead_work(R, V, 256, 1) > 0
+    kw = dict(gscale=0.5, want_dw=False, one_sweep=True)
+    loss, lse, dX, _ = LH.lm_head_train(x, None, W, t, **kw)
+    real = LH._split_work
+    LH._split_work = lambda *a: None
+    try:
+        wloss, wlse, wdX, _ = LH.lm_head_train(x, None, W, t, **kw)
+    finally:
+        LH._split_work = real
+    _lib.assert_ok()
+    rl, rlse, _, _ = LH.lm_head_reference(x, None, W, t, want_grads=False)
+    assert torch.allclose(lse, rlse, rtol=1e-3, atol=2e-2) and torch.allclose(loss, rl, rtol=1e-3, atol=3e-2)
+    assert torch.allclose(lse, wlse, rtol=0, atol=2e-4) and torch.allclose(loss, wloss, rtol=0, atol=2e-4)
+    assert (dX.float() - wdX.float()).norm() <= 2e-3 * wdX.float().norm()
