@@ -302,13 +302,24 @@ __device__ __forceinline__ void store_grad4(__nv_bfloat16* o, float4 v) {
   *reinterpret_cast<uint2*>(o) = q;
 }
 __device__ __forceinline__ void store_grad1(float* o, float v) { *o = v; }
+// Where row n of the result goes: one [N, K] tensor, or up to four of `rows` rows each (a packed weight whose parts are
+// parameters of their own, with gradients in allocations of their own).
+template <typename OT>
+struct SpkOut {
+  OT* p[4];
+  int rows;
+  __device__ __forceinline__ OT* row(int n, int K) const {
+    const int i = n / rows;
+    return p[i] + (long long)(n - i * rows) * K;
+  }
+};
 __device__ __forceinline__ void store_grad1(__nv_bfloat16* o, float v) { *o = __float2bfloat16(v); }
 
 template <int G, typename OT>
 __global__ void __launch_bounds__(128 * G)
 splitk_tile_kernel(const float* __restrict__ part, int S, long long split_stride, int N, int K,
                    const __nv_bfloat16* __restrict__ colscale, const __nv_bfloat16* __restrict__ W,
-                   const float* __restrict__ scale, OT* __restrict__ out, float* __restrict__ colpart) {
+                   const float* __restrict__ scale, const SpkOut<OT> out, float* __restrict__ colpart) {
   __shared__ float4 join[G > 1 ? (G - 1) * 128 : 1];
   __shared__ float4 colj[128];
   const int slot = threadIdx.x & 127, g = threadIdx.x >> 7;
@@ -357,7 +368,7 @@ splitk_tile_kernel(const float* __restrict__ part, int S, long long split_stride
         const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y);
         acc.x *= a.x; acc.y *= a.y; acc.z *= b.x; acc.w *= b.y;
       }
-      store_grad4(out + o, acc);
+      store_grad4(out.row(n, K) + k, acc);
     }
     if (colpart != nullptr) colj[slot] = w;
   }
@@ -380,7 +391,7 @@ template <typename OT>
 __global__ void splitk_reduce_kernel(const float* __restrict__ part, int S, long long split_stride,
                                      int N, int K, const __nv_bfloat16* __restrict__ colscale,
                                      const __nv_bfloat16* __restrict__ W, const float* __restrict__ scale,
-                                     OT* __restrict__ out, int accumulate, float* __restrict__ colpart) {
+                                     const SpkOut<OT> out, int accumulate, float* __restrict__ colpart) {
   const float up = scale ? __ldg(scale) : 1.f;
   const int n0 = blockIdx.x * SPK_ROWS;
   for (int k = threadIdx.x; k < K; k += blockDim.x) {
@@ -404,7 +415,8 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int S, long
         const long long o = (long long)n * K + k;
         if (W) cacc += s * __bfloat162float(W[o]);
         const float val = s * cs;
-        store_grad1(out + o, accumulate ? (float)out[o] + val : val);
+        OT* dst = out.row(n, K) + k;
+        store_grad1(dst, accumulate ? (float)*dst + val : val);
       }
     }
     if (colpart) colpart[(long long)blockIdx.x * K + k] = cacc;
@@ -1124,10 +1136,17 @@ static int launch_colsum(const float* part, int64_t NB, int64_t K, void* out, in
 
 template <typename OT>
 static int launch_splitk(const float* part, int64_t S, int64_t split_stride, int64_t N, int64_t K,
-                         const __nv_bfloat16* colscale, const __nv_bfloat16* W, const float* scale, OT* out,
-                         int64_t accumulate, float* colpart, cudaStream_t s) {
+                         const __nv_bfloat16* colscale, const __nv_bfloat16* W, const float* scale, void* const* parts,
+                         int64_t nparts, int64_t accumulate, float* colpart, cudaStream_t s) {
+  SpkOut<OT> out = {};
+  uintptr_t outs = 0;
+  for (int i = 0; i < nparts; ++i) {
+    out.p[i] = (OT*)parts[i];
+    outs |= (uintptr_t)parts[i];
+  }
+  out.rows = (int)(N / nparts);
   const unsigned nb = (unsigned)((N + SPK_ROWS - 1) / SPK_ROWS);
-  const uintptr_t wide = (uintptr_t)part | (uintptr_t)out;                  // 16-byte accesses
+  const uintptr_t wide = (uintptr_t)part | outs;                            // 16-byte accesses
   const uintptr_t half = (uintptr_t)colscale | (uintptr_t)W;                // 8-byte accesses
   const bool tile = !accumulate && K % 4 == 0 && split_stride % 4 == 0 && (wide & 15) == 0 && (half & 7) == 0 &&
                     (K + SPK_COLS - 1) / SPK_COLS <= 65535;
@@ -1146,22 +1165,33 @@ static int launch_splitk(const float* part, int64_t S, int64_t split_stride, int
   return 0;
 }
 
-// `out` and `colsum_out` are fp32, or bf16 with out_bf16; `scale` (device, may be null) multiplies the sums.
-extern "C" int ccb_splitk_reduce_as(const float* part, int64_t S, int64_t split_stride, int64_t N, int64_t K,
-                                    const void* colscale, const void* W, const float* scale, void* out,
-                                    int64_t out_bf16, int64_t accumulate, float* colpart, void* colsum_out,
-                                    int64_t colsum_accumulate, void* stream) {
+// The results go to `nout` tensors of N / nout rows (1 to 4); they and `colsum_out` are fp32, or bf16 with out_bf16;
+// `scale` (device, may be null) multiplies the sums.
+extern "C" int ccb_splitk_reduce_parts(const float* part, int64_t S, int64_t split_stride, int64_t N, int64_t K,
+                                       const void* colscale, const void* W, const float* scale, void* const* outs,
+                                       int64_t nout, int64_t out_bf16, int64_t accumulate, float* colpart,
+                                       void* colsum_out, int64_t colsum_accumulate, void* stream) {
   if (N <= 0 || K <= 0) return 0;
+  if (nout < 1 || nout > 4 || N % nout != 0)
+    return set_error("ccb_splitk_reduce: %lld rows into %lld tensors", (long long)N, (long long)nout);
   cudaStream_t s = (cudaStream_t)stream;
   const __nv_bfloat16* cs = (const __nv_bfloat16*)colscale;
   const __nv_bfloat16* w = (const __nv_bfloat16*)W;
   float* cp = W ? colpart : nullptr;
-  const int rc = out_bf16 ? launch_splitk(part, S, split_stride, N, K, cs, w, scale, (__nv_bfloat16*)out, accumulate, cp, s)
-                          : launch_splitk(part, S, split_stride, N, K, cs, w, scale, (float*)out, accumulate, cp, s);
+  const int rc = out_bf16 ? launch_splitk<__nv_bfloat16>(part, S, split_stride, N, K, cs, w, scale, outs, nout, accumulate, cp, s)
+                          : launch_splitk<float>(part, S, split_stride, N, K, cs, w, scale, outs, nout, accumulate, cp, s);
   if (rc) return rc;
   if (cp && colsum_out)
     return launch_colsum(cp, (N + SPK_ROWS - 1) / SPK_ROWS, K, colsum_out, (int)out_bf16, colsum_accumulate, s);
   return 0;
+}
+
+extern "C" int ccb_splitk_reduce_as(const float* part, int64_t S, int64_t split_stride, int64_t N, int64_t K,
+                                    const void* colscale, const void* W, const float* scale, void* out,
+                                    int64_t out_bf16, int64_t accumulate, float* colpart, void* colsum_out,
+                                    int64_t colsum_accumulate, void* stream) {
+  return ccb_splitk_reduce_parts(part, S, split_stride, N, K, colscale, W, scale, &out, 1, out_bf16, accumulate, colpart,
+                                 colsum_out, colsum_accumulate, stream);
 }
 
 extern "C" int ccb_splitk_reduce(const float* part, int64_t S, int64_t split_stride, int64_t N,

@@ -18,9 +18,10 @@ int ccb_scan_fwd(const void* P, int64_t ldp, const float* log_a, const float* h0
 int ccb_scan_bwd(const void* P, int64_t ldp, const float* log_a, const float* h0, const void* hstates, const void* dy,
                  const float* dhT, const float* rowss, float inv_dim, float eps, void* dP, int64_t lddp,
                  float* dloga_part, float* dh0, int64_t B, int64_t T, int64_t D, int64_t la_bstride, void* stream);
-int ccb_splitk_reduce_as(const float* part, int64_t S, int64_t split_stride, int64_t N, int64_t K, const void* colscale,
-                         const void* W, const float* scale, void* out, int64_t out_bf16, int64_t accumulate,
-                         float* colpart, void* colsum_out, int64_t colsum_accumulate, void* stream);
+int ccb_splitk_reduce_parts(const float* part, int64_t S, int64_t split_stride, int64_t N, int64_t K,
+                            const void* colscale, const void* W, const float* scale, void* const* outs, int64_t nout,
+                            int64_t out_bf16, int64_t accumulate, float* colpart, void* colsum_out,
+                            int64_t colsum_accumulate, void* stream);
 int ccb_colsum_as(const float* part, int64_t NB, int64_t K, void* out, int64_t out_bf16, int64_t accumulate, void* stream);
 
 typedef struct CcbLayerArgs {
@@ -43,7 +44,8 @@ typedef struct CcbLayerArgs {
   const float* dhT;
   void* ws16;                             // ccb_layer_bwd_ws16 elements
   float* ws32;                            // ccb_layer_bwd_ws32 elements
-  void *dx, *dWp, *dWo, *dWfc, *dWproj, *dwn1, *dwn2, *dlog_a;
+  void *dx, *dWp[4];                      // one [4D, D] (dWp[1] null) or four [D, D]
+  void *dWo, *dWfc, *dWproj, *dwn1, *dwn2, *dlog_a;
   float* dh0;
 } CcbLayerArgs;
 }
@@ -86,14 +88,15 @@ static int resid(const void* y, int64_t K, const void* W, const void* x, void* o
 
 // out[N, K] = dy^T x over R rows, with the folded norm weight's gradient when wn is given
 static int wgrad(const void* dy, int64_t N, const void* x, int64_t K, int64_t R, float* part, float* colpart,
-                 const void* wn, const void* W, void* out, void* dwn, int64_t out_bf16, cudaStream_t s) {
+                 const void* wn, const void* W, void* const* outs, int64_t nout, void* dwn, int64_t out_bf16,
+                 cudaStream_t s) {
   CcbGemmArgs a = gemm_args(dy, N, x, K, part, N, K, R);
   a.a_mn = 1; a.b_mn = 1;
   a.out_fp32 = 1;
   a.splits = wgrad_splits(N, K, R);
   a.c_split = a.splits > 1 ? N * K : 0;
   if (int rc = ccb_gemm(&a, s)) return rc;
-  return ccb_splitk_reduce_as(part, a.splits, N * K, N, K, wn, W, nullptr, out, out_bf16, 0, colpart, dwn, 0, s);
+  return ccb_splitk_reduce_parts(part, a.splits, N * K, N, K, wn, W, nullptr, outs, nout, out_bf16, 0, colpart, dwn, 0, s);
 }
 
 }  // namespace ccb
@@ -146,19 +149,19 @@ extern "C" int ccb_layer_backward(const CcbLayerArgs* p, void* stream) {
   a.R1 = p->u; a.ldr = F;
   a.rowss = p->ss2; a.inv_dim = inv_d; a.eps = p->eps;
   if (int rc = ccb_gemm(&a, s)) return rc;
-  if (int rc = wgrad(p->dx3, D, p->f, F, R, part, nullptr, nullptr, nullptr, p->dWproj, nullptr, p->grad_bf16, s)) return rc;
+  if (int rc = wgrad(p->dx3, D, p->f, F, R, part, nullptr, nullptr, nullptr, &p->dWproj, 1, nullptr, p->grad_bf16, s)) return rc;
   a = gemm_args(du, F, p->Wfc_f, D, dx2, R, D, F);
   a.b_mn = 1;
   a.epi = CCB_EPI_RMSBWD;
   a.R1 = p->x2; a.R2 = p->dx3; a.ldr = D;
   a.rowss = p->ss2; a.inv_dim = inv_d; a.eps = p->eps;
   if (int rc = ccb_gemm(&a, s)) return rc;
-  if (int rc = wgrad(du, F, p->x2, D, R, part, colpart, p->wn2, p->Wfc, p->dWfc, p->dwn2, p->grad_bf16, s)) return rc;
+  if (int rc = wgrad(du, F, p->x2, D, R, part, colpart, p->wn2, p->Wfc, &p->dWfc, 1, p->dwn2, p->grad_bf16, s)) return rc;
   // recurrence half
   a = gemm_args(dx2, D, p->Wo, D, dy, R, D, D);
   a.b_mn = 1;
   if (int rc = ccb_gemm(&a, s)) return rc;
-  if (int rc = wgrad(dx2, D, p->y, D, R, part, nullptr, nullptr, nullptr, p->dWo, nullptr, p->grad_bf16, s)) return rc;
+  if (int rc = wgrad(dx2, D, p->y, D, R, part, nullptr, nullptr, nullptr, &p->dWo, 1, nullptr, p->grad_bf16, s)) return rc;
   if (int rc = ccb_scan_bwd(p->P, 4 * D, p->log_a, p->h0, p->h, dy, p->dhT, p->ss1, inv_d, p->eps, dP, 4 * D, dla, p->dh0,
                             p->B, p->T, D, 0, s)) return rc;
   if (int rc = ccb_colsum_as(dla, p->B, D, p->dlog_a, p->grad_bf16, 0, s)) return rc;
@@ -168,5 +171,5 @@ extern "C" int ccb_layer_backward(const CcbLayerArgs* p, void* stream) {
   a.R1 = p->x; a.R2 = dx2; a.ldr = D;
   a.rowss = p->ss1; a.inv_dim = inv_d; a.eps = p->eps;
   if (int rc = ccb_gemm(&a, s)) return rc;
-  return wgrad(dP, 4 * D, p->x, D, R, part, colpart, p->wn1, p->Wp, p->dWp, p->dwn1, p->grad_bf16, s);
+  return wgrad(dP, 4 * D, p->x, D, R, part, colpart, p->wn1, p->Wp, p->dWp, p->dWp[1] ? 4 : 1, p->dwn1, p->grad_bf16, s);
 }

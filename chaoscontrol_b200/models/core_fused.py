@@ -112,10 +112,11 @@ class _BlockFn(torch.autograd.Function):
     def backward(ctx, go, _ghT):
         B, Tn, D = ctx.dims
         dx, g = T.layer_backward(go.reshape(B * Tn, D).contiguous(), ctx.c, ctx.w, B, Tn, None,
-                                 want_dh0=ctx.has_h0 and ctx.needs_input_grad[1], grad_dtype=ctx.w.Wo.dtype)
+                                 want_dh0=ctx.has_h0 and ctx.needs_input_grad[1], grad_dtype=ctx.w.Wo.dtype,
+                                 split_wp=True)
         ctx.c = None
         wdt = ctx.w.Wo.dtype
-        dsel, dinp, dgate, ddelta = (t.to(wdt) for t in g.dWp.split(D, 0))
+        dsel, dinp, dgate, ddelta = (t.to(wdt) for t in g.dWp)
         ndt, adt = ctx.dtypes
         return (dx.view(B, Tn, D), g.dh0 if ctx.has_h0 else None, dsel, dinp, dgate, ddelta, g.dWo.to(wdt),
                 g.dWfc.to(wdt), g.dWproj.to(wdt), g.dwn1.to(ndt), g.dwn2.to(ndt), g.dlog_a.to(adt))

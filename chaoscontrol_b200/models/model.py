@@ -151,10 +151,9 @@ class _TrunkFn(torch.autograd.Function):
         for i in reversed(range(L)):
             w, c = ctx.ws[i], ctx.ctxs[i]
             dhT = dhT_stack[i].float().contiguous() if use_dhT else None
-            dx, g = T.layer_backward(dx, c, w, B, Tn, dhT, want_dh0=ctx.has_h0, grad_dtype=w.Wo.dtype)
-            D = w.Wo.shape[0]
+            dx, g = T.layer_backward(dx, c, w, B, Tn, dhT, want_dh0=ctx.has_h0, grad_dtype=w.Wo.dtype, split_wp=True)
             pd = w.Wo.dtype
-            dsel, dinp, dgate, ddelta = (t.to(pd) for t in g.dWp.split(D, dim=0))
+            dsel, dinp, dgate, ddelta = (t.to(pd) for t in g.dWp)
             grads = [dsel, dinp, dgate, ddelta, g.dWo.to(pd), g.dWfc.to(pd), g.dWproj.to(pd),
                      g.dwn1.to(w.wn1.dtype), g.dwn2.to(w.wn2.dtype),
                      g.dlog_a.to(w.log_a.dtype)] + grads

@@ -44,7 +44,7 @@ class LayerArgs(C.Structure):
     _fields_ = [("B", i64), ("T", i64), ("D", i64), ("F", i64), ("eps", f32), ("grad_bf16", i64)] + [
         (n, vp) for n in ("Wp_f", "Wfc_f", "Wo", "Wproj", "Wp", "Wfc", "wn1", "wn2", "log_a", "h0",
                           "x", "ss1", "P", "y", "h", "x2", "u", "f", "ss2", "x3", "ss3", "hT",
-                          "dx3", "dhT", "ws16", "ws32", "dx", "dWp", "dWo", "dWfc", "dWproj", "dwn1", "dwn2",
+                          "dx3", "dhT", "ws16", "ws32", "dx", "dWp", "dWp1", "dWp2", "dWp3", "dWo", "dWfc", "dWproj", "dwn1", "dwn2",
                           "dlog_a", "dh0")]
 
 

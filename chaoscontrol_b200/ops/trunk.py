@@ -300,7 +300,7 @@ class PackedCtx:
 
 @dataclass
 class LayerGrads:
-    dWp: torch.Tensor       # [4D, D] fp32 (or the grad_dtype asked for)
+    dWp: torch.Tensor       # [4D, D] fp32 (or the grad_dtype asked for), or four [D, D] (split_wp)
     dWo: torch.Tensor
     dWfc: torch.Tensor
     dWproj: torch.Tensor
@@ -393,7 +393,7 @@ def _layer_forward_native(x, ss1, w, B, T, h0, save):
 _GRAD_KEYS = ("dWp", "dWo", "dWfc", "dWproj", "dwn1", "dwn2", "dlog_a")
 
 
-def _layer_backward_native(dx3, ctx, w, B, T, dhT, want_dh0, outs, grad_dtype):
+def _layer_backward_native(dx3, ctx, w, B, T, dhT, want_dh0, outs, grad_dtype, split_wp=False):
     """:func:`layer_backward` as one native call; None when an operand is not plain."""
     R, D = ctx.x.shape
     F_ = ctx.F
@@ -409,9 +409,9 @@ def _layer_backward_native(dx3, ctx, w, B, T, dhT, want_dh0, outs, grad_dtype):
             return None
         g = [outs[k] for k in _GRAD_KEYS]
     elif grad_dtype in (torch.float32, torch.bfloat16):
-        sizes = (4 * D * D, D * D, F_ * D, D * F_, D, D, D)
-        flat = torch.empty(sum(sizes), dtype=grad_dtype, device=dev).split(sizes)
-        g = [flat[0].view(4 * D, D), flat[1].view(D, D), flat[2].view(F_, D), flat[3].view(D, F_), *flat[4:]]
+        # an allocation each: a gradient that is kept, saved or changed in place leaves the others alone
+        each = lambda *ss: [torch.empty(s, dtype=grad_dtype, device=dev) for s in ss]
+        g = [tuple(each(*[(D, D)] * 4)), *each(*shapes[1:])] if split_wp else each(*shapes)
     else:
         return None
     L = _lib.lib()
@@ -424,7 +424,11 @@ def _layer_backward_native(dx3, ctx, w, B, T, dhT, want_dh0, outs, grad_dtype):
     a.Wp, a.Wfc, a.wn1, a.wn2 = w.Wp.data_ptr(), w.Wfc.data_ptr(), w.wn1.data_ptr(), w.wn2.data_ptr()
     a.dx3, a.dhT, a.ws16, a.ws32 = dx3.data_ptr(), _lib.ptr(dhT), ws16.data_ptr(), ws32.data_ptr()
     a.dx, a.dh0 = dx.data_ptr(), _lib.ptr(dh0)
-    a.dWp, a.dWo, a.dWfc, a.dWproj, a.dwn1, a.dwn2, a.dlog_a = (t.data_ptr() for t in g)
+    if split_wp:
+        a.dWp, a.dWp1, a.dWp2, a.dWp3 = (t.data_ptr() for t in g[0])
+    else:
+        a.dWp = g[0].data_ptr()
+    a.dWo, a.dWfc, a.dWproj, a.dwn1, a.dwn2, a.dlog_a = (t.data_ptr() for t in g[1:])
     _lib.check(L.ccb_layer_backward(C.byref(a), _lib.stream_ptr()), "layer_backward")
     return dx, LayerGrads(*g, dh0)
 
@@ -453,15 +457,18 @@ def layer_forward(x: torch.Tensor, ss1: torch.Tensor, w: LayerWeights, B: int, T
 
 def layer_backward(dx3: torch.Tensor, ctx: LayerCtx, w: LayerWeights, B: int, T: int,
                    dhT: Optional[torch.Tensor] = None, *, want_dh0: bool = False,
-                   outs: Optional[dict] = None, grad_dtype: torch.dtype = torch.float32):
+                   outs: Optional[dict] = None, grad_dtype: torch.dtype = torch.float32, split_wp: bool = False):
     """Backward of :func:`layer_forward`.  Returns ``(dx, LayerGrads)``.
 
-    Weight gradients are fp32, or rounded once to ``grad_dtype`` as they are stored.
+    Weight gradients are fp32, or rounded once to ``grad_dtype`` as they are stored.  ``split_wp`` (without
+    ``outs``): the gradients of the four packed projections as four tensors of their own.
     ``outs`` may map ``dWp / dWo / dWfc / dWproj / dwn1 / dwn2`` to preallocated
     fp32 tensors (views of a flat gradient buffer) that receive the results.
     """
+    if outs and split_wp:
+        raise ValueError("layer_backward: split_wp allocates the gradients; it takes no outs")
     if isinstance(ctx, PackedCtx):
-        res = _layer_backward_native(dx3, ctx, w, B, T, dhT, want_dh0, outs, grad_dtype)
+        res = _layer_backward_native(dx3, ctx, w, B, T, dhT, want_dh0, outs, grad_dtype, split_wp)
         if res is not None:
             return res
     R, D = ctx.x.shape
@@ -486,4 +493,6 @@ def layer_backward(dx3: torch.Tensor, ctx: LayerCtx, w: LayerWeights, B: int, T:
                               dcol_out=o.get("dwn1"), out_dtype=gd)
     if "dlog_a" in o:
         o["dlog_a"].copy_(dlog_a)
+    if split_wp:
+        dWp = tuple(t.clone() for t in dWp.split(D, 0))
     return dx, LayerGrads(dWp, dWo, dWfc, dWproj, dwn1, dwn2, dlog_a, dh0)

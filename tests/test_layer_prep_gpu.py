@@ -96,3 +96,34 @@ def test_embed_bwd_token_widths(V, dt, D):
     mag = torch.zeros(V, D, dtype=torch.float64, device="cuda").index_add_(0, tok[ok].long(), dx[ok].double().abs())
     assert ((got.double() - ref).abs() <= 2048 * 2.0 ** -24 * mag).all()          # at most 2000 fp32 additions a row
     assert torch.equal(got, trunk.embed_bwd(tok, dx, V, sort_cache=torch.sort(tok.long(), stable=True)))
+
+
+@pytest.mark.parametrize("B,T,D,F", [(1, 3, 64, 128), (5, 200, 256, 512), (2, 129, 320, 640)])
+def test_split_projection_gradients(B, T, D, F, monkeypatch):
+    """The four projections' gradients as tensors of their own: the rows of the packed one, bit for bit."""
+    g = torch.Generator(device="cuda").manual_seed(D)
+    rnd = lambda *s, k=1.0: (torch.randn(*s, generator=g, device="cuda") * k)
+    w = _weights(rnd, D, F)
+    x, dx3 = rnd(B * T, D).bfloat16(), rnd(B * T, D).bfloat16()
+    for native in (True, False):
+        if not native:
+            monkeypatch.setattr(trunk, "_layer_forward_native", lambda *a, **k: None)
+        c = trunk.layer_forward(x, trunk.row_ss(x), w, B, T)[3]
+        for dt in (torch.float32, torch.bfloat16):
+            one = trunk.layer_backward(dx3, c, w, B, T, grad_dtype=dt)[1]
+            four = trunk.layer_backward(dx3, c, w, B, T, grad_dtype=dt, split_wp=True)[1]
+            assert [t.dtype for t in four.dWp] == [dt] * 4 and torch.equal(torch.cat(four.dWp), one.dWp)
+            assert all(torch.equal(getattr(four, k), getattr(one, k)) for k in ("dWo", "dWfc", "dWproj", "dwn1", "dwn2"))
+
+
+def test_parameter_gradients_own_their_memory():
+    """No two gradients of a block share an allocation or a version counter."""
+    from chaoscontrol_b200.models.core_fused import FusedCareSSMBlock
+    blk = FusedCareSSMBlock(64).cuda().bfloat16()
+    x = torch.randn(2, 9, 64, device="cuda").bfloat16()
+    grads = torch.autograd.grad(blk(x).float().square().sum(), list(blk.parameters()))
+    assert len({t.untyped_storage().data_ptr() for t in grads}) == len(grads)
+    assert all(t.untyped_storage().nbytes() == t.numel() * t.element_size() for t in grads)
+    seen = [t._version for t in grads]
+    grads[0].zero_()
+    assert [t._version for t in grads[1:]] == seen[1:]
