@@ -281,7 +281,7 @@ class PackedCtx:
     """The same activations of a layer that ran as one native call: all bf16 ones in ``acts``."""
     x: torch.Tensor
     ss1: torch.Tensor
-    acts: torch.Tensor      # P [R,4D] | y [R,D] | h [R,D] | x2 [R,D] | u [R,F] | f [R,F]
+    acts: torch.Tensor      # P [R,4D] | y [R,D] | x2 [R,D] | u [R,F] | f [R,F] | h [R,D] (last: evaluation goes without)
     ss2: torch.Tensor
     h0: Optional[torch.Tensor]
     F: int
@@ -292,10 +292,10 @@ class PackedCtx:
 
     P = property(lambda c: c._part(0, 4 * c.x.shape[1]))
     y = property(lambda c: c._part(4 * c.x.shape[1], c.x.shape[1]))
-    h = property(lambda c: c._part(5 * c.x.shape[1], c.x.shape[1]))
-    x2 = property(lambda c: c._part(6 * c.x.shape[1], c.x.shape[1]))
-    u = property(lambda c: c._part(7 * c.x.shape[1], c.F))
-    f = property(lambda c: c._part(7 * c.x.shape[1] + c.F, c.F))
+    x2 = property(lambda c: c._part(5 * c.x.shape[1], c.x.shape[1]))
+    u = property(lambda c: c._part(6 * c.x.shape[1], c.F))
+    f = property(lambda c: c._part(6 * c.x.shape[1] + c.F, c.F))
+    h = property(lambda c: c._part(6 * c.x.shape[1] + 2 * c.F, c.x.shape[1]))
 
 
 @dataclass
@@ -363,8 +363,9 @@ def _layer_args(w: LayerWeights, B: int, T: int, D: int, F_: int, x, ss1, h0, ac
     a.x, a.ss1, a.ss2 = x.data_ptr(), ss1.data_ptr(), ss2.data_ptr()
     rd = 2 * x.numel()
     a.P = p = acts.data_ptr()
-    a.y, a.h, a.x2, a.u = p + 4 * rd, p + 5 * rd, p + 6 * rd, p + 7 * rd
-    a.f = p + 7 * rd + 2 * x.shape[0] * F_
+    rf = 2 * x.shape[0] * F_
+    a.y, a.x2, a.u = p + 4 * rd, p + 5 * rd, p + 6 * rd
+    a.f, a.h = p + 6 * rd + rf, p + 6 * rd + 2 * rf
     return a
 
 
@@ -377,7 +378,7 @@ def _layer_forward_native(x, ss1, w, B, T, h0, save):
             _plain_bf16(x, w.Wp_f, w.Wfc_f, w.Wo, w.Wproj) and _plain_f32(ss1, w.log_a32, h0)):
         return None
     dev = x.device
-    acts = torch.empty(R * (7 * D + 2 * F_), dtype=torch.bfloat16, device=dev)
+    acts = torch.empty(R * ((7 if save else 6) * D + 2 * F_), dtype=torch.bfloat16, device=dev)
     x3 = torch.empty_like(x)
     ss2 = torch.empty(R, dtype=torch.float32, device=dev)
     ss3 = torch.empty(R, dtype=torch.float32, device=dev)

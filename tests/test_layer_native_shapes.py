@@ -72,3 +72,32 @@ def test_fold_packed(lib, bad):
 def test_fold_parts(lib, i):
     parts = [torch.zeros(D - 8 if k == i else D, D) for k in range(4)]
     assert _weights()._fold_launch(parts) == (i is None) and lib.calls == (["ccb_layer_fold"] if i is None else [])
+
+
+@pytest.mark.parametrize("save", [True, False])
+def test_activation_buffer(lib, monkeypatch, save):
+    """The parts of the packed activations tile the buffer without gaps, and the states, which only backward reads, are
+    neither allocated nor passed without ``save``."""
+    got = {}
+    monkeypatch.setattr(_FakeLib, "ccb_layer_forward", lambda self, a, s: got.setdefault("a", a._obj) and 0, raising=False)
+    sizes = []
+    real = torch.empty
+
+    def empty(*a, **k):
+        t = real(*a, **k)
+        sizes.append((t.data_ptr(), t.numel() * t.element_size()))
+        return t
+    monkeypatch.setattr(T.torch, "empty", empty)
+    R = B * TN
+    res = T._layer_forward_native(torch.zeros(R, D), torch.zeros(R), _weights(), B, TN, None, save)
+    a = got["a"]
+    spans = [(a.P, 8 * R * D), (a.y, 2 * R * D), (a.x2, 2 * R * D), (a.u, 2 * R * F), (a.f, 2 * R * F)]
+    spans += [(a.h, 2 * R * D)] if save else []
+    assert save or not a.h
+    spans.sort()
+    assert all(p + n == q for (p, n), (q, _) in zip(spans, spans[1:]))
+    assert (spans[0][0], sum(n for _, n in spans)) in sizes
+    if save:
+        ctx = res[3]
+        assert [ctx.P.data_ptr(), ctx.y.data_ptr(), ctx.x2.data_ptr(), ctx.u.data_ptr(), ctx.f.data_ptr(),
+                ctx.h.data_ptr()] == [a.P, a.y, a.x2, a.u, a.f, a.h]
