@@ -424,13 +424,13 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int S, long
 }
 
 // out[k] (+)= sum_b part[b, k].  Block: 32 columns x 32 row groups; group g adds rows g, g+32, ...
-// in order, then the group sums are added in group order: a fixed tree, so the result
-// does not depend on scheduling.
+// in order, then a warp adds the 32 group sums of a column as a binary tree: a fixed order, so the
+// result does not depend on scheduling, with five roundings at the size of the total instead of 31.
 constexpr int COLSUM_COLS = 32, COLSUM_GROUPS = 32;
 template <typename OT>
 __global__ void colsum_kernel(const float* __restrict__ part, int NB, int K, OT* __restrict__ out,
                               int accumulate) {
-  __shared__ float sm[COLSUM_GROUPS][COLSUM_COLS];
+  __shared__ float sm[COLSUM_GROUPS][COLSUM_COLS + 1];
   const int col = threadIdx.x & (COLSUM_COLS - 1), grp = threadIdx.x / COLSUM_COLS;
   const int k = blockIdx.x * COLSUM_COLS + col;
   float s = 0.f;
@@ -447,19 +447,19 @@ __global__ void colsum_kernel(const float* __restrict__ part, int NB, int K, OT*
   }
   sm[grp][col] = s;
   __syncthreads();
-  if (grp == 0 && k < K) {
-    float t = sm[0][col];
+  float t = sm[col][grp];                  // lane = group, warp = column
 #pragma unroll
-    for (int g = 1; g < COLSUM_GROUPS; ++g) t += sm[g][col];
-    store_grad1(out + k, accumulate ? (float)out[k] + t : t);
-  }
+  for (int o = 1; o < COLSUM_GROUPS; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  const int kc = blockIdx.x * COLSUM_COLS + grp;
+  if (col == 0 && kc < K) store_grad1(out + kc, accumulate ? (float)out[kc] + t : t);
 }
 
 // Partial column sums of a bf16 [R, N] matrix (a bias gradient): part[b, n] over the rows of row block b, which the
 // column sum above then adds in block order.  A warp takes 256 columns, 8 to a lane in one 16-byte load, and every
-// eighth row of the block, four rows in flight; the warps are joined in warp order.  Bound by HBM: 64 095 x 1024
+// eighth row of the block, four rows in flight; the warps are joined as a binary tree.  Bound by HBM: 64 095 x 1024
 // with the column sum 38 us (an fp32 copy of the matrix and a reduction over it: 262); 8000 x 512 13 (41).  Error of
-// the fp32 sums against 64 bits there: rms 2.8e-5 (2.8e-5) and 5.7e-6 (4.5e-6), of sums of the order of 250 and 90.
+// the fp32 sums against 64 bits there: rms 1.6e-5 (2.8e-5) and 4.1e-6 (4.5e-6), of sums of the order of 250 and 90; with
+// the warps and the groups added one after the other it was 2.8e-5 and 5.7e-6.
 // grid: (ceil(N / 256), row blocks); N a multiple of 8, 16-byte aligned rows.
 __global__ void __launch_bounds__(256)
 colsum_rows_kernel(const __nv_bfloat16* __restrict__ x, long long R, int N, int rows_per_block, float* __restrict__ part) {
@@ -491,10 +491,14 @@ colsum_rows_kernel(const __nv_bfloat16* __restrict__ x, long long R, int N, int 
   __syncthreads();
   const int col = blockIdx.x * 256 + threadIdx.x;
   if (col < N) {
-    float t = sm[0][threadIdx.x];
+    float t[8];
 #pragma unroll
-    for (int w = 1; w < 8; ++w) t += sm[w][threadIdx.x];
-    part[(long long)blockIdx.y * N + col] = t;
+    for (int w = 0; w < 8; ++w) t[w] = sm[w][threadIdx.x];
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+      for (int w = 0; w < 8; w += 2 * o) t[w] += t[w + o];
+    part[(long long)blockIdx.y * N + col] = t[0];
   }
 }
 

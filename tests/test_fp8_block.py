@@ -208,3 +208,13 @@ def test_bias_gradient_column_sums(R, N, dt):
     rnd = 2.0 ** -8 if dt is torch.bfloat16 else 0.0
     assert got.dtype == dt and ((got.double() - ref).abs() <= (R + 1) * 2.0 ** -24 * mag + rnd * ref.abs()).all()
     assert torch.equal(got, FB._bias_grad(x, dt))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("R,N", [(8000, 512), (64095, 1024), (2001, 128)])
+def test_bias_gradient_error_is_no_larger_than_that_of_the_fp32_reduction(R, N):
+    """fp32 column sums against 64 bits, next to PyTorch's reduction of an fp32 copy, which they take the place of."""
+    x = torch.randn(R, N, generator=torch.Generator(device="cuda").manual_seed(R), device="cuda").bfloat16()
+    ref = x.double().sum(0)
+    rms = lambda s: float((s.double() - ref).square().mean().sqrt())
+    assert rms(FB._bias_grad(x, torch.float32)) <= rms(x.float().sum(0))
