@@ -1104,10 +1104,10 @@ static int launch_embed_bwd(const TokT* st, const long long* pm, const __nv_bflo
 extern "C" int ccb_embed_bwd_sorted_as(const void* sorted_tok, int64_t tok_bytes, const int64_t* perm, const void* dx,
                                        float* dE, float* slots, int64_t R, int64_t D, int64_t V, void* stream) {
   if (R <= 0) return 0;
-  if (slots == nullptr) return set_error("ccb_embed_bwd_sorted: the boundary-slot workspace is required");
-  if (tok_bytes != 8 && tok_bytes != 2) return set_error("ccb_embed_bwd_sorted: tokens of %lld bytes", (long long)tok_bytes);
+  if (slots == nullptr) return set_error("ccb_embed_bwd_sorted_as: the boundary-slot workspace is required");
+  if (tok_bytes != 8 && tok_bytes != 2) return set_error("ccb_embed_bwd_sorted_as: tokens of %lld bytes", (long long)tok_bytes);
   if (D != 256 && D != 512 && D != 1024)
-    return set_error("ccb_embed_bwd_sorted: D=%lld unsupported (256, 512, 1024)", (long long)D);
+    return set_error("ccb_embed_bwd_sorted_as: D=%lld unsupported (256, 512, 1024)", (long long)D);
   cudaStream_t s = (cudaStream_t)stream;
   const long long* pm = (const long long*)perm;
   const __nv_bfloat16* g = (const __nv_bfloat16*)dx;
@@ -1120,11 +1120,6 @@ extern "C" int ccb_embed_bwd_sorted_as(const void* sorted_tok, int64_t tok_bytes
     return launch_embed_bwd<4>(st, pm, g, dE, slots, fp, lp, R, V, s);
   };
   return tok_bytes == 8 ? run((const long long*)sorted_tok) : run((const short*)sorted_tok);
-}
-extern "C" int ccb_embed_bwd_sorted(const int64_t* sorted_tok, const int64_t* perm, const void* dx,
-                                    float* dE, float* slots, int64_t R, int64_t D, int64_t V,
-                                    void* stream) {
-  return ccb_embed_bwd_sorted_as(sorted_tok, 8, perm, dx, dE, slots, R, D, V, stream);
 }
 
 static int launch_colsum(const float* part, int64_t NB, int64_t K, void* out, int out_bf16, int64_t accumulate,
@@ -1177,7 +1172,7 @@ extern "C" int ccb_splitk_reduce_parts(const float* part, int64_t S, int64_t spl
                                        void* colsum_out, int64_t colsum_accumulate, void* stream) {
   if (N <= 0 || K <= 0) return 0;
   if (nout < 1 || nout > 4 || N % nout != 0)
-    return set_error("ccb_splitk_reduce: %lld rows into %lld tensors", (long long)N, (long long)nout);
+    return set_error("ccb_splitk_reduce_parts: %lld rows into %lld tensors", (long long)N, (long long)nout);
   cudaStream_t s = (cudaStream_t)stream;
   const __nv_bfloat16* cs = (const __nv_bfloat16*)colscale;
   const __nv_bfloat16* w = (const __nv_bfloat16*)W;
@@ -1196,14 +1191,6 @@ extern "C" int ccb_splitk_reduce_as(const float* part, int64_t S, int64_t split_
                                     int64_t colsum_accumulate, void* stream) {
   return ccb_splitk_reduce_parts(part, S, split_stride, N, K, colscale, W, scale, &out, 1, out_bf16, accumulate, colpart,
                                  colsum_out, colsum_accumulate, stream);
-}
-
-extern "C" int ccb_splitk_reduce(const float* part, int64_t S, int64_t split_stride, int64_t N,
-                                 int64_t K, const void* colscale, const void* W, float* out,
-                                 int64_t accumulate, float* colpart, float* colsum_out,
-                                 int64_t colsum_accumulate, void* stream) {
-  return ccb_splitk_reduce_as(part, S, split_stride, N, K, colscale, W, nullptr, out, 0, accumulate, colpart,
-                              colsum_out, colsum_accumulate, stream);
 }
 
 extern "C" int ccb_colsum_as(const float* part, int64_t NB, int64_t K, void* out, int64_t out_bf16,

@@ -79,7 +79,6 @@ _SIGS = {
     "ccb_plain_scan_fwd": ([vp, i64, vp, i64, vp, vp, vp, i64, i64, i64, vp], C.c_int),
     "ccb_plain_scan_bwd": ([vp, i64, vp, vp, vp, i64, vp, vp, vp, i64, i64, i64, vp], C.c_int),
     "ccb_embed_fwd": ([vp, i64, vp, vp, vp, i64, i64, i64, vp], C.c_int),
-    "ccb_embed_bwd_sorted": ([vp, vp, vp, vp, vp, i64, i64, i64, vp], C.c_int),
     "ccb_embed_bwd_sorted_as": ([vp, i64, vp, vp, vp, vp, i64, i64, i64, vp], C.c_int),
     "ccb_token_keys": ([vp, i64, vp, i64, i64, vp], C.c_int),
     "ccb_embed_bwd_slots": ([i64, i64, i64], C.c_int64),
@@ -90,7 +89,6 @@ _SIGS = {
     "ccb_gemm_l2_prefetch": ([C.c_int], C.c_int),
     "ccb_lmhead_debug": ([C.c_int], C.c_int),
     "ccb_lmhead_deep_ring": ([C.c_int], C.c_int),
-    "ccb_splitk_reduce": ([vp, i64, i64, i64, i64, vp, vp, vp, i64, vp, vp, i64, vp], C.c_int),
     "ccb_splitk_reduce_as": ([vp, i64, i64, i64, i64, vp, vp, vp, vp, i64, i64, vp, vp, i64, vp], C.c_int),
     "ccb_colsum": ([vp, i64, i64, vp, i64, vp], C.c_int),
     "ccb_colsum_as": ([vp, i64, i64, vp, i64, i64, vp], C.c_int),
