@@ -829,6 +829,63 @@ plain_scan_bwd_kernel(const DT* __restrict__ decay, const float* __restrict__ st
   }
 }
 
+// The same recurrence, one thread to VEC channels for all steps: for short sequences, where most warps of the
+// kernels above have no step and only pass the state on (the rule is at plain_scan_serial).  Same arithmetic, same bits.
+template <typename DT, typename UT, int VEC>
+__global__ void __launch_bounds__(SCAN_THREADS)
+plain_scan_serial_fwd_kernel(const DT* __restrict__ decay, const UT* __restrict__ update, const float* __restrict__ h0,
+                             float* __restrict__ states, UT* __restrict__ out, int T, int D) {
+  const int b = blockIdx.y, d = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
+  if (d >= D) return;
+  float s[VEC];
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) s[i] = h0 ? h0[(long long)b * D + d + i] : 0.f;
+  long long o = (long long)b * T * D + d;
+  for (int t = 0; t < T; ++t, o += D) {
+    float df[VEC], uf[VEC];
+    raw_get<DT, VEC>(raw_ld<DT, VEC>(decay + o), df);
+    raw_get<UT, VEC>(raw_ld<UT, VEC>(update + o), uf);
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) s[i] = fmaf(df[i], s[i], uf[i]);
+    if (states) raw_st<float, VEC>(states + o, s);
+    if (out) raw_st<UT, VEC>(out + o, s);
+  }
+}
+
+template <typename DT, typename UT, int VEC>
+__global__ void __launch_bounds__(SCAN_THREADS)
+plain_scan_serial_bwd_kernel(const DT* __restrict__ decay, const float* __restrict__ states,
+                             const float* __restrict__ h0, const UT* __restrict__ gstates,
+                             DT* __restrict__ gdecay, UT* __restrict__ gupdate, float* __restrict__ gh0, int T, int D) {
+  const int b = blockIdx.y, d = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
+  if (d >= D) return;
+  const long long base = (long long)b * T * D + d;
+  float g[VEC], dp[VEC];
+  for (int t = T - 1; t >= 0; --t) {
+    const long long o = base + (long long)t * D;
+    float gf[VEC], pf[VEC], gd[VEC];
+    raw_get<UT, VEC>(raw_ld<UT, VEC>(gstates + o), gf);
+    if (t > 0) {
+      raw_get<float, VEC>(raw_ld<float, VEC>(states + o - D), pf);
+    } else {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) pf[i] = h0 ? h0[(long long)b * D + d + i] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+      g[i] = t < T - 1 ? fmaf(g[i], dp[i], gf[i]) : gf[i];
+      gd[i] = g[i] * pf[i];
+    }
+    raw_get<DT, VEC>(raw_ld<DT, VEC>(decay + o), dp);
+    raw_st<UT, VEC>(gupdate + o, g);
+    raw_st<DT, VEC>(gdecay + o, gd);
+  }
+  if (gh0) {
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) gh0[(long long)b * D + d + i] = g[i] * dp[i];
+  }
+}
+
 }  // namespace ccb
 
 using namespace ccb;
@@ -974,6 +1031,19 @@ static inline bool plain_scan_pairs(int64_t D, int64_t dd, int64_t ud, const voi
          ((uintptr_t)st & 7) == 0;
 }
 
+// Whether one thread takes all steps.  A block of the eight-warp kernels costs its hand-over chain whatever the number of
+// steps (2 us forward and 3 backward for every 440 of them), the serial kernels cost a step's latency T times.  Measured
+// on a B200, D = 256, bf16, eight warps / serial in us, forward and backward (events, cold L2; blocks = B x D / 64):
+//   T = 1:  64 rows 8 / 6, 7 / 7         1024 rows 25 / 6, 34 / 6       4096 rows 76 / 8, 117 / 8
+//   T = 8:  64 rows 8 / 8, 8 / 11         256 rows 12 / 8, 15 / 12      4096 rows 84 / 20, 139 / 27
+//   T = 32: 256 rows 12 / 14, 16 / 25     512 rows 18 / 16, 27 / 27     1024 rows 31 / 20, 45 / 35
+//   T = 48: 512 rows 20 / 20, 29 / 39    1024 rows 33 / 29, 51 / 47     2048 rows 57 / 51, 90 / 61
+static bool plain_scan_serial(int64_t B, int64_t T, int64_t lanes, int64_t blocks_per_step) {
+  return T < PS_TT && B * ((lanes + 31) / 32) > blocks_per_step * T;
+}
+// Threads of a serial block: narrow rows do not leave warps idle.
+static int64_t plain_scan_threads(int64_t lanes) { return lanes < SCAN_THREADS ? (lanes + 31) / 32 * 32 : SCAN_THREADS; }
+
 // states: fp32 (kept for backward), out: the states in the update's dtype; either may be null.
 extern "C" int ccb_plain_scan_fwd(const void* decay, int64_t decay_dtype, const void* update,
                                   int64_t update_dtype, const float* h0, float* states, void* out, int64_t B,
@@ -984,10 +1054,13 @@ extern "C" int ccb_plain_scan_fwd(const void* decay, int64_t decay_dtype, const 
                      (long long)decay_dtype, (long long)update_dtype);
   const bool pairs = plain_scan_pairs(D, decay_dtype, update_dtype, decay, decay, update, out ? out : update, states);
   const int64_t lanes = pairs ? D / 2 : D;
-  dim3 grid((unsigned)((lanes + 31) / 32), (unsigned)B);
+  const bool serial = plain_scan_serial(B, T, lanes, 48);
+  const int64_t width = serial ? plain_scan_threads(lanes) : 32;       // lanes of a block
+  dim3 grid((unsigned)((lanes + width - 1) / width), (unsigned)B);
   CCB_SCAN_DISPATCH(decay_dtype, update_dtype, {
-    auto kern = pairs ? plain_scan_fwd_kernel<DT, UT, 2> : plain_scan_fwd_kernel<DT, UT, 1>;
-    kern<<<grid, 32 * PS_NW, 0, (cudaStream_t)stream>>>((const DT*)decay, (const UT*)update, h0, states, (UT*)out, (int)T,
+    auto kern = serial ? (pairs ? plain_scan_serial_fwd_kernel<DT, UT, 2> : plain_scan_serial_fwd_kernel<DT, UT, 1>)
+                       : (pairs ? plain_scan_fwd_kernel<DT, UT, 2> : plain_scan_fwd_kernel<DT, UT, 1>);
+    kern<<<grid, (unsigned)(serial ? width : 32 * PS_NW), 0, (cudaStream_t)stream>>>((const DT*)decay, (const UT*)update, h0, states, (UT*)out, (int)T,
                                                         (int)D);
   });
   count_launch();
@@ -1005,10 +1078,13 @@ extern "C" int ccb_plain_scan_bwd(const void* decay, int64_t decay_dtype, const 
                      (long long)decay_dtype, (long long)update_dtype);
   const bool pairs = plain_scan_pairs(D, decay_dtype, update_dtype, decay, gdecay, gstates, gupdate, states);
   const int64_t lanes = pairs ? D / 2 : D;
-  dim3 grid((unsigned)((lanes + 31) / 32), (unsigned)B);
+  const bool serial = plain_scan_serial(B, T, lanes, 80);
+  const int64_t width = serial ? plain_scan_threads(lanes) : 32;
+  dim3 grid((unsigned)((lanes + width - 1) / width), (unsigned)B);
   CCB_SCAN_DISPATCH(decay_dtype, update_dtype, {
-    auto kern = pairs ? plain_scan_bwd_kernel<DT, UT, 2> : plain_scan_bwd_kernel<DT, UT, 1>;
-    kern<<<grid, 32 * PS_NW, 0, (cudaStream_t)stream>>>((const DT*)decay, states, h0, (const UT*)gstates, (DT*)gdecay,
+    auto kern = serial ? (pairs ? plain_scan_serial_bwd_kernel<DT, UT, 2> : plain_scan_serial_bwd_kernel<DT, UT, 1>)
+                       : (pairs ? plain_scan_bwd_kernel<DT, UT, 2> : plain_scan_bwd_kernel<DT, UT, 1>);
+    kern<<<grid, (unsigned)(serial ? width : 32 * PS_NW), 0, (cudaStream_t)stream>>>((const DT*)decay, states, h0, (const UT*)gstates, (DT*)gdecay,
                                                         (UT*)gupdate, gh0, (int)T, (int)D);
   });
   count_launch();

@@ -237,3 +237,27 @@ def test_ssm_scan_tiles_against_64_bits(B, T, D, ddt, udt, shift):
         assert ((got[0][:, t].double() - ref).abs() <= rnd[ddt] * ref.abs() + 2 * fp * gm * pm[:, t] + tiny).all()
         c, cm = gg * d64[:, t], gm * d64[:, t].abs()
     assert ((got[2].double() - c).abs() <= 2.0 ** -23 * c.abs() + fp * cm).all()
+
+
+# many rows, few steps: one thread a channel (odd widths: one channel a lane)
+@pytest.mark.parametrize("B,T,D", [(300, 1, 64), (2000, 7, 33), (600, 16, 256), (4100, 31, 66)])
+@pytest.mark.parametrize("ddt,udt", [_COMBOS[0], _COMBOS[3], _COMBOS[5]], ids=lambda d: str(d).replace("torch.", ""))
+@pytest.mark.parametrize("with_h0", [False, True])
+def test_ssm_scan_many_short_rows(B, T, D, ddt, udt, with_h0):
+    """The serial kernels against the eight-warp ones, which the same rows taken four at a time run: the same bits."""
+    g = torch.Generator(device="cuda").manual_seed(B + T)
+    decay = torch.rand(B, T, D, generator=g, device="cuda").to(ddt)
+    update = torch.randn(B, T, D, generator=g, device="cuda").to(udt)
+    h0 = torch.randn(B, D, generator=g, device="cuda") if with_h0 else None
+    go = torch.randn(B, T, D, generator=g, device="cuda").to(udt)
+
+    def run(rows):
+        ins = [t[rows].clone().requires_grad_(True) for t in (decay, update) + ((h0,) if with_h0 else ())]
+        out = S.ssm_scan(*ins)
+        with torch.no_grad():
+            assert torch.equal(S.ssm_scan(*ins), out)
+        return (out, *torch.autograd.grad(out, ins, go[rows]))
+    whole = run(slice(0, B))
+    for rows in (slice(0, 4), slice(B - 4, B)):
+        for a, b in zip(whole, run(rows)):
+            assert torch.equal(a[rows], b)
