@@ -939,9 +939,11 @@ static int launch_tile_bwd(const void* P, int64_t ldp, const float* log_a, const
 //   forward   B = 1: 117 / 11   64: 126 / 32   256: 146 / 91    512: 189 / 167   1024: 283 / 318
 //   backward  B = 1: 181 / 20   64: 191 / 63   256: 228 / 185   512: 318 / 353   1024: 576 / 687
 // so the line lies at 16 (forward) and 8 (backward) warps per SM.  Below 64 steps a tile is partly empty and the
-// lines are equal nearer: B = 256, T = 16: 13 / 17 and 19 / 26; B = 128, T = 32: 15 / 13 and 23 / 19.
+// line is nearer.  4 warps per SM: T = 32 15 / 14 and 24 / 20, T = 24 12 / 12 and 20 / 20; T = 16 10 / 12 and 17 / 17,
+// T = 1 8 / 10 and 13 / 15.  2 per SM: T = 16 10 / 10 and 17 / 13, T = 8 8 / 8 and 13 / 13.  8 per SM: T = 32 16 / 21 and
+// 28 / 28, T = 16 12 / 18 and 19 / 24.
 static bool scan_tiled(int64_t warps, int64_t T, int per_sm) {
-  return g_scan_poly_exp == 2 && warps <= (int64_t)(T >= 64 ? per_sm : 4) * ccb_num_sms();
+  return g_scan_poly_exp == 2 && warps <= (int64_t)(T >= 64 ? per_sm : (T >= 24 ? 4 : 2)) * ccb_num_sms();
 }
 // Blocks of a cluster: while they fit two to an SM and each still has steps (B = 1: 23 us with one block, 11 with
 // eight; 16 rows of 256 channels: 25 with one, 17 with four, 19 with eight).
