@@ -976,10 +976,10 @@ __global__ void sgd_kernel(__nv_bfloat16* __restrict__ p, const float* __restric
 }
 
 // lse[m] from per-(tile, half) partials (max, sum 2^(z - max)) in the log2 domain;
-// partials are laid out [nparts][M], so the lanes of a warp read consecutive rows.  A block takes 32 rows and
-// its warps the partials w, w + LSC_WARPS, ... of each, merged as they arrive and then across warps in warp
-// order: the 128 partials of a 16 384-word vocabulary are one dependent chain when a thread has a row to
-// itself, 26 us for the 511 rows of an evaluation chunk whose logits GEMM takes 12; 4 us with this split.
+// partials are laid out [nparts][M], so the lanes of a warp read consecutive rows.  PW warps of a block share 32 rows
+// and take the partials w, w + PW, ... of each, merged as they arrive and then across warps in warp order: the
+// 128 partials of a 16 384-word vocabulary are one dependent chain when a thread has a row to itself, 26 us for
+// the 511 rows of an evaluation chunk whose logits GEMM takes 12; 4 us with sixteen warps.
 constexpr int LSC_WARPS = 16;
 __device__ __forceinline__ void lse_merge(float2& a, const float2 v) {
   // An empty partial (sum zero) adds nothing, whatever its maximum.  Every other one is merged, so that a sum that is
@@ -990,29 +990,32 @@ __device__ __forceinline__ void lse_merge(float2& a, const float2 v) {
     a.x = m;
   }
 }
+template <int PW>
 __global__ void __launch_bounds__(32 * LSC_WARPS)
 lse_combine_kernel(const float2* __restrict__ part, int nparts, long long M,
                    const float* __restrict__ zt, float* __restrict__ lse, float* __restrict__ loss) {
-  __shared__ float2 join[LSC_WARPS][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long m = (long long)blockIdx.x * 32 + lane;
+  __shared__ float2 join[PW > 1 ? LSC_WARPS : 1][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w0 = warp % PW;
+  const long long m = ((long long)blockIdx.x * (LSC_WARPS / PW) + warp / PW) * 32 + lane;
   float2 a = make_float2(-INFINITY, 0.f);
   if (m < M) {
-    int i = warp;
-    for (; i + 3 * LSC_WARPS < nparts; i += 4 * LSC_WARPS) {
+    int i = w0;
+    for (; i + 3 * PW < nparts; i += 4 * PW) {
       float2 v[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = __ldg(&part[(long long)(i + u * LSC_WARPS) * M + m]);
+      for (int u = 0; u < 4; ++u) v[u] = __ldg(&part[(long long)(i + u * PW) * M + m]);
 #pragma unroll
       for (int u = 0; u < 4; ++u) lse_merge(a, v[u]);
     }
-    for (; i < nparts; i += LSC_WARPS) lse_merge(a, __ldg(&part[(long long)i * M + m]));
+    for (; i < nparts; i += PW) lse_merge(a, __ldg(&part[(long long)i * M + m]));
   }
-  join[warp][lane] = a;
-  __syncthreads();
-  if (warp == 0 && m < M) {
+  if constexpr (PW > 1) {
+    join[warp][lane] = a;
+    __syncthreads();
+  }
+  if (w0 == 0 && m < M) {
 #pragma unroll
-    for (int w = 1; w < LSC_WARPS; ++w) lse_merge(a, join[w][lane]);
+    for (int w = 1; w < PW; ++w) lse_merge(a, join[warp + w][lane]);
     const float l = (a.x + log2f(a.y)) * 0.6931471805599453f;
     lse[m] = l;
     if (loss != nullptr && zt != nullptr) loss[m] = l - zt[m];
@@ -1434,7 +1437,13 @@ extern "C" int ccb_sgd(void* p, const float* g, int64_t n, float lr, void* strea
 extern "C" int ccb_lse_combine(const float* part, int64_t nparts, int64_t M, const float* zt, float* lse,
                                float* loss, void* stream) {
   if (M <= 0) return 0;
-  lse_combine_kernel<<<(unsigned)((M + 31) / 32), 32 * LSC_WARPS, 0, (cudaStream_t)stream>>>(
+  // Warps to a row: one while its partials are two rounds of loads, sixteen for long lists of few rows, else four.
+  // 1 / 4 / 16 in us (events, cold L2): 65 536 rows of 4 partials 8 / 8 / 16, of 32 14 / 12 / 23, of 128 38 / 22 / 30;
+  // 9000 rows of 64 21 / 10 / 10, of 128 33 / 14 / 10; 20 000 rows of 128 33 / 15 / 15; 511 rows of 32 12 / 8 / 8.
+  const int pw = nparts <= 8 ? 1 : (nparts > 32 && M <= 16384 ? 16 : 4);
+  const long long rows = 32 * (LSC_WARPS / pw);
+  auto kern = pw == 1 ? lse_combine_kernel<1> : (pw == 4 ? lse_combine_kernel<4> : lse_combine_kernel<16>);
+  kern<<<(unsigned)((M + rows - 1) / rows), 32 * LSC_WARPS, 0, (cudaStream_t)stream>>>(
       (const float2*)part, (int)nparts, (long long)M, zt, lse, loss);
   CCB_CHECK_LAUNCH("lse_combine");
   return 0;

@@ -325,3 +325,23 @@ def test_split_one_sweep_keeps_the_rows_own_reference(R, V, epilogue_parts):
     assert torch.allclose(lse, rlse, rtol=1e-3, atol=2e-2) and torch.allclose(loss, rl, rtol=1e-3, atol=3e-2)
     assert torch.allclose(lse, wlse, rtol=0, atol=2e-4) and torch.allclose(loss, wloss, rtol=0, atol=2e-4)
     assert (dX.float() - wdX.float()).norm() <= 2e-3 * wdX.float().norm()
+
+
+# one warp to a row (at most 8 partials), four, and sixteen (more than 32 partials, at most 16 384 rows)
+@pytest.mark.parametrize("nparts,M", [(8, 513), (9, 129), (32, 127), (33, 33), (33, 16384), (33, 16385)])
+def test_lse_combine_warps_to_a_row(nparts, M):
+    """Against 64 bits, tolerance as above; and the same bits on every run."""
+    g = torch.Generator(device="cuda").manual_seed(nparts + M)
+    part = torch.stack([torch.randn(nparts, M, generator=g, device="cuda") * 30,
+                        torch.rand(nparts, M, generator=g, device="cuda") * 100 + 1e-3], -1).contiguous()
+    zt = torch.randn(M, generator=g, device="cuda")
+    res = []
+    for _ in range(2):
+        lse, loss = torch.empty(M, device="cuda"), torch.empty(M, device="cuda")
+        _lib.check(_lib.lib().ccb_lse_combine(part.data_ptr(), nparts, M, zt.data_ptr(), lse.data_ptr(), loss.data_ptr(),
+                                              _lib.stream_ptr()), "lse_combine")
+        res.append((lse, loss))
+    ref = torch.logsumexp(part[..., 0].double() * 0.6931471805599453 + part[..., 1].double().log(), 0)
+    tol = (nparts + 8) * 2.0 ** -23 + 2.0 ** -23 * ref.abs()
+    assert ((res[0][0].double() - ref).abs() <= tol).all()
+    assert all(torch.equal(a, b) for a, b in zip(*res))
