@@ -556,6 +556,30 @@ extern "C" int ccb_fp8_quant_blocks(const void* w, void* q, void* qt, float* s, 
   return e == cudaSuccess ? 0 : set_error("fp8_quant_blocks launch: %s", cudaGetErrorString(e));
 }
 
+// Column tiles of a CTA in the resident-weight kernel (as many as fit, and as leave every CTA at least two row blocks;
+// more than one only while a row block fits the activation ring), or 0: the streaming kernel.  Fewer tiles than SMs: one
+// tile a CTA, streaming.  Otherwise what decides is the tiles of the busiest CTA.  Streaming deals single tiles out, the
+// resident kernel whole column groups, floor(SMs / groups) CTAs to each: 75 groups of a 9600-wide result leave 73 of 148
+// SMs without any.  Its tiles are cheaper, more so where a row block serves several of them.  Measured at 65 536 rows
+// (events, cold L2; work = tiles of the busiest CTA, resident / streaming; time = resident / streaming):
+//   K = 128 (up to 8 tiles):     work 1.00 time 0.88, 1.16 0.97, 1.24 1.02, 1.29 1.06, 1.60 1.29    -> up to 7/6
+//   K = 256 .. 512 (2 or 4):     1.00 0.73-0.85, 1.19 0.89-0.99, 1.32 0.94-0.98, 1.33 0.97-1.09, 1.48 1.25-1.28, 1.97 1.4
+//                                                                                                    -> below 4/3
+//   K = 640 .. 1024 (1):         1.00 0.89-0.96, 1.06 0.97, 1.15 1.10, 1.18 1.08, 1.48 1.27-1.53, 1.97 1.67 -> up to 17/16
+extern "C" int64_t ccb_fp8_block_plan(int64_t M, int64_t N, int64_t K, int64_t sms) {
+  const int64_t kb = K / 128, tm = (M + FB_BM - 1) / FB_BM, tn = (N + FB_BN - 1) / FB_BN, total = tm * tn;
+  if (kb < 1 || kb > FbCfg<1>::RES_TILES || total <= sms) return 0;
+  int64_t nt = kb <= 4 ? FbCfg<1>::RES_TILES / kb : 1;
+  if (nt > total / (2 * sms)) nt = total / (2 * sms);
+  if (nt < 1) nt = 1;
+  const int64_t groups = (tn + nt - 1) / nt;
+  if (groups > sms) return 0;
+  const int64_t walkers = sms / groups < tm ? sms / groups : tm;
+  const int64_t res = (tm + walkers - 1) / walkers * (nt < tn ? nt : tn), str = (total + sms - 1) / sms;
+  const bool even = kb == 1 ? 6 * res <= 7 * str : (kb <= 4 ? 3 * res < 4 * str : 16 * res <= 17 * str);
+  return even ? nt : 0;
+}
+
 extern "C" int ccb_fp8_block_gemm(const void* A8, const float* sa_t, const void* B8, const float* sb,
                                   int64_t sb_so, int64_t sb_sk, void* C, int64_t ldc, int64_t out_fp32,
                                   const void* bias, int64_t M, int64_t N, int64_t K, void* stream) {
@@ -581,14 +605,10 @@ extern "C" int ccb_fp8_block_gemm(const void* A8, const float* sa_t, const void*
   p.status = ccb_status_ptr();
   const long long total = (long long)p.tiles_m * p.tiles_n;
   const int sms = ccb_num_sms();
-  // Resident weights: column tiles of a CTA as many as fit, and as leave every CTA at least two row blocks; more
-  // than one only while the row block fits the activation ring.  Fewer tiles than SMs: one tile a CTA.
-  int nt = p.kblocks <= 4 ? FbCfg<1>::RES_TILES / p.kblocks : 1;
-  if (nt > total / (2 * sms)) nt = (int)(total / (2 * sms));
-  if (nt < 1) nt = 1;
-  p.nt = nt;
-  p.groups = (p.tiles_n + nt - 1) / nt;
-  if (p.kblocks <= FbCfg<1>::RES_TILES && total > sms && p.groups <= sms) {
+  p.nt = (int)ccb_fp8_block_plan(M, N, K, sms);
+  p.groups = 1;
+  if (p.nt > 0) {
+    p.groups = (p.tiles_n + p.nt - 1) / p.nt;
     const long long walkers = sms / p.groups < p.tiles_m ? sms / p.groups : p.tiles_m;
     return launch_block_gemm<1>((int)(walkers * p.groups), tmA, tmB, tmC, p, (cudaStream_t)stream);
   }

@@ -63,6 +63,7 @@ _SIGS = {
     "ccb_newton_schulz": ([vp, vp, vp, vp, i64, i64, i64, i64, f32, f32, f32, vp], C.c_int),
     "ccb_lse_combine": ([vp, i64, i64, vp, vp, vp, vp], C.c_int),
     "ccb_fp8_quant_rows": ([vp, i64, vp, f32, vp, vp, vp, vp, i64, i64, vp], C.c_int),
+    "ccb_fp8_block_plan": ([i64, i64, i64, i64], i64),
     "ccb_fp8_quant_blocks": ([vp, vp, vp, vp, i64, i64, vp], C.c_int),
     "ccb_fp8_block_gemm": ([vp, vp, vp, vp, i64, i64, vp, i64, i64, vp, i64, i64, i64, vp], C.c_int),
     "ccb_fp8_cast_amax": ([vp, vp, vp, vp, i64, i64, vp], C.c_int),

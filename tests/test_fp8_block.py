@@ -218,3 +218,63 @@ def test_bias_gradient_error_is_no_larger_than_that_of_the_fp32_reduction(R, N):
     ref = x.double().sum(0)
     rms = lambda s: float((s.double() - ref).square().mean().sqrt())
     assert rms(FB._bias_grad(x, torch.float32)) <= rms(x.float().sum(0))
+
+
+def _plan(M, N, K, sms=148):
+    from chaoscontrol_b200.ops import _lib
+    if not _lib._LIB_PATH.exists():
+        pytest.skip("the kernel library is not built")
+    return int(_lib.lib().ccb_fp8_block_plan(M, N, K, sms))
+
+
+def _work(M, N, K, nt, sms=148):
+    """Tiles of the busiest CTA: of the resident kernel with ``nt`` column tiles to a CTA, of the streaming kernel."""
+    tm, tn = -(-M // 128), -(-N // 128)
+    if nt == 0:
+        return -(-tm * tn // sms)
+    return -(-tm // min(sms // -(-tn // nt), tm)) * min(nt, tn)
+
+
+@pytest.mark.parametrize("K", [128, 256, 384, 512, 640, 1024, 1152])
+def test_resident_weights_keep_the_sms_busy(K):
+    """Over the sizes of a layer and far beyond: the resident kernel is taken only while its busiest CTA has little more
+    to do than the streaming kernel's."""
+    limit = 7 / 6 if K == 128 else (4 / 3 if K <= 512 else 17 / 16)
+    taken = 0
+    for M in (100, 2560, 9000, 18944, 20000, 65536, 300001):
+        for N in list(range(128, 2049, 128)) + [136, 2500, 3200, 6400, 9600, 12800, 18944, 19200, 50304]:
+            nt = _plan(M, N, K)
+            if nt:
+                taken += 1
+                assert K <= 1024 and nt * (K // 128) <= 8 and (nt == 1 or K <= 512)
+                assert _work(M, N, K, nt) <= limit * _work(M, N, K, 0), (M, N)
+    assert (taken > 0) == (K <= 1024)
+
+
+@pytest.mark.parametrize("M,N,K,resident", [(65536, 1024, 256, True), (65536, 1024, 1024, True), (65536, 896, 1024, True),
+                                            (65536, 640, 384, True), (65536, 9600, 1024, False), (65536, 6400, 1024, False),
+                                            (65536, 19200, 512, False), (65536, 18944, 512, True), (128, 1024, 256, False)])
+def test_resident_weights_at_measured_sizes(M, N, K, resident):
+    assert (_plan(M, N, K) > 0) == resident
+
+
+# four column tiles to a CTA with a last group of three, two with a last group of one, eight; ragged last row and column
+# tiles; wide results that stream
+@pytest.mark.gpu
+@pytest.mark.parametrize("R,K,N,nt", [(37838, 256, 888, 4), (37627, 512, 520, 2), (75700, 128, 1024, 8),
+                                      (2500, 1024, 9600, 0), (2500, 512, 19000, 0)])
+def test_block_gemm_column_groups(R, K, N, nt):
+    """As the resident-weight test above, against 64-bit products."""
+    from chaoscontrol_b200.ops import _lib
+    assert _plan(R, N, K, _lib.lib().ccb_num_sms()) == nt
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    qa, _, _ = FB.quant_rows(torch.randn(R, K, generator=g, device="cuda").bfloat16())
+    q, _, s = FB.quant_blocks((torch.randn(N, K, generator=g, device="cuda") * 0.1).bfloat16())
+    out = FB.block_gemm(qa, q, s, sb_strides=(s.shape[1], 1))
+    _lib.assert_ok()
+    a = (qa.q.double().view(R, K // 128, 128) * qa.s_t.double().t().unsqueeze(-1)).view(R, K)
+    nb = s.shape[0]
+    pad = torch.nn.functional.pad(q.double(), (0, 0, 0, nb * 128 - N)).view(nb, 128, K // 128, 128)
+    w = (pad * s.double()[:, None, :, None]).view(nb * 128, K)[:N]
+    ref, mag = a @ w.t(), a.abs() @ w.abs().t()
+    assert ((out.double() - ref).abs() <= (K + 8) * 2.0 ** -24 * mag + 2.0 ** -8 * ref.abs()).all()
