@@ -232,8 +232,10 @@ class LayerWeights:
         if not _plain_bf16(*ops):
             return False
         F_, D = self.Wfc.shape
-        mats = [(t, (D, D)) for t in parts] if parts is not None else [(self.Wp, (4 * D, D))]
-        if not _shaped((self.wn1, (D,)), (self.wn2, (D,)), (self.log_a, (D,)), *mats):
+        sq = (D, D)
+        if not (self.wn1.shape == (D,) and self.wn2.shape == (D,) and self.log_a.shape == (D,) and
+                (self.Wp.shape == (4 * D, D) if parts is None else
+                 parts[0].shape == sq and parts[1].shape == sq and parts[2].shape == sq and parts[3].shape == sq)):
             return False
         dev = self.Wfc.device
         Wp = torch.empty(4 * D, D, dtype=torch.bfloat16, device=dev) if parts is not None else None
@@ -341,14 +343,12 @@ def _plain_bf16(*ts) -> bool:
     return all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() for t in ts)
 
 
-def _shaped(*pairs) -> bool:
-    """The native layer calls take addresses and the sizes of one layer: every (tensor, shape) has to be as they say.
-    Anything else goes through the step-by-step form, whose operations check (or broadcast) what they are given."""
-    return all(tuple(t.shape) == shape for t, shape in pairs)
-
-
 def _layer_shaped(w: "LayerWeights", D: int, F_: int) -> bool:
-    return _shaped((w.Wp_f, (4 * D, D)), (w.Wfc_f, (F_, D)), (w.Wo, (D, D)), (w.Wproj, (D, F_)), (w.log_a32, (D,)))
+    """The native layer calls take addresses and the sizes of one layer: every operand's shape has to be as they say.
+    Anything else goes through the step-by-step form, whose operations check (or broadcast) what they are given.
+    (Written out: a layer's host time is part of a small batch's.)"""
+    return (w.Wp_f.shape == (4 * D, D) and w.Wfc_f.shape == (F_, D) and w.Wo.shape == (D, D) and
+            w.Wproj.shape == (D, F_) and w.log_a32.shape == (D,))
 
 
 def _plain_f32(*ts) -> bool:
@@ -374,7 +374,7 @@ def _layer_forward_native(x, ss1, w, B, T, h0, save):
     R, D = x.shape
     F_ = w.Wfc.shape[0]
     if not (R == B * T and R > 0 and D % 8 == 0 and F_ % 8 == 0 and _layer_shaped(w, D, F_) and
-            _shaped((ss1, (R,))) and
+            ss1.shape == (R,) and
             _plain_bf16(x, w.Wp_f, w.Wfc_f, w.Wo, w.Wproj) and _plain_f32(ss1, w.log_a32, h0)):
         return None
     dev = x.device
@@ -400,19 +400,25 @@ def _layer_backward_native(dx3, ctx, w, B, T, dhT, want_dh0, outs, grad_dtype, s
     F_ = ctx.F
     if not (_plain_bf16(dx3, w.Wp_f, w.Wfc_f, w.Wo, w.Wproj, w.Wp, w.Wfc, w.wn1, w.wn2) and
             _plain_f32(w.log_a32, dhT) and dx3.shape == ctx.x.shape and _layer_shaped(w, D, F_) and
-            _shaped((w.Wp, (4 * D, D)), (w.Wfc, (F_, D)), (w.wn1, (D,)), (w.wn2, (D,)))):
+            w.Wp.shape == (4 * D, D) and w.Wfc.shape == (F_, D) and w.wn1.shape == (D,) and w.wn2.shape == (D,)):
         return None
     dev = dx3.device
-    shapes = ((4 * D, D), (D, D), (F_, D), (D, F_), (D,), (D,), (D,))      # in the order of _GRAD_KEYS
     if outs:
-        if grad_dtype != torch.float32 or any(k not in outs for k in _GRAD_KEYS) or not _plain_f32(
-                *(outs[k] for k in _GRAD_KEYS)) or not _shaped(*((outs[k], s) for k, s in zip(_GRAD_KEYS, shapes))):
+        if grad_dtype != torch.float32 or any(k not in outs for k in _GRAD_KEYS):
             return None
         g = [outs[k] for k in _GRAD_KEYS]
+        if not (_plain_f32(*g) and g[0].shape == (4 * D, D) and g[1].shape == (D, D) and g[2].shape == (F_, D) and
+                g[3].shape == (D, F_) and g[4].shape == g[5].shape == g[6].shape == (D,)):
+            return None
     elif grad_dtype in (torch.float32, torch.bfloat16):
         # an allocation each: a gradient that is kept, saved or changed in place leaves the others alone
-        each = lambda *ss: [torch.empty(s, dtype=grad_dtype, device=dev) for s in ss]
-        g = [tuple(each(*[(D, D)] * 4)), *each(*shapes[1:])] if split_wp else each(*shapes)
+        new, Wo, wn1 = torch.empty_like, w.Wo, w.wn1
+        if grad_dtype == torch.bfloat16:
+            g = [new(Wo), new(w.Wfc), new(w.Wproj), new(wn1), new(wn1), new(wn1)]
+            g.insert(0, (new(Wo), new(Wo), new(Wo), new(Wo)) if split_wp else new(w.Wp))
+        else:
+            g = [new(t, dtype=grad_dtype) for t in (Wo, w.Wfc, w.Wproj, wn1, wn1, wn1)]
+            g.insert(0, tuple(new(Wo, dtype=grad_dtype) for _ in range(4)) if split_wp else new(w.Wp, dtype=grad_dtype))
     else:
         return None
     L = _lib.lib()
