@@ -309,7 +309,7 @@ struct SpkOut {
   OT* p[4];
   int rows;
   __device__ __forceinline__ OT* row(int n, int K) const {
-    const int i = n / rows;
+    const int i = (n >= rows) + (n - rows >= rows) + (n - rows - rows >= rows);      // rows = N for one tensor
     return p[i] + (long long)(n - i * rows) * K;
   }
 };
