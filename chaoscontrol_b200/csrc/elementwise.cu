@@ -186,21 +186,23 @@ __global__ void embed_bwd_runs_kernel(const TokT* __restrict__ sorted_tok,
 // A token's boundary slots k = w, w + 16, ... are added by warp w in order (lane l owns columns
 // [l * D/32, (l+1) * D/32)) and the sixteen sums are added in warp order: a fixed tree, wide enough that the most
 // frequent token of a Zipf batch (thousands of chunks) does not serialise behind one warp.  Up to sixteen slots the
-// tree is a plain sum in slot order, which one warp does by itself.  So a block takes JOIN_TOKS tokens, a grid apart
-// so that neighbouring ids (frequent ones come together) spread over blocks: its warps take the short ones side by
-// side, then all of them each long one.  A block of sixteen warps per token, most of which had nothing to join,
-// took 44 us at 32 768 rows and V = 16 384; 10 now.
+// tree is a plain sum in slot order, which one warp does by itself.  So a block takes up to JOIN_TOKS tokens, a grid
+// apart so that neighbouring ids (frequent ones come together) spread over blocks: its warps take the short ones side
+// by side, then all of them each long one.  A block of sixteen warps per token, most of which had nothing to join,
+// took 44 us at 32 768 rows and V = 16 384; 10 now.  A small vocabulary has few tokens and all of them long: its blocks
+// take fewer, four blocks to an SM.  With 32 tokens to a block 262 144 rows over 256 words ran on 8 SMs (runs and join
+// 102 us, one token to a block 53).
 // first_pos / last_pos come from stage 1; last_pos is -1 for tokens that do not occur.
 constexpr int EMB_JOIN_WARPS = 16, EMB_JOIN_TOKS = 32;
 template <int FPL>   // floats per lane: D = 32 * FPL
 __global__ void __launch_bounds__(EMB_JOIN_WARPS * 32)
 embed_bwd_join_kernel(const long long* __restrict__ first_pos, const long long* __restrict__ last_pos,
-                      const float* __restrict__ slots, float* __restrict__ dE, int D, int V) {
+                      const float* __restrict__ slots, float* __restrict__ dE, int D, int V, int toks) {
   extern __shared__ float sm_join[];          // [EMB_JOIN_WARPS][D]
   __shared__ long long s_first[EMB_JOIN_TOKS], s_n[EMB_JOIN_TOKS];     // first position; slots to add (0: none)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = lane * FPL;
-  if (threadIdx.x < EMB_JOIN_TOKS) {
+  if (threadIdx.x < toks) {
     const long long tk = (long long)blockIdx.x + (long long)threadIdx.x * gridDim.x;
     long long s = 0, n = 0;
     if (tk < V) {
@@ -250,7 +252,7 @@ embed_bwd_join_kernel(const long long* __restrict__ first_pos, const long long* 
       }
     }
   };
-  for (int j = warp; j < EMB_JOIN_TOKS; j += EMB_JOIN_WARPS) {
+  for (int j = warp; j < toks; j += EMB_JOIN_WARPS) {
     const long long n = s_n[j];
     if (n == 0 || n > EMB_JOIN_WARPS) continue;
     add_slots(j, 0, n, 1);
@@ -258,7 +260,7 @@ embed_bwd_join_kernel(const long long* __restrict__ first_pos, const long long* 
 #pragma unroll
     for (int i = 0; i < FPL / 4; ++i) o[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
   }
-  for (int j = 0; j < EMB_JOIN_TOKS; ++j) {
+  for (int j = 0; j < toks; ++j) {
     const long long n = s_n[j];
     if (n <= EMB_JOIN_WARPS) continue;        // the same for the whole block
     add_slots(j, warp, n, EMB_JOIN_WARPS);
@@ -1097,8 +1099,10 @@ static int launch_embed_bwd(const TokT* st, const long long* pm, const __nv_bflo
   constexpr int smem = EMB_JOIN_WARPS * D * (int)sizeof(float);
   // sixteen [1024] strips are 64 KiB of shared memory: above the default limit, opt in
   if (smem > 48 * 1024) cudaFuncSetAttribute(embed_bwd_join_kernel<D / 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  embed_bwd_join_kernel<D / 32><<<(unsigned)((V + EMB_JOIN_TOKS - 1) / EMB_JOIN_TOKS), EMB_JOIN_WARPS * 32, smem, s>>>(
-      fp, lp, slots, dE, D, (int)V);
+  const int64_t want = (V + 4 * ccb_num_sms() - 1) / (4 * ccb_num_sms());
+  const int toks = (int)(want < EMB_JOIN_TOKS ? want : EMB_JOIN_TOKS);
+  embed_bwd_join_kernel<D / 32><<<(unsigned)((V + toks - 1) / toks), EMB_JOIN_WARPS * 32, smem, s>>>(
+      fp, lp, slots, dE, D, (int)V, toks);
   CCB_CHECK_LAUNCH("embed_bwd_join");
   return 0;
 }

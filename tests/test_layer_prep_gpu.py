@@ -127,3 +127,17 @@ def test_parameter_gradients_own_their_memory():
     seen = [t._version for t in grads]
     grads[0].zero_()
     assert [t._version for t in grads[1:]] == seen[1:]
+
+
+# tokens of a join block: 1, 2 and 7 (four blocks to an SM), then 32; the block's share that is not full
+@pytest.mark.parametrize("V", [256, 600, 4100, 20000])
+def test_embed_bwd_join_blocks(V):
+    """Every word joined, long and short runs side by side, against 64-bit sums (at most 9000 fp32 additions a row)."""
+    g = torch.Generator(device="cuda").manual_seed(V)
+    tok = torch.cat([torch.randint(0, V, (60000,), generator=g, device="cuda"),
+                     torch.full((8000,), V - 1, device="cuda"), torch.full((700,), V // 2, device="cuda")])
+    dx = torch.randn(tok.numel(), 256, generator=g, device="cuda").bfloat16()
+    got = trunk.embed_bwd(tok, dx, V)
+    ref = torch.zeros(V, 256, dtype=torch.float64, device="cuda").index_add_(0, tok, dx.double())
+    mag = torch.zeros(V, 256, dtype=torch.float64, device="cuda").index_add_(0, tok, dx.double().abs())
+    assert ((got.double() - ref).abs() <= 9000 * 2.0 ** -24 * mag).all()
