@@ -288,7 +288,7 @@ embed_bwd_join_kernel(const long long* __restrict__ first_pos, const long long* 
 // Bound by the latency of the partials' loads (they sit in L2): a weight gradient of the trunk is only
 // N x K = 64 K elements with S = 148 / tiles partials each.  So a block is small (8 rows x 64 columns,
 // one float4 per thread) and the partials are split over G thread groups, each adding a contiguous range
-// of them in index order; the groups are joined in group order through shared memory: a fixed tree.
+// of them, four at a time in pairs; the groups are joined in group order through shared memory: a fixed tree.
 // A block of 8 full rows with one thread per column (the kernel below, 32 blocks for a 256 x 256 output)
 // took 630 of the 4 260 us of a 4-layer training step at 32 768 rows; with this one the step went from
 // 4.51 to 4.04 ms, a 131 072-row block's forward and backward from 1.63 to 1.48 ms.
@@ -341,7 +341,8 @@ splitk_tile_kernel(const float* __restrict__ part, int S, long long split_stride
       const float4 v1 = __ldg(reinterpret_cast<const float4*>(pp + (long long)(sp + 1) * split_stride));
       const float4 v2 = __ldg(reinterpret_cast<const float4*>(pp + (long long)(sp + 2) * split_stride));
       const float4 v3 = __ldg(reinterpret_cast<const float4*>(pp + (long long)(sp + 3) * split_stride));
-      add(v0); add(v1); add(v2); add(v3);
+      add(make_float4((v0.x + v1.x) + (v2.x + v3.x), (v0.y + v1.y) + (v2.y + v3.y), (v0.z + v1.z) + (v2.z + v3.z),
+                      (v0.w + v1.w) + (v2.w + v3.w)));
     }
     for (; sp < s1; ++sp) add(__ldg(reinterpret_cast<const float4*>(pp + (long long)sp * split_stride)));
   }
@@ -1158,10 +1159,17 @@ static int launch_splitk(const float* part, int64_t S, int64_t split_stride, int
                     (K + SPK_COLS - 1) / SPK_COLS <= 65535;
   if (tile) {
     const dim3 grid(nb, (unsigned)((K + SPK_COLS - 1) / SPK_COLS));
-    // groups: each keeps at least four partials, so that its loads are in flight together
-    if (S <= 4) splitk_tile_kernel<1, OT><<<grid, 128, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out, colpart);
-    else if (S <= 8) splitk_tile_kernel<2, OT><<<grid, 256, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out, colpart);
-    else if (S <= 24) splitk_tile_kernel<4, OT><<<grid, 512, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out, colpart);
+    // Groups: as many as make about 1000 blocks' worth of threads, and each keeps at least four partials so that its
+    // loads are in flight together.  A result with blocks enough needs none: they then only cost the joins and read each
+    // partial in smaller pieces.  us with 1 / 2 / 4 / 8 groups (events, cold L2): 74 partials of 256 x 256 20 / 16 / 14 /
+    // 12, 64 of 512 x 256 18 / 16 / 16 / 16, 74 of 1024 x 256 29 / 25 / 31 / 33, 25 of 2048 x 512 31 / 33 / 37 / 47,
+    // 15 of 16 384 x 512 102 / 115 / 143 / 313 (one thread a column: 133).
+    const int64_t blocks = (int64_t)grid.x * grid.y, most = S <= 4 ? 1 : (S <= 8 ? 2 : (S <= 24 ? 4 : 8));
+    int64_t groups = most;
+    while (groups > 1 && blocks * groups > 8 * (int64_t)ccb_num_sms()) groups /= 2;
+    if (groups == 1) splitk_tile_kernel<1, OT><<<grid, 128, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out, colpart);
+    else if (groups == 2) splitk_tile_kernel<2, OT><<<grid, 256, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out, colpart);
+    else if (groups == 4) splitk_tile_kernel<4, OT><<<grid, 512, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out, colpart);
     else splitk_tile_kernel<8, OT><<<grid, 1024, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out, colpart);
   } else {
     splitk_reduce_kernel<OT><<<nb, 256, 0, s>>>(part, (int)S, split_stride, (int)N, (int)K, colscale, W, scale, out,

@@ -46,3 +46,15 @@ def test_splitk_reduce_scale(S, N, K):
     for dt in (torch.float32, torch.bfloat16):
         for a, b in zip(splitk_reduce(part, W=W, out_dtype=dt, scale=up), splitk_reduce(part, W=W, out_dtype=dt)):
             assert torch.equal(a, b * -0.5)
+
+
+# blocks of the result on both sides of the group rule (about 1000 blocks times groups), every group count
+@pytest.mark.parametrize("S,N,K", [(30, 64, 256), (30, 584, 256), (30, 1192, 256), (30, 2376, 256), (12, 1200, 256),
+                                   (6, 2400, 256), (15, 4096, 512)])
+def test_splitk_reduce_group_rule(S, N, K):
+    """fp32 sums against 64 bits: at most S roundings on the sum of magnitudes; the same bits on every run."""
+    part = torch.randn(S, N, K, generator=torch.Generator(device="cuda").manual_seed(N), device="cuda")
+    out, _ = splitk_reduce(part)
+    p64 = part.double()
+    assert ((out.double() - p64.sum(0)).abs() <= S * 2.0 ** -24 * p64.abs().sum(0) + 1e-30).all()
+    assert torch.equal(out, splitk_reduce(part)[0])
