@@ -1216,6 +1216,8 @@ extern "C" int ccb_gemm(const CcbGemmArgs* a, void* stream_) {
       case 1: return launch_gemm<256, 0, 1>(a, stream);
       case 3: {
         const int64_t splits = a->splits < 1 ? 1 : a->splits;
+        // The caller lays the partials out, so their number is what says which tile height it planned for: with the
+        // rule's count for 256-row tiles these fill the SMs, with any other they would leave some idle or go round twice.
         if (a->epi == CCB_EPI_STORE && a->batch == 1 && a->out_fp32 && a->Cin == nullptr && a->bias == nullptr &&
             ccb_gemm_wgrad_splits(a->M, a->N, a->K, 1) == splits)
           return launch_gemm<256, 1, 1, 0, CCB_EPI_STORE, 1, 0, 1>(a, stream);

@@ -101,9 +101,9 @@ struct LmHeadArgs {
 // 71 leave half of the chip idle.  With a workspace the m-tile x v-tile steps are dealt out evenly instead: CTA i
 // takes steps [i * share, (i + 1) * share) of the flattened order, i.e. at most one partial m-tile at either end of
 // its range and whole ones between.  A partial m-tile's row sums and accumulators go to slot 2i or 2i + 1, and
-// lmhead_join_kernel adds the pieces of each m-tile in vocabulary order.  V = 16 384: gradient sweep with a given lse
-// at 512 m-tiles 865 -> 740 us and 11 for the join, one-sweep training at 256 m-tiles 476 -> 420 and 15, scoring at
-// 512 505 -> 490 and 9.
+// lmhead_join_kernel adds the pieces of each m-tile in vocabulary order.  V = 16 384, whole tiles / split with its join:
+// gradient sweep with a given lse at 512 m-tiles 952 -> 830 us, one-sweep training at 250 m-tiles 459 -> 417 (the
+// reference step of its pieces is 4 of them), scoring at 512 639 -> 560.
 struct LhWalk {
   int mode_dw, n_vtiles, n_mtiles, per_chunk;
   int unit, step, units;              // whole units
@@ -160,8 +160,8 @@ __device__ __forceinline__ float ex2f(float x) {
   return y;
 }
 
-// DEEP = 1 (single-sweep kernels: one-sweep training, training with a given lse, dW): the unit's X tile is the logits MMA's A operand from tensor
-// memory instead of shared memory, the 64 KiB it occupied become a THIRD W' stage, and one logits
+// DEEP = 1 (single-sweep kernels: one-sweep training, training with a given lse, dW): the unit's X tile is the
+// logits MMA's A operand from tensor memory instead of shared memory, the 64 KiB it occupied become a THIRD W' stage, and one logits
 // buffer (handed back as soon as the epilogue holds it in registers) makes room for X in tensor
 // memory.  With two stages a W' tile is pinned from its logits MMA until the dX MMA of the same tile
 // retires, about one and a half tile periods, which leaves the next load half a period to cross the
@@ -1041,7 +1041,11 @@ __global__ void __launch_bounds__(256) lmhead_join_kernel(const LmHeadArgs p, in
 }
 
 // Whether the sweep over `n_mtiles` row tiles is split: where whole tiles would leave the SMs at least SPLIT_STEPS
-// v-tile steps short of even.
+// v-tile steps short of even, which is what the pieces' stores and the join cost.  Whole / split in us (scoring, given
+// lse, one sweep; events, cold L2), by the steps short of even:
+//   10 (100 row tiles, V = 4096)   47 / 54, 72 / 77, 80 / 79      15 (130, 16 384)  152 / 155, 225 / 222, 242 / 237
+//   12 (430, 16 384)  424 / 429, 631 / 638, 686 / 683             16 (370, 4096)    129 / 124, 201 / 189, 221 / 204
+//   20 (100, 8192)    80 / 77, 121 / 112, 130 / 118               39 (250, 16 384)  287 / 265, 424 / 390, 459 / 417
 constexpr int LH_SPLIT_STEPS = 16;
 static bool lh_split(long long n_mtiles, long long n_vtiles) {
   const long long sms = ccb_num_sms(), waves = (n_mtiles + sms - 1) / sms;

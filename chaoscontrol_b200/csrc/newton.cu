@@ -190,10 +190,14 @@ newton_kernel(const NewtonArgs p) {
   }
 }
 
-// One tile of every product to a CTA, and not more clusters than two rounds of four-CTA ones or one of eight-CTA
-// ones.  Measured, five iterations on the device, one launch / fifteen in us: 16 of 256 x 256 74 / 134, 64 of them
-// 150 / 189, 4 of 512 x 256 84 / 139, 3 of 72 x 200 50 / 107; 32 of 512 x 256 246 / 175, and with two tiles to a CTA
-// 1 of 512 x 512 178 / 160, 16 of them 357 / 220.
+// One tile of every product to a CTA (with two, 1 of 512 x 512 took 178 us against 160, 16 of them 357 against 220), and
+// not more CTAs than the lines below.  A matrix takes about 75 us whatever the batch, so time goes up by that with
+// every round of clusters: 148 SMs hold 14 clusters of eight at once, 36 of four.  Five iterations, one launch /
+// fifteen in us (events, cold L2):
+//   eight CTAs (512 x 256):  8 matrices 86 / 153, 14 88 / 163, 16 166 / 165, 32 248 / 216    -> 16: 7/8 of the SMs
+//   four (256 x 256):        32 80 / 177, 64 154 / 224, 74 225 / 226, 148 373 / 329          -> 74: twice the SMs
+//   two (128 x 256):         74 72 / 153, 148 137 / 187          one (128 x 128):  148 70 / 165, 296 131 / 230
+// Past its line the gain comes and goes with the last round (20 of 512 x 256 168 / 214, 80 of 256 x 256 225 / 308).
 static bool newton_fits(int64_t G, int64_t tiles, int cl) {
   const int64_t sms = ccb_num_sms();
   return tiles <= cl && G * cl <= (cl == 8 ? sms * 7 / 8 : 2 * sms);
