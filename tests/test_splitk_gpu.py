@@ -58,3 +58,14 @@ def test_splitk_reduce_group_rule(S, N, K):
     p64 = part.double()
     assert ((out.double() - p64.sum(0)).abs() <= S * 2.0 ** -24 * p64.abs().sum(0) + 1e-30).all()
     assert torch.equal(out, splitk_reduce(part)[0])
+
+
+@pytest.mark.parametrize("S,N,K", [(5, 8192, 256), (15, 4096, 512), (37, 1024, 256), (74, 256, 256), (40, 4096, 256)])
+def test_splitk_reduce_error_is_below_that_of_a_serial_sum(S, N, K):
+    """fp32 sums of random partials against 64 bits, next to adding them one after the other in fp32."""
+    part = torch.randn(S, N, K, generator=torch.Generator(device="cuda").manual_seed(S), device="cuda")
+    serial = torch.zeros(N, K, device="cuda")
+    for p in part:
+        serial += p
+    ref = part.double().sum(0)
+    assert (splitk_reduce(part)[0].double() - ref).norm() <= 0.98 * (serial.double() - ref).norm()
