@@ -313,8 +313,11 @@ struct SpkOut {
   OT* p[4];
   int rows;
   __device__ __forceinline__ OT* row(int n, int K) const {
-    const int i = (n >= rows) + (n - rows >= rows) + (n - rows - rows >= rows);      // rows = N for one tensor
-    return p[i] + (long long)(n - i * rows) * K;
+    OT* q = p[0];                              // rows = N for one tensor
+    if (n >= rows) { q = p[1]; n -= rows; }
+    if (n >= rows) { q = p[2]; n -= rows; }
+    if (n >= rows) { q = p[3]; n -= rows; }
+    return q + (long long)n * K;
   }
 };
 __device__ __forceinline__ void store_grad1(__nv_bfloat16* o, float v) { *o = __float2bfloat16(v); }
