@@ -339,8 +339,11 @@ def _scan_bwd(P, log_a32, h0, h, dy, dhT, rowss, inv_dim, eps, B, T, D, want_dh0
     return dP.to(P.dtype), grads[1], (grads[2] if len(grads) > 2 else None)
 
 
-def _plain_bf16(*ts) -> bool:
-    return all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() for t in ts)
+def _plain_bf16(*ts, dtype=torch.bfloat16) -> bool:
+    for t in ts:                                # loops: half the time of a generator, on every layer call
+        if not (t.is_cuda and t.dtype is dtype and t.is_contiguous()):
+            return False
+    return True
 
 
 def _layer_shaped(w: "LayerWeights", D: int, F_: int) -> bool:
@@ -351,8 +354,11 @@ def _layer_shaped(w: "LayerWeights", D: int, F_: int) -> bool:
             w.Wproj.shape == (D, F_) and w.log_a32.shape == (D,))
 
 
-def _plain_f32(*ts) -> bool:
-    return all(t is None or (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()) for t in ts)
+def _plain_f32(*ts, dtype=torch.float32) -> bool:
+    for t in ts:
+        if t is not None and not (t.is_cuda and t.dtype is dtype and t.is_contiguous()):
+            return False
+    return True
 
 
 def _layer_args(w: LayerWeights, B: int, T: int, D: int, F_: int, x, ss1, h0, acts, ss2) -> "_lib.LayerArgs":
