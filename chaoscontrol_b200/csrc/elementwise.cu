@@ -1342,11 +1342,13 @@ extern "C" int ccb_rmsnorm_fwd(const void* x, const void* res, const void* w, vo
 // gw_part must hold ccb_rmsnorm_bwd_blocks(R) * D floats.  Eight per-warp [D] strips of shared
 // memory bound the channel count (48 KiB without an opt-in).
 constexpr int RMSNORM_BWD_MAX_DIM = 1536;
-// Rows of a block: four blocks to an SM, at least one row for each of the eight warps.  (256 rows, the
-// former constant, left 9 000 rows on 36 of 148 SMs: 89 us at 384 channels, now 7.)
+// Rows of a block: whole rounds of the two blocks that an SM holds, at least two rounds and no block of more than 256
+// rows; at least one row for each of the eight warps.  256 rows for every size left 9 000 rows on 36 SMs (89 us at 384
+// channels, now 7); always two rounds made the blocks of large batches long, and the last ones late: 300 000 x 256
+// 124 us (110 in four rounds), 1 000 000 x 66 357 (308 in blocks of 256, which cost 160 000 x 512 a third round: 97 -> 114).
 static inline int64_t rmsnorm_bwd_rows(int64_t R) {
-  const int64_t blocks = 4 * (int64_t)ccb_num_sms();
-  const int64_t rows = (R + blocks - 1) / blocks;
+  const int64_t round = 2 * (int64_t)ccb_num_sms(), rounds = (R + 256 * round - 1) / (256 * round);
+  const int64_t blocks = round * (rounds < 2 ? 2 : rounds), rows = (R + blocks - 1) / blocks;
   return rows < 8 ? 8 : (rows + 7) / 8 * 8;
 }
 extern "C" int64_t ccb_rmsnorm_bwd_blocks(int64_t R) {

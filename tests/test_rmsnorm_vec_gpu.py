@@ -33,3 +33,21 @@ def test_rmsnorm_against_64_bits(R, D, shift):
     assert ((gx.double() - inv * (gwt - xh * dot)).abs() <= rnd * (inv * (gwt - xh * dot)).abs() + fp * mag).all()
     ref = (g64 * xh).sum(0)
     assert ((gw.double() - ref).abs() <= rnd * ref.abs() + (R + 16) * 2.0 ** -24 * (g64 * xh).abs().sum(0)).all()
+
+
+# one row more than two rounds of 256-row blocks on 148 SMs, and several rounds; whole vectors and not
+@pytest.mark.parametrize("R,D", [(2 * 296 * 256 + 1, 64), (400003, 66)])
+def test_rmsnorm_backward_of_many_rows(R, D):
+    """The weight gradient over several rounds of blocks against 64 bits (R fp32 products and additions at most, rounded
+    to bf16), and the same bits on every run."""
+    from chaoscontrol_b200.kernels import fused_rms_norm
+    g = torch.Generator(device="cuda").manual_seed(R)
+    x = torch.randn(R, D, generator=g, device="cuda").bfloat16()
+    w = torch.ones(D, device="cuda").bfloat16().requires_grad_(True)
+    go = torch.randn(R, D, generator=g, device="cuda").bfloat16()
+    (gw,) = torch.autograd.grad(fused_rms_norm(x, w), (w,), go)
+    xd = x.double()
+    terms = go.double() * xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-6)
+    ref, mag = terms.sum(0), terms.abs().sum(0)
+    assert ((gw.double() - ref).abs() <= R * 2.0 ** -24 * mag + 2.0 ** -8 * ref.abs()).all()
+    assert torch.equal(gw, torch.autograd.grad(fused_rms_norm(x, w), (w,), go)[0])
