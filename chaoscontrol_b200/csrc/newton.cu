@@ -197,7 +197,8 @@ newton_kernel(const NewtonArgs p) {
 //   eight CTAs (512 x 256):  8 matrices 86 / 153, 14 88 / 163, 16 166 / 165, 32 248 / 216    -> 16: 7/8 of the SMs
 //   four (256 x 256):        32 80 / 177, 64 154 / 224, 74 225 / 226, 148 373 / 329          -> 74: twice the SMs
 //   two (128 x 256):         74 72 / 153, 148 137 / 187          one (128 x 128):  148 70 / 165, 296 131 / 230
-// Past its line the gain comes and goes with how full the last wave of clusters is (20 of 512 x 256 168 / 214, 80 of 256 x 256 225 / 308).
+// Past its line the gain comes and goes with how full the last wave of clusters is (20 of 512 x 256 168 / 214, 80 of
+// 256 x 256 225 / 308).
 static bool newton_fits(int64_t G, int64_t tiles, int cl) {
   const int64_t sms = ccb_num_sms();
   return tiles <= cl && G * cl <= (cl == 8 ? sms * 7 / 8 : 2 * sms);
